@@ -3,6 +3,10 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include <type_traits>
+
+#include "gbhf_ff.cuh"
+
 #define TWO_PI_2P5 34.98683665524972   // 2 pi^(5/2)
 #define GBHF_PI 3.141592653589793
 
@@ -61,6 +65,17 @@ __device__ __forceinline__ void load_bra_prim(const float* __restrict__ r, BraPr
   b.p = x0.x, b.invp = x0.y, b.Px = x0.z, b.Py = x0.w, b.Pz = x1.x, b.PAx = x1.y, b.PAy = x1.z;
   b.PAz = x1.w, b.PBx = x2.x, b.PBy = x2.y, b.PBz = x2.z, b.K = x2.w, b.a = x3.x;
 }
+// Two-float pairs: the centre P is held as P - A only (X = (A - C) + (P - A) -
+// (Q - C) keeps the small differences exact), so Px, Py, Pz are P - A here.
+__device__ __forceinline__ void load_bra_prim(const gbhf::ff* __restrict__ r, BraPrim<gbhf::ff>& b) {
+  const float4* v = reinterpret_cast<const float4*>(r);
+  const float4 x0 = v[0], x2 = v[2], x3 = v[3], x4 = v[4], x5 = v[5], x6 = v[6];
+  using gbhf::ff;
+  b.p = ff(x0.x, x0.y), b.invp = ff(x0.z, x0.w), b.PAx = ff(x2.z, x2.w), b.PAy = ff(x3.x, x3.y);
+  b.PAz = ff(x3.z, x3.w), b.PBx = ff(x4.x, x4.y), b.PBy = ff(x4.z, x4.w), b.PBz = ff(x5.x, x5.y);
+  b.K = ff(x5.z, x5.w), b.a = ff(x6.x, x6.y);
+  b.Px = b.PAx, b.Py = b.PAy, b.Pz = b.PAz;
+}
 
 // 1/sqrt(x) in FP64 with few FP64-pipe instructions (that pipe is 1/64 of the
 // FP32 rate on this GPU): x is truncated to single precision by moving its
@@ -91,9 +106,26 @@ __device__ __forceinline__ double widen(float x) {
   return __hiloint2double(hi, (int)((unsigned)b << 29));
 }
 
+// A kernel's result as the double to accumulate; two-float results also take
+// the power of two 2^e that their density was scaled by.  Exponent arithmetic on
+// both halves and one FP64 addition; a head that is not finite is kept as it is.
+__device__ __forceinline__ double widen(double x, int) { return x; }
+__device__ __forceinline__ double widen(float x, int) { return widen(x); }
+__device__ __forceinline__ double scale_exp(float x, int e) {
+  const int b = __float_as_int(x);
+  if ((b & 0x7f800000) == 0) return 0.0;
+  const int hi = (b & (int)0x80000000) | ((((b >> 23) & 0xff) + 896 + e) << 20) | ((b >> 3) & 0xfffff);
+  return __hiloint2double(hi, (int)((unsigned)b << 29));
+}
+__device__ __forceinline__ double widen(gbhf::ff x, int e) {
+  if (!(fabsf(x.h) <= 3.4e38f)) return (double)x.h;
+  return scale_exp(x.h, e) + scale_exp(x.l, e);
+}
+
 template <typename T> __device__ __forceinline__ T rsqrt_t(T x);
 template <> __device__ __forceinline__ double rsqrt_t<double>(double x) { return rsqrt_d(x); }
 template <> __device__ __forceinline__ float rsqrt_t<float>(float x) { return rsqrtf(x); }
+template <> __device__ __forceinline__ gbhf::ff rsqrt_t<gbhf::ff>(gbhf::ff x) { return gbhf::rsqrt_ff(gbhf::nrm(x)); }
 
 // Nearest integer j of x (0 <= x < 2^22), returned as j and as the exact
 // floating-point value of j: adding 1.5 * 2^52 (1.5 * 2^23 for float) leaves j in
@@ -103,19 +135,26 @@ __device__ __forceinline__ double round_node(double x, int& j) {
   j = __double2loint(r);
   return r - 6755399441055744.0;
 }
-__device__ __forceinline__ float round_node(float x, int& j) {
-  const float r = x + 12582912.0f;
-  j = __float_as_int(r) - 0x4B400000;
-  return r - 12582912.0f;
-}
 
 template <typename T> __device__ __forceinline__ T fma_t(T a, T b, T c);
-__device__ __forceinline__ double fabs_t(double x) { return fabs(x); }
-__device__ __forceinline__ float fabs_t(float x) { return fabsf(x); }
 __device__ __forceinline__ double fmax_t(double a, double b) { return fmax(a, b); }
 __device__ __forceinline__ float fmax_t(float a, float b) { return fmaxf(a, b); }
 template <> __device__ __forceinline__ double fma_t<double>(double a, double b, double c) { return fma(a, b, c); }
 template <> __device__ __forceinline__ float fma_t<float>(float a, float b, float c) { return fmaf(a, b, c); }
+template <> __device__ __forceinline__ gbhf::ff fma_t<gbhf::ff>(gbhf::ff a, gbhf::ff b, gbhf::ff c) {
+  return gbhf::fma_ff(a, b, c);
+}
+// magnitude for screening (FP32 for two-float values)
+__device__ __forceinline__ double mag(double x) { return fabs(x); }
+__device__ __forceinline__ float mag(float x) { return fabsf(x); }
+__device__ __forceinline__ float mag(gbhf::ff x) { return fabsf(x.h); }
+template <typename T>
+__device__ __forceinline__ T shfl_xor_t(T v, int o) {
+  if constexpr (std::is_same<T, gbhf::ff>::value)
+    return gbhf::ff(__shfl_xor_sync(0xffffffffu, v.h, o), __shfl_xor_sync(0xffffffffu, v.l, o));
+  else
+    return __shfl_xor_sync(0xffffffffu, v, o);
+}
 
 // F_0..F_L(T) from the table by Taylor expansion about the nearest node;
 // asymptotic form F_0 = sqrt(pi/T)/2, F_m = F_(m-1) (2m-1)/(2T) beyond TMAX.
@@ -135,7 +174,6 @@ template <int L> struct BoysCfg<float, L> {
 // FMAs each.  The lower orders follow by the downward recursion
 // F_m = (2t F_(m+1) + exp(-t)) / (2m + 1), whose terms are all positive.  Rows are
 // 16-byte aligned and read with vector loads.
-#define BOYSH_LMAX 9   // (dd|dd) gradient: L = 9
 #define BOYSH64_STRIDE 16   // 6 + 6 doubles, the node T_j, padding
 #define BOYSH32_STRIDE 8    // 4 + 4 floats (two 16-byte loads)
 template <typename T> struct BoysHStride;
@@ -170,7 +208,7 @@ __device__ __forceinline__ void boys_row(const float* __restrict__ row, float* c
 }
 
 template <typename T, int L>
-__device__ __forceinline__ void boys_eval(T t, const T* __restrict__ tab, T* F) {
+__device__ __forceinline__ void boys_eval_num(T t, const T* __restrict__ tab, T* F) {
   using C = BoysCfg<T, L>;
   static_assert(L <= BOYSH_LMAX, "the Boys tables hold orders up to BOYSH_LMAX");
   // Node index and range test in FP32 for FP64 arguments (t truncated to float by
@@ -216,6 +254,12 @@ __device__ __forceinline__ void boys_eval(T t, const T* __restrict__ tab, T* F) 
 #pragma unroll
     for (int m = 1; m <= L; ++m) F[m] = F[m - 1] * T(2 * m - 1) * h;
   }
+}
+
+template <typename T, int L>
+__device__ __forceinline__ void boys_eval(T t, const T* __restrict__ tab, T* F) {
+  if constexpr (std::is_same<T, gbhf::ff>::value) gbhf::boys_eval_ff<L>(t, tab, F);
+  else boys_eval_num<T, L>(t, tab, F);
 }
 
 // Error codes written by kernels into the context's device status word.

@@ -166,6 +166,12 @@ constexpr int GRAD_COMBO_BRA[NCOMBO_MAX] = {0, 0, 0, 1, 1, 1, 2, 2, 2, 0, 0, 0, 
 constexpr int GRAD_COMBO_KET[NCOMBO_MAX] = {0, 1, 2, 0, 1, 2, 0, 1, 2, 3, 4, 5, 3, 4, 5, 3, 4, 5,
                                             0, 1, 2, 3, 4, 5, 0, 1, 2, 3, 4, 5, 0, 1, 2, 3, 4, 5};
 
+// Precision tiers of the direct builds, one task list each: FP64, FP32 (mixed
+// precision) and two-float (gbhf_ff.cuh; the part of the FP64 work whose bound
+// allows it).
+constexpr int NTIER = 3;
+constexpr int TIER_64 = 0, TIER_32 = 1, TIER_FF = 2;
+
 struct Segment {
   int start, end, K;   // global pair indices [start, end), primitive pairs per pair
   int data_off;        // offset of this segment's ket-layout primitive data
@@ -215,17 +221,19 @@ struct PairData {
   // (segment-transposed: prim k of pair j at data_off + k*len + (j-start)).
   DBuf<double> bra64, ket64;   // BRA_NFIELD arrays of length nprimpairs each
   DBuf<float> bra32, ket32;
+  DBuf<ff> braff, ketff;       // two-float values; Px, Py, Pz unused (P - A stands for P)
+  DBuf<double> ffq;            // per molecule: two-float below this Q_ab Q_cd (0: never)
   size_t nprim_pairs = 0;
 };
 
 struct TaskLists {
-  DBuf<int> item_count;    // per (combo, bra) item: [n64, n32]
-  DBuf<int> item_off;      // exclusive scan
+  DBuf<int> item_count;    // per (combo, bra) item: tasks of each tier
+  DBuf<int> item_off;      // exclusive scans, one row per tier
   DBuf<int> scan_part;     // per scan tile: sums, then their exclusive scan
-  DBuf<int4> tasks64, tasks32;
-  DBuf<int> ranges;        // per combo: start64, end64, start32, end32
-  DBuf<int> counters;      // per combo & precision: work-queue heads
-  DBuf<unsigned long long> stats;  // per combo: shell quartets, fn quartets, prim quartets (64, 32)
+  DBuf<int4> tasks[NTIER];
+  DBuf<int> ranges;        // per combo and tier: first task, end
+  DBuf<int> counters;      // per combo and tier: work-queue heads
+  DBuf<unsigned long long> stats;  // per combo and tier: shell quartets, fn quartets, prim quartets
   bool stats_pending = false;      // stats holds counts of builds not yet added to the profile
   DBuf<int> ics_d, cls_d, scs_d;   // task generation inputs (live until its kernels have run)
   int nitems = 0;
@@ -233,9 +241,10 @@ struct TaskLists {
   double thr_all = -1, thr64 = -1;     // thresholds the current lists were built for
   double thr_exact = 0;                // per-quartet density screening cutoff of the current build
   int ncombo = 0;
-  int hranges[4 * NCOMBO_MAX] = {0};   // host copy of ranges
+  int hranges[2 * NTIER * NCOMBO_MAX] = {0};   // host copy of ranges
   DBuf<int> f0;                        // first basis function per shell
   DBuf<double> sscale;                 // per shell: 6 component scales (d shells; 1 otherwise)
+  DBuf<float4> cen;                    // per shell: its centre in three FP32 parts (two-float kernels)
   DBuf<int> nc;                        // components per shell
   DBuf<int> atom;                      // atom of each shell
   DBuf<int> smol;                      // molecule of each shell
@@ -293,6 +302,7 @@ struct gbhf_ctx {
   gbhf::DBuf<float> boys32;      // exact FP32 table
   gbhf::DBuf<double> boysh64;    // Horner tables for the J/K kernels
   gbhf::DBuf<float> boysh32;
+  gbhf::DBuf<float4> boyshff;    // two-float Horner table
   // basis on device (function level, for 1-e integrals and canonical ERIs)
   gbhf::DBuf<double> d_xyz, d_Z, d_coef, d_exp;
   gbhf::DBuf<int> d_fn;          // per CGF: atom, lx, ly, lz, np, off (6 ints)
@@ -333,6 +343,9 @@ struct gbhf_ctx {
   std::map<std::string, std::vector<double>> sad_cache;
   gbhf_ctx* sad_ctx = nullptr;
   gbhf::DBuf<float> dfloat;
+  gbhf::DBuf<gbhf::ff> dff;         // density of the two-float kernels, scaled by 2^-e
+  gbhf::DBuf<int> dff_exp;          // e
+  gbhf::DBuf<double> dff_max;       // max |D| of it
   gbhf::DBuf<int> dev_status;
   int purify_grid = 0;              // co-resident blocks of the fused purification kernel
   int tc2_grid = 0;                 // co-resident blocks of the one-barrier TC2 kernel
@@ -345,9 +358,9 @@ struct gbhf_ctx {
   gbhf::DBuf<double> small;
   gbhf::Profile prof;
   cudaEvent_t ev[4] = {nullptr, nullptr, nullptr, nullptr};
-  cudaEvent_t evc[2 * gbhf::NCOMBO + 1] = {};   // per-class J/K launch boundaries (profiling)
+  cudaEvent_t evc[gbhf::NTIER * gbhf::NCOMBO + 1] = {};   // per-class J/K launch boundaries (profiling)
   cudaEvent_t evu[8] = {};       // user slots (gbhf_event_record)
-  cudaEvent_t evg[2 * gbhf::NCOMBO_MAX + 1] = {};   // per-combo gradient launch boundaries (profiling)
+  cudaEvent_t evg[gbhf::NTIER * gbhf::NCOMBO_MAX + 1] = {};   // per-combo gradient launch boundaries (profiling)
   cudaEvent_t evp[5] = {};       // SCF step phase boundaries (Fock, DIIS, density, convergence)
   // task budgets of the direct builds per quartet class (J/K) and class pair
   // (gradient): primitive quartets per lane and task, kets per task
@@ -479,19 +492,22 @@ gbhf_status jk_build(gbhf_ctx* c, const double* d_Dsq, double* d_G, int precisio
 // bra-layout primitive data at d_poff), FP64 class code.
 gbhf_status schwarz_classes_dev(gbhf_ctx* c, const int* cls_start, const int* d_K, const int* d_poff,
                                 const double* d_bra, long long npp, double* d_Q);
+// The two-float instances (jk_ff.cu, grad_ff.cu) of the lane-per-ket kernels.
+gbhf_status launch_jk_ff(gbhf_ctx* c, cudaStream_t strm, int k, double* G, int nt, int wj);
+gbhf_status launch_grad_ff(gbhf_ctx* c, cudaStream_t strm, int k, double* grad, int nt);
 // jkd.cu / gradd.cu: the classes with a d pair (warp per shell quartet).
 // Schwarz bounds of classes 3..5 (dA, dB: shells of each pair, same order).
 gbhf_status schwarz_dclasses_dev(gbhf_ctx* c, const int* cls_start, const int* dA, const int* dB, const int* d_K,
                                  const int* d_poff, const double* d_bra, long long npp, double* d_Q);
-// J/K launch of combo 6..20 (COMBO_BRA/COMBO_KET), precision 0 = FP64, 1 = FP32.
-gbhf_status launch_jk_dclass(gbhf_ctx* c, cudaStream_t strm, int combo, int prec, const double* D64,
-                             const float* D32, double* G, int ntask, int with_j);
+// J/K launch of the combos without generated code (COMBO_BRA/COMBO_KET).
+gbhf_status launch_jk_dclass(gbhf_ctx* c, cudaStream_t strm, int combo, int tier, const double* D64, double* G,
+                             int ntask, int with_j);
 // Gradient combos on the generated lane-per-ket kernels (grad.cu); the rest
 // go to launch_grad_dclass.
 bool grad_gen_combo(int k);
 // Gradient launch of a combo 9..35 (GRAD_COMBO_BRA/GRAD_COMBO_KET) without generated code.
-gbhf_status launch_grad_dclass(gbhf_ctx* c, cudaStream_t strm, int combo, int prec, const double* D64,
-                               const float* D32, double* grad, int ntask);
+gbhf_status launch_grad_dclass(gbhf_ctx* c, cudaStream_t strm, int combo, int tier, const double* D64, double* grad,
+                               int ntask);
 // linalg.cu
 // sym: C (square) is known to be symmetric; only its upper tiles are computed and mirrored.
 gbhf_status gemm(gbhf_ctx* c, bool ta, bool tb, int m, int n, int k, double alpha, const double* A, int lda,
@@ -554,5 +570,23 @@ gbhf_status purify_finish(gbhf_ctx* c, const double* rec);
 gbhf_status purify_flush(gbhf_ctx* c);
 gbhf_status max_abs_dev(gbhf_ctx* c, size_t n, const double* d_x, double* d_out);   // into device memory
 gbhf_status to_float(gbhf_ctx* c, size_t n, const double* d_x, float* d_y);
+gbhf_status to_ff(gbhf_ctx* c, size_t n, const double* d_x);   // into c->dff, c->dff_exp
+
+// Primitive-pair data and Boys table of a kernel's value type.
+template <typename T> inline const T* pair_bra(const PairData& P) {
+  if constexpr (std::is_same<T, ff>::value) return P.braff.p;
+  else if constexpr (sizeof(T) == 4) return P.bra32.p;
+  else return P.bra64.p;
+}
+template <typename T> inline const T* pair_ket(const PairData& P) {
+  if constexpr (std::is_same<T, ff>::value) return P.ketff.p;
+  else if constexpr (sizeof(T) == 4) return P.ket32.p;
+  else return P.ket64.p;
+}
+template <typename T> inline const T* boys_table(const gbhf_ctx* c) {
+  if constexpr (std::is_same<T, ff>::value) return reinterpret_cast<const ff*>(c->boyshff.p);
+  else if constexpr (sizeof(T) == 4) return c->boysh32.p;
+  else return c->boysh64.p;
+}
 
 }  // namespace gbhf

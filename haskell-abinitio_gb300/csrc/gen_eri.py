@@ -71,7 +71,7 @@ def e_axis_code(prefix, pa, pb, h, lmax_a, lmax_b, needed):
                 return None
             s = " + ".join(inner)
             coef = h if t == 1 else f"({h} * T({1.0 / t!r}))"
-            terms = [f"{coef} * ({s})"]
+            terms = [coef if s == "ONE" else f"{coef} * ({s})"]
         if not terms:
             memo[key] = None
             return None
@@ -165,7 +165,7 @@ def gen_class(la, lb, lc, ld):
     w("    const T QCx, const T QCy, const T QCz, const T QDx, const T QDy, const T QDz,")
     w("    const T Kcd, const T* __restrict__ boys, Acc& acc) {")
     w("  const T ONE = T(1);")
-    w("  (void)QCx; (void)QCy; (void)QCz; (void)QDx; (void)QDy; (void)QDz;")
+    w("  (void)ONE; (void)QCx; (void)QCy; (void)QCz; (void)QDx; (void)QDy; (void)QDz;")
     # ket E (hoisted out of the bra loop)
     w("  const T hq = T(0.5) * invq;")
     kneed = axis_needs(cc, cd)
@@ -189,13 +189,13 @@ def gen_class(la, lb, lc, ld):
             fac = [f for f in (fx, fy, fz) if f != "ONE"]
             sign = -1 if (t + u + v) % 2 else 1
             nm = f"ekp{ic}{idd}_{t}{u}{v}"
-            if not fac:
-                expr = "ONE" if sign > 0 else "-ONE"
+            if not fac:   # a unit coefficient: no product with it
+                nm = "ONE" if sign > 0 else "-ONE"
             else:
                 expr = " * ".join(fac)
                 if sign < 0:
                     expr = f"-({expr})"
-            w(f"  const T {nm} = {expr};")
+                w(f"  const T {nm} = {expr};")
             lst.append((nm, (t, u, v)))
         ket_terms[(ic, idd)] = lst
     # (ss|ss) and (ps|ss): two bra primitives in flight (two independent load
@@ -335,7 +335,7 @@ def gen_class_deferred(la, lb, lc, ld):
     w("    const T QCx, const T QCy, const T QCz, const T QDx, const T QDy, const T QDz,")
     w("    const T Kcd, const T* __restrict__ boys, Acc& acc) {")
     w("  const T ONE = T(1);")
-    w("  (void)QCx; (void)QCy; (void)QCz; (void)QDx; (void)QDy; (void)QDz;")
+    w("  (void)ONE; (void)QCx; (void)QCy; (void)QCz; (void)QDx; (void)QDy; (void)QDz;")
     w("  const T hq = T(0.5) * invq;")
     kneed = axis_needs(cc, cd)
     kmaps = []
@@ -357,13 +357,13 @@ def gen_class_deferred(la, lb, lc, ld):
             fac = [f for f in (fx, fy, fz) if f != "ONE"]
             sign = -1 if (t + u + v) % 2 else 1
             nm = f"ekp{ic}{idd}_{t}{u}{v}"
-            if not fac:
-                expr = "ONE" if sign > 0 else "-ONE"
+            if not fac:   # a unit coefficient: no product with it
+                nm = "ONE" if sign > 0 else "-ONE"
             else:
                 expr = " * ".join(fac)
                 if sign < 0:
                     expr = f"-({expr})"
-            w(f"  const T {nm} = {expr};")
+                w(f"  const T {nm} = {expr};")
             lst.append((nm, (t, u, v)))
         ket_terms[(ic, idd)] = lst
     ket_union = sorted({h for lst in ket_terms.values() for (_, h) in lst}, key=lambda k: (sum(k), k))

@@ -200,13 +200,13 @@ def gen_class(la, lb, lc, ld):
             fac = [f for f in (fx, fy, fz) if f != "ONE"]
             sign = -1 if (t + u + v) % 2 else 1
             nm = f"ekp{ic}{idd}_{t}{u}{v}"
-            if not fac:
-                expr = "ONE" if sign > 0 else "-ONE"
+            if not fac:   # a unit coefficient: no product with it
+                nm = "ONE" if sign > 0 else "-ONE"
             else:
                 expr = " * ".join(fac)
                 if sign < 0:
                     expr = f"-({expr})"
-            w(f"  const T {nm} = {expr};")
+                w(f"  const T {nm} = {expr};")
             lst[(t, u, v)] = nm
         ket_terms[(ic, idd)] = lst
     # T_ab(tau) = sum_cd Gamma_abcd ekp_cd(tau)

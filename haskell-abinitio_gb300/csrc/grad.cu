@@ -25,310 +25,9 @@
 
 #include "gbhf_internal.h"
 #include "gbhf_md.cuh"
-#include "grad_gen.cuh"
+#include "grad_kern.cuh"
 
 namespace gbhf {
-
-// ----------------------------------------------------------- two-electron ----
-// Warp per task (bra shell pair, up to 32 kets of one segment, a range of bra
-// primitives), as the J/K kernels: the bra primitive pairs are staged in
-// shared memory, each lane runs the generated bra-derivative code for its ket
-// pair against them, and the warp reduces the six bra-centre components before
-// one set of atomics.  Summed over every ordered pair of shell pairs with
-// weights (2 - delta_AB)(2 - delta_CD), the bra-centre derivatives give the
-// whole two-electron gradient (the ket-centre terms of (P|Q) are the
-// bra-centre terms of (Q|P)).
-
-constexpr int GR_THREADS = 128;
-constexpr int GR_WARPS = GR_THREADS / 32;
-
-template <typename T, int N>
-struct GamReg {
-  T v[N];
-  __device__ __forceinline__ T get(int i) const { return v[i]; }
-  __device__ __forceinline__ void set(int i, T x) { v[i] = x; }
-};
-template <typename T, int N>
-struct GamSmem {   // per-thread column of a [N][GR_THREADS] shared array
-  T* p;
-  // volatile: a read stays where the code places it (the bra loop reads T_ab
-  // block by block; hoisted out of the loop, all of T would be live at once)
-  __device__ __forceinline__ T get(int i) const { return *(volatile const T*)(p + i * GR_THREADS); }
-  __device__ __forceinline__ void set(int i, T x) { p[i * GR_THREADS] = x; }
-};
-
-template <int LA, int LB, int LC, int LD>
-struct GradFn;
-#define GBHF_GRAD_FN(la, lb, lc, ld, name)                                                                      \
-  template <>                                                                                                  \
-  struct GradFn<la, lb, lc, ld> {                                                                              \
-    template <typename T, typename G, typename TK>                                                             \
-    static __device__ __forceinline__ void ket(T invq, T QCx, T QCy, T QCz, T QDx, T QDy, T QDz, const G& gam, \
-                                               TK& tk) {                                                       \
-      grad_ket_##name<T, G, TK>(invq, QCx, QCy, QCz, QDx, QDy, QDz, gam, tk);                                  \
-    }                                                                                                          \
-    template <typename T, typename TK>                                                                         \
-    static __device__ __forceinline__ void run(const T* sb, int nbra, int bstep, T q, T Qx, T Qy, T Qz, T Kcd, \
-                                               const T* boys, const TK& tk, T* g) {                            \
-      grad_ketprim_##name<T, TK>(sb, nbra, bstep, q, Qx, Qy, Qz, Kcd, boys, tk, g);                            \
-    }                                                                                                          \
-  };
-GBHF_GRAD_FN(0, 0, 2, 0, ssds)
-GBHF_GRAD_FN(0, 0, 2, 1, ssdp)
-GBHF_GRAD_FN(1, 0, 2, 0, psds)
-GBHF_GRAD_FN(2, 0, 0, 0, dsss)
-GBHF_GRAD_FN(2, 0, 1, 0, dsps)
-GBHF_GRAD_FN(0, 0, 0, 0, ssss)
-GBHF_GRAD_FN(0, 0, 1, 0, ssps)
-GBHF_GRAD_FN(0, 0, 1, 1, sspp)
-GBHF_GRAD_FN(1, 0, 0, 0, psss)
-GBHF_GRAD_FN(1, 0, 1, 0, psps)
-GBHF_GRAD_FN(1, 0, 1, 1, pspp)
-GBHF_GRAD_FN(1, 1, 0, 0, ppss)
-GBHF_GRAD_FN(1, 1, 1, 0, ppps)
-GBHF_GRAD_FN(1, 1, 1, 1, pppp)
-
-template <typename T>
-struct GradArgs {
-  const int4* tasks;
-  const int* range;          // start, end of this class and precision
-  int* counter;
-  const int *pA, *pB, *pK, *poff, *kseg;
-  const int4* seg;
-  const T* bra;
-  const T* ket;
-  long long npp;
-  const int* shell_f0;
-  const int* shell_atom;     // global atom of each shell (grad index)
-  const int* pmol;
-  const int* mn;
-  const long long* moff;
-  const T* D;                // stacked n_m x n_m densities, this precision
-  const T* boys;
-  double* grad;              // 3 * natoms
-  const double* sscale;      // per shell 6 component scales (d shells)
-  const double* Q;           // Schwarz bound of each pair, and in FP32
-  const float* Qf;
-  double thr;                // drop a quartet when Q_ab Q_cd max|Gamma_abcd| is below
-  float thrf;
-  T jcoef;                   // weight of the Coulomb term D_ab D_cd in Gamma (0: exchange only)
-};
-
-__device__ __forceinline__ double warp_sum_d(double v) {
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-  return v;
-}
-
-template <int LA, int LB, int LC, int LD, typename T, bool SG>
-__global__ void __launch_bounds__(GR_THREADS) k_grad_jk(GradArgs<T> a) {
-  constexpr int NA = ncart_c(LA), NB = ncart_c(LB), NC = ncart_c(LC), ND = ncart_c(LD);
-  constexpr int NAB = NA * NB, NCD = NC * ND, NOUT = NAB * NCD;
-  __shared__ __align__(16) T sbra[GR_WARPS][KMAX_PRIM_PAIRS * BRA_SB];
-  __shared__ T sDab[GR_WARPS][NAB];
-  extern __shared__ double gsm_dyn[];
-  constexpr int NT = NAB * nherm_c(LC + LD);
-  using GamT = typename std::conditional<SG, GamSmem<T, NOUT>, GamReg<T, NOUT>>::type;
-  using TkT = typename std::conditional<SG, GamSmem<T, NT>, GamReg<T, NT>>::type;
-  GamT gam;
-  TkT tk;
-  if constexpr (SG) {
-    gam.p = reinterpret_cast<T*>(gsm_dyn) + threadIdx.x;
-    tk.p = reinterpret_cast<T*>(gsm_dyn) + NOUT * GR_THREADS + threadIdx.x;
-  }
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int start = a.range[0];
-  const int ntask = a.range[1] - start;
-  const long long npp = a.npp;
-  while (true) {
-    int t = 0;
-    if (lane == 0) t = atomicAdd(a.counter, 1);
-    t = __shfl_sync(0xffffffffu, t, 0);
-    if (t >= ntask) break;
-    const int4 task = a.tasks[start + t];
-    const int ib = task.x;
-    // lanes beyond the task's kets split the primitive quartets (as in k_jk):
-    // ket on the low lg bits of the lane, an nsb x nsk grid of bra and ket
-    // primitive slices on the rest; the closing warp sum adds the slices
-    const int nk = task.z;
-    const int lg = 32 - __clz(max(nk, 1) - 1);
-    const int nsl = 32 >> lg;
-    const int slice = lane >> lg;
-    const int jk = task.y + (lane & ((1 << lg) - 1));
-    const int mol = a.pmol[ib];
-    const int n = a.mn[mol];
-    const T* __restrict__ Dm = a.D + a.moff[mol];
-    const bool active = (lane & ((1 << lg) - 1)) < nk;
-    const int kb0 = task.w & 0xffff, Kb = (task.w >> 16) - kb0, pb0 = a.poff[ib] + kb0;
-    const int K = a.seg[a.kseg[task.y]].z;
-    constexpr int KETC = sizeof(T) == 4 ? 1 : 0;   // per-ket-primitive work, as in k_jk
-    int lb = 0;
-    for (int l = 0, best = 1 << 30; (1 << l) <= nsl; ++l) {
-      const int cost = (((Kb + (1 << l) - 1) >> l) + KETC) * ((K + (nsl >> l) - 1) / (nsl >> l));
-      if (KETC ? cost < best : cost <= best) {
-        best = cost;
-        lb = l;
-      }
-    }
-    const int nsb = 1 << lb, nsk = nsl >> lb;
-    const int sb = slice & (nsb - 1), sk = slice >> lb;
-    const unsigned rkb = (65536u + Kb - 1) / Kb;   // idx / Kb = (idx * rkb) >> 16 for idx < 16 * 36
-    for (int idx = lane; idx < BRA_NFIELD * Kb; idx += 32) {
-      const int f = (int)(((unsigned)idx * rkb) >> 16), k = idx - f * Kb;
-      sbra[warp][k * BRA_SB + f] = a.bra[(long long)f * npp + pb0 + k];
-    }
-    const int A = a.pA[ib], B = a.pB[ib];
-    const int a0 = a.shell_f0[A], b0 = a.shell_f0[B];
-    for (int i = lane; i < NAB; i += 32) sDab[warp][i] = Dm[(long long)(a0 + i / NB) * n + b0 + i % NB];
-    __syncwarp();
-    T g[6] = {0, 0, 0, 0, 0, 0};
-    T wgt = 0;
-    if (active) {
-      const int C = a.pA[jk], Dd = a.pB[jk];
-      const int c0 = a.shell_f0[C], d0 = a.shell_f0[Dd];
-      T gmax = T(0);
-      // Gamma_abcd = jcoef D_ab D_cd - (D_ac D_bd + D_ad D_bc) / 4
-#pragma unroll
-      for (int ia = 0; ia < NA; ++ia)
-#pragma unroll
-        for (int ibb = 0; ibb < NB; ++ibb)
-#pragma unroll
-          for (int ic = 0; ic < NC; ++ic)
-#pragma unroll
-            for (int id = 0; id < ND; ++id) {
-              const T dab = sDab[warp][ia * NB + ibb];
-              const T dcd = Dm[(long long)(c0 + ic) * n + d0 + id];
-              const T dac = Dm[(long long)(a0 + ia) * n + c0 + ic];
-              const T dbd = Dm[(long long)(b0 + ibb) * n + d0 + id];
-              const T dad = Dm[(long long)(a0 + ia) * n + d0 + id];
-              const T dbc = Dm[(long long)(b0 + ibb) * n + c0 + ic];
-              T gv = a.jcoef * dab * dcd - T(0.25) * (dac * dbd + dad * dbc);
-              if constexpr (LA == 2 || LB == 2 || LC == 2 || LD == 2) {   // d components: scaled functions
-                if (LA == 2) gv *= T(a.sscale[6 * A + ia]);
-                if (LB == 2) gv *= T(a.sscale[6 * B + ibb]);
-                if (LC == 2) gv *= T(a.sscale[6 * C + ic]);
-                if (LD == 2) gv *= T(a.sscale[6 * Dd + id]);
-              }
-              gam.set(((ia * NB + ibb) * NC + ic) * ND + id, gv);
-              gmax = fmax_t(gmax, fabs_t(gv));
-            }
-      // exact screening of this quartet by its own Gamma (the task lists bound it
-      // by the pairs' density weights)
-      bool keep;
-      if constexpr (sizeof(T) == 4) keep = a.Qf[ib] * a.Qf[jk] * gmax >= a.thrf;
-      else keep = a.Q[ib] * a.Q[jk] * gmax >= a.thr;
-      const int4 sg = a.seg[a.kseg[jk]];
-      const int len = sg.y - sg.x;
-      const long long base = (long long)sg.w + (jk - sg.x);
-      const int nbl = sb < Kb && keep ? (Kb - sb + nsb - 1) / nsb : 0;
-      for (int kc = sk; keep && kc < K; kc += nsk) {
-        const long long idx = base + (long long)kc * len;
-        const T q = a.ket[BRA_P * npp + idx];
-        const T invq = a.ket[BRA_INVP * npp + idx];
-        const T Qx = a.ket[BRA_PX * npp + idx], Qy = a.ket[BRA_PY * npp + idx], Qz = a.ket[BRA_PZ * npp + idx];
-        T QCx = 0, QCy = 0, QCz = 0, QDx = 0, QDy = 0, QDz = 0;
-        if (LC >= 1) {
-          QCx = a.ket[BRA_PAX * npp + idx];
-          QCy = a.ket[BRA_PAY * npp + idx];
-          QCz = a.ket[BRA_PAZ * npp + idx];
-        }
-        if (LD >= 1) {
-          QDx = a.ket[BRA_PBX * npp + idx];
-          QDy = a.ket[BRA_PBY * npp + idx];
-          QDz = a.ket[BRA_PBZ * npp + idx];
-        }
-        const T Kcd = a.ket[BRA_K * npp + idx];
-        GradFn<LA, LB, LC, LD>::ket(invq, QCx, QCy, QCz, QDx, QDy, QDz, gam, tk);
-        GradFn<LA, LB, LC, LD>::run(sbra[warp] + sb * BRA_SB, nbl, nsb * BRA_SB, q, Qx, Qy, Qz, Kcd, a.boys, tk, g);
-      }
-      wgt = (A == B ? T(1) : T(2)) * (C == Dd ? T(1) : T(2));
-    }
-#pragma unroll
-    for (int x = 0; x < 6; ++x) {
-      T v = wgt * g[x];
-#pragma unroll
-      for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-      if (lane == 0) atomicAdd(&a.grad[3 * a.shell_atom[x < 3 ? A : B] + x % 3], widen(v));
-    }
-    __syncwarp();
-  }
-}
-
-template <int LA, int LB, int LC, int LD, typename T>
-static gbhf_status launch_grad_class(gbhf_ctx* c, cudaStream_t strm, int combo, int prec, const T* D, const T* bra,
-                                     const T* ket, const T* boys, double* grad, int ntask) {
-  if (ntask <= 0) return GBHF_OK;
-  constexpr int NOUT = ncart_c(LA) * ncart_c(LB) * ncart_c(LC) * ncart_c(LD);
-  constexpr int NT = ncart_c(LA) * ncart_c(LB) * nherm_c(LC + LD);
-  constexpr bool SG = sizeof(T) == 8 ? NOUT > 9 : NOUT > 27;   // Gamma and T in shared memory
-  const size_t smem = SG ? (size_t)(NOUT + NT) * GR_THREADS * sizeof(T) : 0;
-  auto kern = k_grad_jk<LA, LB, LC, LD, T, SG>;
-  static bool attr_set = false;
-  if (SG && !attr_set) {
-    GBHF_CUDA(c, cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    attr_set = true;
-  }
-  int per_sm = 0;
-  GBHF_CUDA(c, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, GR_THREADS, smem));
-  per_sm = std::max(per_sm, 1);
-  const int grid = std::min(c->nsm * per_sm, (ntask + GR_WARPS - 1) / GR_WARPS);
-  PairData& P = c->pairs;
-  TaskLists& gt = c->gtasks;
-  GradArgs<T> a;
-  a.tasks = prec == 0 ? gt.tasks64.p : gt.tasks32.p;
-  a.range = gt.ranges.p + 4 * combo + 2 * prec;
-  a.counter = gt.counters.p + 2 * combo + prec;
-  a.pA = P.A.p;
-  a.pB = P.B.p;
-  a.pK = P.K.p;
-  a.poff = P.poff.p;
-  a.kseg = P.kseg.p;
-  a.seg = P.seg_info.p;
-  a.bra = bra;
-  a.ket = ket;
-  a.npp = (long long)P.nprim_pairs;
-  a.shell_f0 = c->tasks.f0.p;
-  a.shell_atom = c->tasks.atom.p;
-  a.pmol = P.mol.p;
-  a.mn = c->tasks.mn.p;
-  a.moff = c->tasks.moff.p;
-  a.D = D;
-  a.boys = boys;
-  a.grad = grad;
-  a.sscale = c->tasks.sscale.p;
-  a.Q = P.Q.p;
-  a.Qf = P.Qf.p;
-  a.thr = gt.thr_exact;
-  a.thrf = (float)gt.thr_exact;
-  a.jcoef = T(c->grad_jcoef);
-  kern<<<grid, GR_THREADS, smem, strm>>>(a);
-  count_launch(c);
-  GBHF_CUDA(c, cudaGetLastError());
-  return GBHF_OK;
-}
-
-template <typename T>
-static gbhf_status launch_grad_combo(gbhf_ctx* c, cudaStream_t strm, int k, int prec, const T* D, const T* bra,
-                                     const T* ket, const T* boys, double* grad, int nt) {
-  switch (k) {   // (bra class, ket class) = (k / 3, k % 3); class 0 = ss, 1 = ps, 2 = pp
-    case 0: return launch_grad_class<0, 0, 0, 0, T>(c, strm, k, prec, D, bra, ket, boys, grad, nt);
-    case 1: return launch_grad_class<0, 0, 1, 0, T>(c, strm, k, prec, D, bra, ket, boys, grad, nt);
-    case 2: return launch_grad_class<0, 0, 1, 1, T>(c, strm, k, prec, D, bra, ket, boys, grad, nt);
-    case 3: return launch_grad_class<1, 0, 0, 0, T>(c, strm, k, prec, D, bra, ket, boys, grad, nt);
-    case 4: return launch_grad_class<1, 0, 1, 0, T>(c, strm, k, prec, D, bra, ket, boys, grad, nt);
-    case 5: return launch_grad_class<1, 0, 1, 1, T>(c, strm, k, prec, D, bra, ket, boys, grad, nt);
-    case 6: return launch_grad_class<1, 1, 0, 0, T>(c, strm, k, prec, D, bra, ket, boys, grad, nt);
-    case 7: return launch_grad_class<1, 1, 1, 0, T>(c, strm, k, prec, D, bra, ket, boys, grad, nt);
-    case 8: return launch_grad_class<1, 1, 1, 1, T>(c, strm, k, prec, D, bra, ket, boys, grad, nt);
-    // combinations with a d pair on generated code (GRAD_COMBO_BRA / GRAD_COMBO_KET)
-    case 9: return launch_grad_class<0, 0, 2, 0, T>(c, strm, k, prec, D, bra, ket, boys, grad, nt);
-    case 10: return launch_grad_class<0, 0, 2, 1, T>(c, strm, k, prec, D, bra, ket, boys, grad, nt);
-    case 12: return launch_grad_class<1, 0, 2, 0, T>(c, strm, k, prec, D, bra, ket, boys, grad, nt);
-    case 18: return launch_grad_class<2, 0, 0, 0, T>(c, strm, k, prec, D, bra, ket, boys, grad, nt);
-    case 19: return launch_grad_class<2, 0, 1, 0, T>(c, strm, k, prec, D, bra, ket, boys, grad, nt);
-    default: return fail(c, GBHF_ERR_UNSUPPORTED, "no generated gradient kernel for combo " + std::to_string(k));
-  }
-}
 
 // Gradient combinations with a d pair evaluated by the generated lane-per-ket
 // code; the others go to the warp-per-quartet kernels of gradd.cu.
@@ -345,43 +44,45 @@ gbhf_status grad_2e(gbhf_ctx* c, const double* d_D, double schwarz, double mixed
   TaskLists& gt = c->gtasks;
   gt.thr_exact = schwarz;   // per-quartet Gamma test in the kernels
   const size_t nst = (size_t)c->basis.stacked;
-  bool any32 = false;
-  for (int k = 0; k < NCOMBO_MAX; ++k) any32 |= gt.hranges[4 * k + 3] > gt.hranges[4 * k + 2];
-  if (any32) {
+  int nts[NCOMBO_MAX][NTIER];
+  bool any[NTIER] = {};
+  for (int k = 0; k < NCOMBO_MAX; ++k)
+    for (int t = 0; t < NTIER; ++t) {
+      nts[k][t] = gt.hranges[2 * (NTIER * k + t) + 1] - gt.hranges[2 * (NTIER * k + t)];
+      any[t] |= nts[k][t] > 0;
+    }
+  if (any[TIER_32]) {
     GBHF_CUDA(c, c->dfloat.alloc(nst));
     GBHF_TRY(to_float(c, nst, d_D, c->dfloat.p));
   }
-  GBHF_CUDA(c, cudaMemsetAsync(gt.counters.p, 0, 2 * NCOMBO_MAX * sizeof(int), c->stream));
+  if (any[TIER_FF]) GBHF_TRY(to_ff(c, nst, d_D));
+  GBHF_CUDA(c, cudaMemsetAsync(gt.counters.p, 0, NTIER * NCOMBO_MAX * sizeof(int), c->stream));
   const bool ev = c->prof.events;
-  int ne = 0, ev_combo[2 * NCOMBO_MAX], ev_prec[2 * NCOMBO_MAX];
+  int ne = 0, ev_combo[NTIER * NCOMBO_MAX], ev_prec[NTIER * NCOMBO_MAX];
   if (ev) {
     GBHF_CUDA(c, cudaEventRecord(c->evg[0], c->stream));
   } else {
     GBHF_CUDA(c, cudaEventRecord(c->fork_ev, c->stream));
     for (int i = 0; i < gbhf_ctx::NSIDE_GRAD; ++i) GBHF_CUDA(c, cudaStreamWaitEvent(c->side[i], c->fork_ev, 0));
   }
-  PairData& P = c->pairs;
   int nl = 0;
   // heaviest first: the d combinations, then the s/p ones
   static const int order[NCOMBO_MAX] = {35, 34, 29, 33, 28, 23, 32, 27, 22, 17, 31, 26, 21, 16, 11, 30, 25, 20,
                                         15, 14, 10, 24, 19, 13, 9, 18, 12, 8, 7, 5, 6, 4, 2, 3, 1, 0};
-  for (int prec = 0; prec < 2; ++prec) {
-    if (prec == 1 && !any32) break;
+  static const int tiers[NTIER] = {TIER_64, TIER_FF, TIER_32};
+  for (const int tier : tiers) {
     for (int oi = 0; oi < NCOMBO_MAX; ++oi) {
       const int k = order[oi];
-      const int nt = gt.hranges[4 * k + 2 * prec + 1] - gt.hranges[4 * k + 2 * prec];
+      const int nt = nts[k][tier];
       if (nt <= 0) continue;
       cudaStream_t strm = ev ? c->stream : c->side[nl++ % gbhf_ctx::NSIDE_GRAD];
-      if (!grad_gen_combo(k))
-        GBHF_TRY(launch_grad_dclass(c, strm, k, prec, d_D, c->dfloat.p, d_grad, nt));
-      else if (prec == 0)
-        GBHF_TRY(launch_grad_combo<double>(c, strm, k, 0, d_D, P.bra64.p, P.ket64.p, c->boysh64.p, d_grad, nt));
-      else
-        GBHF_TRY(launch_grad_combo<float>(c, strm, k, 1, c->dfloat.p, P.bra32.p, P.ket32.p, c->boysh32.p, d_grad,
-                                          nt));
+      if (!grad_gen_combo(k)) GBHF_TRY(launch_grad_dclass(c, strm, k, tier, d_D, d_grad, nt));
+      else if (tier == TIER_64) GBHF_TRY(launch_grad_combo<double>(c, strm, k, tier, d_D, d_grad, nt));
+      else if (tier == TIER_32) GBHF_TRY(launch_grad_combo<float>(c, strm, k, tier, c->dfloat.p, d_grad, nt));
+      else GBHF_TRY(launch_grad_ff(c, strm, k, d_grad, nt));
       if (ev) {
         ev_combo[ne] = k;
-        ev_prec[ne] = prec;
+        ev_prec[ne] = tier == TIER_32 ? 1 : 0;   // two-float work counts as FP64 in the profile
         ++ne;
         GBHF_CUDA(c, cudaEventRecord(c->evg[ne], c->stream));
       }

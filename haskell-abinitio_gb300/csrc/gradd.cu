@@ -47,6 +47,8 @@ struct GradDArgs {
   double thr;            // drop a quartet when Q_ab Q_cd max|Gamma_abcd| is below
   double* grad;
   T jcoef;               // weight of the Coulomb term D_ab D_cd in Gamma (0: exchange only)
+  const float4* cen;     // two-float kernels: shell centres and the density's scale exponent (as k_jk)
+  const int* dexp;
 };
 
 template <int LA, int LB, int LC, int LD, typename T>
@@ -60,6 +62,14 @@ __global__ void __launch_bounds__(GRD_THREADS) k_gradd(GradDArgs<T> a) {
   T* ws = reinterpret_cast<T*>(grd_smem + GRD_TUV_BYTES) + warp * C::WS;
   T* sbra = ws + C::OFF_SB;
   T* Gam = ws + C::OFF_G;
+  constexpr bool FF = std::is_same<T, ff>::value;
+  using S = const_t<T>;
+  int dex = 0;          // two-float: Gamma is 2^-dex times the density's
+  double thr = a.thr;
+  if constexpr (FF) {
+    dex = 2 * *a.dexp;
+    thr = scalbn(thr, -dex);
+  }
   const int start = a.range[0], ntask = a.range[1] - start;
   const long long npp = a.npp;
   while (true) {
@@ -85,8 +95,8 @@ __global__ void __launch_bounds__(GRD_THREADS) k_gradd(GradDArgs<T> a) {
       const int jk = task.y + q;
       const int Cs = a.pA[jk], Ds = a.pB[jk];
       const int c0 = a.shell_f0[Cs], d0 = a.shell_f0[Ds];
-      const T wgt = (A == B ? T(1) : T(2)) * (Cs == Ds ? T(1) : T(2));
-      double gmax = 0.0;
+      const S wgt = (A == B ? S(1) : S(2)) * (Cs == Ds ? S(1) : S(2));
+      S gmax = S(0);
       for (int e = lane; e < C::NOUT; e += 32) {
         const int ab = e / C::NCD, cd = e - ab * C::NCD;
         const int ia = ab / C::NB, ibb = ab - ia * C::NB, ic = cd / C::ND, id = cd - ic * C::ND;
@@ -94,18 +104,20 @@ __global__ void __launch_bounds__(GRD_THREADS) k_gradd(GradDArgs<T> a) {
         const T dac = Dm[(long long)(a0 + ia) * n + c0 + ic], dbd = Dm[(long long)(b0 + ibb) * n + d0 + id];
         const T dad = Dm[(long long)(a0 + ia) * n + d0 + id], dbc = Dm[(long long)(b0 + ibb) * n + c0 + ic];
         const double sc = a.sscale[6 * A + ia] * a.sscale[6 * B + ibb] * a.sscale[6 * Cs + ic] * a.sscale[6 * Ds + id];
-        const T gv = (a.jcoef * dab * dcd - T(0.25) * (dac * dbd + dad * dbc)) * T(sc);
-        Gam[e] = gv * wgt;
-        gmax = fmax(gmax, fabs((double)gv));
+        const T gv = (a.jcoef * dab * dcd - S(0.25) * (dac * dbd + dad * dbc)) * T(sc);
+        Gam[e] = wgt * gv;
+        gmax = fmax_t(gmax, mag(gv));
       }
       __syncwarp();
       // exact screening of this quartet by its own Gamma (warp-uniform decision)
 #pragma unroll
-      for (int o = 16; o > 0; o >>= 1) gmax = fmax(gmax, __shfl_xor_sync(0xffffffffu, gmax, o));
-      if (a.Q[ib] * a.Q[jk] * gmax < a.thr) continue;
+      for (int o = 16; o > 0; o >>= 1) gmax = fmax_t(gmax, shfl_xor_t(gmax, o));
+      if (a.Q[ib] * a.Q[jk] * (double)gmax < thr) continue;
       const int4 sg = a.seg[a.kseg[jk]];
       const int K = sg.z, len = sg.y - sg.x;
       const long long base = (long long)sg.w + (jk - sg.x);
+      ff AC[3];
+      if constexpr (FF) md_centre(a.cen, A, Cs, AC);
       for (int kb = 0; kb < Kb; ++kb) {
         MDPrim<T> bp;
         md_row_prim(sbra + kb * BRA_SB, bp);
@@ -114,6 +126,7 @@ __global__ void __launch_bounds__(GRD_THREADS) k_gradd(GradDArgs<T> a) {
         for (int kc = 0; kc < K; ++kc) {
           MDPrim<T> kp;
           md_load_prim(a.ket, npp, base + (long long)kc * len, kp);
+          md_shift(bp, kp, AC);
           md_prim_x<C>(ws, tuv, bp, kp, a.boys, lane);
           md_bra_grad<C>(ws, tuv, ea, eb, g, lane);
           __syncwarp();
@@ -124,16 +137,16 @@ __global__ void __launch_bounds__(GRD_THREADS) k_gradd(GradDArgs<T> a) {
     for (int x = 0; x < 6; ++x) {
       T v = g[x];
 #pragma unroll
-      for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-      if (lane == 0) atomicAdd(&a.grad[3 * a.shell_atom[x < 3 ? A : B] + x % 3], widen(v));
+      for (int o = 16; o > 0; o >>= 1) v += shfl_xor_t(v, o);
+      if (lane == 0) atomicAdd(&a.grad[3 * a.shell_atom[x < 3 ? A : B] + x % 3], widen(v, dex));
     }
     __syncwarp();
   }
 }
 
 template <int LA, int LB, int LC, int LD, typename T>
-static gbhf_status launch_gradd_t(gbhf_ctx* c, cudaStream_t strm, int combo, int prec, const T* D, const T* bra,
-                                  const T* ket, const T* boys, double* grad, int ntask) {
+static gbhf_status launch_gradd_t(gbhf_ctx* c, cudaStream_t strm, int combo, int prec, const T* D, double* grad,
+                                  int ntask) {
   if (ntask <= 0) return GBHF_OK;
   using C = MDCfg<LA, LB, LC, LD, 1>;
   const size_t smem = GRD_TUV_BYTES + (size_t)GRD_WARPS * C::WS * sizeof(T);
@@ -150,16 +163,16 @@ static gbhf_status launch_gradd_t(gbhf_ctx* c, cudaStream_t strm, int combo, int
   PairData& P = c->pairs;
   TaskLists& gt = c->gtasks;
   GradDArgs<T> a;
-  a.tasks = prec == 0 ? gt.tasks64.p : gt.tasks32.p;
-  a.range = gt.ranges.p + 4 * combo + 2 * prec;
-  a.counter = gt.counters.p + 2 * combo + prec;
+  a.tasks = gt.tasks[prec].p;
+  a.range = gt.ranges.p + 2 * (NTIER * combo + prec);
+  a.counter = gt.counters.p + NTIER * combo + prec;
   a.pA = P.A.p;
   a.pB = P.B.p;
   a.poff = P.poff.p;
   a.kseg = P.kseg.p;
   a.seg = P.seg_info.p;
-  a.bra = bra;
-  a.ket = ket;
+  a.bra = pair_bra<T>(P);
+  a.ket = pair_ket<T>(P);
   a.npp = (long long)P.nprim_pairs;
   a.shell_f0 = c->tasks.f0.p;
   a.shell_atom = c->tasks.atom.p;
@@ -171,7 +184,9 @@ static gbhf_status launch_gradd_t(gbhf_ctx* c, cudaStream_t strm, int combo, int
   a.thr = gt.thr_exact;
   a.jcoef = T(c->grad_jcoef);
   a.D = D;
-  a.boys = boys;
+  a.boys = boys_table<T>(c);
+  a.cen = c->tasks.cen.p;
+  a.dexp = c->dff_exp.p;
   a.grad = grad;
   kern<<<grid, GRD_THREADS, smem, strm>>>(a);
   count_launch(c);
@@ -179,25 +194,19 @@ static gbhf_status launch_gradd_t(gbhf_ctx* c, cudaStream_t strm, int combo, int
   return GBHF_OK;
 }
 
-// Gradient combos 9..35: every ordered (bra class, ket class) with a d pair
-// class (3 = ds, 4 = dp, 5 = dd), in GRAD_COMBO_BRA / GRAD_COMBO_KET order.
+// The (bra class, ket class) combos without generated code (GRAD_COMBO_BRA /
+// GRAD_COMBO_KET; 3 = ds, 4 = dp, 5 = dd).
 template <typename T>
-static gbhf_status launch_gradd_combo(gbhf_ctx* c, cudaStream_t strm, int k, int prec, const T* D, const T* bra,
-                                      const T* ket, const T* boys, double* grad, int nt) {
+static gbhf_status launch_gradd_combo(gbhf_ctx* c, cudaStream_t strm, int k, int prec, const T* D, double* grad, int nt) {
 #define GBHF_GRD(K, la, lb, lc, ld) \
-  case K: return launch_gradd_t<la, lb, lc, ld, T>(c, strm, k, prec, D, bra, ket, boys, grad, nt);
+  case K: return launch_gradd_t<la, lb, lc, ld, T>(c, strm, k, prec, D, grad, nt);
   switch (k) {
-    GBHF_GRD(9, 0, 0, 2, 0)
-    GBHF_GRD(10, 0, 0, 2, 1)
     GBHF_GRD(11, 0, 0, 2, 2)
-    GBHF_GRD(12, 1, 0, 2, 0)
     GBHF_GRD(13, 1, 0, 2, 1)
     GBHF_GRD(14, 1, 0, 2, 2)
     GBHF_GRD(15, 1, 1, 2, 0)
     GBHF_GRD(16, 1, 1, 2, 1)
     GBHF_GRD(17, 1, 1, 2, 2)
-    GBHF_GRD(18, 2, 0, 0, 0)
-    GBHF_GRD(19, 2, 0, 1, 0)
     GBHF_GRD(20, 2, 0, 1, 1)
     GBHF_GRD(21, 2, 0, 2, 0)
     GBHF_GRD(22, 2, 0, 2, 1)
@@ -219,12 +228,11 @@ static gbhf_status launch_gradd_combo(gbhf_ctx* c, cudaStream_t strm, int k, int
 #undef GBHF_GRD
 }
 
-gbhf_status launch_grad_dclass(gbhf_ctx* c, cudaStream_t strm, int combo, int prec, const double* D64,
-                               const float* D32, double* grad, int ntask) {
-  PairData& P = c->pairs;
-  if (prec == 0)
-    return launch_gradd_combo<double>(c, strm, combo, 0, D64, P.bra64.p, P.ket64.p, c->boysh64.p, grad, ntask);
-  return launch_gradd_combo<float>(c, strm, combo, 1, D32, P.bra32.p, P.ket32.p, c->boysh32.p, grad, ntask);
+gbhf_status launch_grad_dclass(gbhf_ctx* c, cudaStream_t strm, int combo, int tier, const double* D64, double* grad,
+                               int ntask) {
+  if (tier == TIER_64) return launch_gradd_combo<double>(c, strm, combo, tier, D64, grad, ntask);
+  if (tier == TIER_32) return launch_gradd_combo<float>(c, strm, combo, tier, c->dfloat.p, grad, ntask);
+  return launch_gradd_combo<ff>(c, strm, combo, tier, c->dff.p, grad, ntask);
 }
 
 }  // namespace gbhf

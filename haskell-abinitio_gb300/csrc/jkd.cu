@@ -42,6 +42,8 @@ struct JKDArgs {
   int with_j;             // 0: exchange only
   const double* Q;        // Schwarz bound of each pair
   double thr;             // per-quartet screening on the six density blocks (as k_jk)
+  const float4* cen;      // two-float kernels: shell centres and the density's scale exponent (as k_jk)
+  const int* dexp;
 };
 
 template <int LA, int LB, int LC, int LD, typename T>
@@ -55,6 +57,14 @@ __global__ void __launch_bounds__(JKD_THREADS) k_jkd(JKDArgs<T> a) {
   T* ws = reinterpret_cast<T*>(jkd_smem + TUV_BYTES) + warp * C::WS;
   T* sbra = ws + C::OFF_SB;
   T* I = ws + C::OFF_R;   // contracted block for the scatter (R is free by then)
+  constexpr bool FF = std::is_same<T, ff>::value;
+  using S = const_t<T>;
+  int dex = 0;          // two-float: D is 2^-dex times the density
+  double thr = a.thr;
+  if constexpr (FF) {
+    dex = *a.dexp;
+    thr = scalbn(thr, -dex);
+  }
   const int start = a.range[0], ntask = a.range[1] - start;
   const long long npp = a.npp;
   unsigned long long cnt_q = 0, cnt_p = 0;
@@ -83,7 +93,7 @@ __global__ void __launch_bounds__(JKD_THREADS) k_jkd(JKDArgs<T> a) {
       const int Cs = a.pA[jk], Ds = a.pB[jk];
       const int c0 = a.shell_f0[Cs], d0 = a.shell_f0[Ds];
       {   // exact screening on the six density blocks of the quartet (as k_jk)
-        double dmx = 0.0;
+        S dmx = S(0);
         constexpr int NB6 = C::NAB + C::NCD + (C::NA + C::NB) * (C::NC + C::ND);
         for (int e = lane; e < NB6; e += 32) {
           int r, q2;
@@ -98,15 +108,17 @@ __global__ void __launch_bounds__(JKD_THREADS) k_jkd(JKDArgs<T> a) {
             r = rr < C::NA ? a0 + rr : b0 + (rr - C::NA);
             q2 = cc < C::NC ? c0 + cc : d0 + (cc - C::NC);
           }
-          dmx = fmax(dmx, fabs((double)Dm[(long long)r * n + q2]));
+          dmx = fmax_t(dmx, mag(Dm[(long long)r * n + q2]));
         }
 #pragma unroll
-        for (int o = 16; o > 0; o >>= 1) dmx = fmax(dmx, __shfl_xor_sync(0xffffffffu, dmx, o));
-        if (a.Q[ib] * a.Q[jk] * dmx < a.thr) continue;   // warp-uniform
+        for (int o = 16; o > 0; o >>= 1) dmx = fmax_t(dmx, shfl_xor_t(dmx, o));
+        if (a.Q[ib] * a.Q[jk] * (double)dmx < thr) continue;   // warp-uniform
       }
       const int4 sg = a.seg[a.kseg[jk]];
       const int K = sg.z, len = sg.y - sg.x;
       const long long base = (long long)sg.w + (jk - sg.x);
+      ff AC[3];
+      if constexpr (FF) md_centre(a.cen, A, Cs, AC);
       T acc[C::NPL];
 #pragma unroll
       for (int k = 0; k < C::NPL; ++k) acc[k] = T(0);
@@ -117,6 +129,7 @@ __global__ void __launch_bounds__(JKD_THREADS) k_jkd(JKDArgs<T> a) {
         for (int kc = 0; kc < K; ++kc) {
           MDPrim<T> kp;
           md_load_prim(a.ket, npp, base + (long long)kc * len, kp);
+          md_shift(bp, kp, AC);
           md_prim_x<C>(ws, tuv, bp, kp, a.boys, lane);
           md_bra_acc<C>(ws, acc, lane);
           __syncwarp();
@@ -125,7 +138,7 @@ __global__ void __launch_bounds__(JKD_THREADS) k_jkd(JKDArgs<T> a) {
       cnt_q += kb0 == 0;
       cnt_p += (unsigned long long)Kb * K;
       // ---- scatter into G'' (as k_jk), with the d-component scales
-      const T s = (A == B ? T(0.5) : T(1)) * (Cs == Ds ? T(0.5) : T(1)) * (ib == jk ? T(0.5) : T(1));
+      const S s = (A == B ? S(0.5) : S(1)) * (Cs == Ds ? S(0.5) : S(1)) * (ib == jk ? S(0.5) : S(1));
 #pragma unroll
       for (int k = 0; k < C::NPL; ++k) {
         const int e = lane + 32 * k;
@@ -144,7 +157,7 @@ __global__ void __launch_bounds__(JKD_THREADS) k_jkd(JKDArgs<T> a) {
           const int ic = cd / C::ND, id = cd - ic * C::ND;
           v = fma_t(I[ab * C::NCD + cd], Dm[(long long)(c0 + ic) * n + d0 + id], v);
         }
-        atomicAdd(&Gm[(long long)(a0 + ia) * n + b0 + ibb], widen(T(2) * v));
+        atomicAdd(&Gm[(long long)(a0 + ia) * n + b0 + ibb], widen(S(2) * v, dex));
       }
       for (int cd = lane; a.with_j && cd < C::NCD; cd += 32) {   // J_cd += 2 sum_ab v D_ab
         const int ic = cd / C::ND, id = cd - ic * C::ND;
@@ -153,7 +166,7 @@ __global__ void __launch_bounds__(JKD_THREADS) k_jkd(JKDArgs<T> a) {
           const int ia = ab / C::NB, ibb = ab - ia * C::NB;
           v = fma_t(I[ab * C::NCD + cd], Dm[(long long)(a0 + ia) * n + b0 + ibb], v);
         }
-        atomicAdd(&Gm[(long long)(c0 + ic) * n + d0 + id], widen(T(2) * v));
+        atomicAdd(&Gm[(long long)(c0 + ic) * n + d0 + id], widen(S(2) * v, dex));
       }
       for (int e = lane; e < C::NA * C::NC; e += 32) {   // K_ac -= 1/2 sum_bd v D_bd
         const int ia = e / C::NC, ic = e - ia * C::NC;
@@ -161,7 +174,7 @@ __global__ void __launch_bounds__(JKD_THREADS) k_jkd(JKDArgs<T> a) {
         for (int ibb = 0; ibb < C::NB; ++ibb)
           for (int id = 0; id < C::ND; ++id)
             v = fma_t(I[(ia * C::NB + ibb) * C::NCD + ic * C::ND + id], Dm[(long long)(b0 + ibb) * n + d0 + id], v);
-        atomicAdd(&Gm[(long long)(a0 + ia) * n + c0 + ic], widen(T(-0.5) * v));
+        atomicAdd(&Gm[(long long)(a0 + ia) * n + c0 + ic], widen(S(-0.5) * v, dex));
       }
       for (int e = lane; e < C::NA * C::ND; e += 32) {   // K_ad -= 1/2 sum_bc v D_bc
         const int ia = e / C::ND, id = e - ia * C::ND;
@@ -169,7 +182,7 @@ __global__ void __launch_bounds__(JKD_THREADS) k_jkd(JKDArgs<T> a) {
         for (int ibb = 0; ibb < C::NB; ++ibb)
           for (int ic = 0; ic < C::NC; ++ic)
             v = fma_t(I[(ia * C::NB + ibb) * C::NCD + ic * C::ND + id], Dm[(long long)(b0 + ibb) * n + c0 + ic], v);
-        atomicAdd(&Gm[(long long)(a0 + ia) * n + d0 + id], widen(T(-0.5) * v));
+        atomicAdd(&Gm[(long long)(a0 + ia) * n + d0 + id], widen(S(-0.5) * v, dex));
       }
       for (int e = lane; e < C::NB * C::NC; e += 32) {   // K_bc -= 1/2 sum_ad v D_ad
         const int ibb = e / C::NC, ic = e - ibb * C::NC;
@@ -177,7 +190,7 @@ __global__ void __launch_bounds__(JKD_THREADS) k_jkd(JKDArgs<T> a) {
         for (int ia = 0; ia < C::NA; ++ia)
           for (int id = 0; id < C::ND; ++id)
             v = fma_t(I[(ia * C::NB + ibb) * C::NCD + ic * C::ND + id], Dm[(long long)(a0 + ia) * n + d0 + id], v);
-        atomicAdd(&Gm[(long long)(b0 + ibb) * n + c0 + ic], widen(T(-0.5) * v));
+        atomicAdd(&Gm[(long long)(b0 + ibb) * n + c0 + ic], widen(S(-0.5) * v, dex));
       }
       for (int e = lane; e < C::NB * C::ND; e += 32) {   // K_bd -= 1/2 sum_ac v D_ac
         const int ibb = e / C::ND, id = e - ibb * C::ND;
@@ -185,7 +198,7 @@ __global__ void __launch_bounds__(JKD_THREADS) k_jkd(JKDArgs<T> a) {
         for (int ia = 0; ia < C::NA; ++ia)
           for (int ic = 0; ic < C::NC; ++ic)
             v = fma_t(I[(ia * C::NB + ibb) * C::NCD + ic * C::ND + id], Dm[(long long)(a0 + ia) * n + c0 + ic], v);
-        atomicAdd(&Gm[(long long)(b0 + ibb) * n + d0 + id], widen(T(-0.5) * v));
+        atomicAdd(&Gm[(long long)(b0 + ibb) * n + d0 + id], widen(S(-0.5) * v, dex));
       }
       __syncwarp();
     }
@@ -198,8 +211,8 @@ __global__ void __launch_bounds__(JKD_THREADS) k_jkd(JKDArgs<T> a) {
 }
 
 template <int LA, int LB, int LC, int LD, typename T>
-static gbhf_status launch_jkd_t(gbhf_ctx* c, cudaStream_t strm, int combo, int prec, const T* D, double* G,
-                                const T* bra, const T* ket, const T* boys, int ntask, int with_j) {
+static gbhf_status launch_jkd_t(gbhf_ctx* c, cudaStream_t strm, int combo, int prec, const T* D, double* G, int ntask,
+                                int with_j) {
   if (ntask <= 0) return GBHF_OK;
   using C = MDCfg<LA, LB, LC, LD, 0>;
   const size_t smem = TUV_BYTES + (size_t)JKD_WARPS * C::WS * sizeof(T);
@@ -215,16 +228,16 @@ static gbhf_status launch_jkd_t(gbhf_ctx* c, cudaStream_t strm, int combo, int p
   const int grid = std::min(c->nsm * per_sm, (ntask + JKD_WARPS - 1) / JKD_WARPS);
   PairData& P = c->pairs;
   JKDArgs<T> a;
-  a.tasks = prec == 0 ? c->tasks.tasks64.p : c->tasks.tasks32.p;
-  a.range = c->tasks.ranges.p + 4 * combo + 2 * prec;
-  a.counter = c->tasks.counters.p + 2 * combo + prec;
+  a.tasks = c->tasks.tasks[prec].p;
+  a.range = c->tasks.ranges.p + 2 * (NTIER * combo + prec);
+  a.counter = c->tasks.counters.p + NTIER * combo + prec;
   a.pA = P.A.p;
   a.pB = P.B.p;
   a.poff = P.poff.p;
   a.kseg = P.kseg.p;
   a.seg = P.seg_info.p;
-  a.bra = bra;
-  a.ket = ket;
+  a.bra = pair_bra<T>(P);
+  a.ket = pair_ket<T>(P);
   a.npp = (long long)P.nprim_pairs;
   a.shell_f0 = c->tasks.f0.p;
   a.pmol = P.mol.p;
@@ -233,11 +246,13 @@ static gbhf_status launch_jkd_t(gbhf_ctx* c, cudaStream_t strm, int combo, int p
   a.sscale = c->tasks.sscale.p;
   a.D = D;
   a.G = G;
-  a.boys = boys;
-  a.stats = c->tasks.stats.p + 3 * (2 * combo + prec);
+  a.boys = boys_table<T>(c);
+  a.stats = c->tasks.stats.p + 3 * (NTIER * combo + prec);
   a.with_j = with_j;
   a.Q = P.Q.p;
   a.thr = c->tasks.thr_exact;
+  a.cen = c->tasks.cen.p;
+  a.dexp = c->dff_exp.p;
   kern<<<grid, JKD_THREADS, smem, strm>>>(a);
   count_launch(c);
   GBHF_CUDA(c, cudaGetLastError());
@@ -245,21 +260,14 @@ static gbhf_status launch_jkd_t(gbhf_ctx* c, cudaStream_t strm, int combo, int p
 }
 
 template <typename T>
-static gbhf_status launch_jkd_combo(gbhf_ctx* c, cudaStream_t strm, int k, int prec, const T* D, double* G,
-                                    const T* bra, const T* ket, const T* boys, int nt, int wj) {
+static gbhf_status launch_jkd_combo(gbhf_ctx* c, cudaStream_t strm, int k, int prec, const T* D, double* G, int nt,
+                                    int wj) {
 #define GBHF_JKD(K, la, lb, lc, ld) \
-  case K: return launch_jkd_t<la, lb, lc, ld, T>(c, strm, k, prec, D, G, bra, ket, boys, nt, wj);
-  switch (k) {   // COMBO_BRA / COMBO_KET 6..20; class 3 = ds, 4 = dp, 5 = dd
-    GBHF_JKD(6, 2, 0, 0, 0)
-    GBHF_JKD(7, 2, 0, 1, 0)
-    GBHF_JKD(8, 2, 0, 1, 1)
-    GBHF_JKD(9, 2, 0, 2, 0)
-    GBHF_JKD(10, 2, 1, 0, 0)
-    GBHF_JKD(11, 2, 1, 1, 0)
+  case K: return launch_jkd_t<la, lb, lc, ld, T>(c, strm, k, prec, D, G, nt, wj);
+  switch (k) {   // COMBO_BRA / COMBO_KET without generated code; class 3 = ds, 4 = dp, 5 = dd
     GBHF_JKD(12, 2, 1, 1, 1)
     GBHF_JKD(13, 2, 1, 2, 0)
     GBHF_JKD(14, 2, 1, 2, 1)
-    GBHF_JKD(15, 2, 2, 0, 0)
     GBHF_JKD(16, 2, 2, 1, 0)
     GBHF_JKD(17, 2, 2, 1, 1)
     GBHF_JKD(18, 2, 2, 2, 0)
@@ -270,12 +278,11 @@ static gbhf_status launch_jkd_combo(gbhf_ctx* c, cudaStream_t strm, int k, int p
 #undef GBHF_JKD
 }
 
-gbhf_status launch_jk_dclass(gbhf_ctx* c, cudaStream_t strm, int combo, int prec, const double* D64,
-                             const float* D32, double* G, int ntask, int with_j) {
-  PairData& P = c->pairs;
-  if (prec == 0)
-    return launch_jkd_combo<double>(c, strm, combo, 0, D64, G, P.bra64.p, P.ket64.p, c->boysh64.p, ntask, with_j);
-  return launch_jkd_combo<float>(c, strm, combo, 1, D32, G, P.bra32.p, P.ket32.p, c->boysh32.p, ntask, with_j);
+gbhf_status launch_jk_dclass(gbhf_ctx* c, cudaStream_t strm, int combo, int tier, const double* D64, double* G,
+                             int ntask, int with_j) {
+  if (tier == TIER_64) return launch_jkd_combo<double>(c, strm, combo, tier, D64, G, ntask, with_j);
+  if (tier == TIER_32) return launch_jkd_combo<float>(c, strm, combo, tier, c->dfloat.p, G, ntask, with_j);
+  return launch_jkd_combo<ff>(c, strm, combo, tier, c->dff.p, G, ntask, with_j);
 }
 
 // --------------------------------------------------------- Schwarz bounds ----

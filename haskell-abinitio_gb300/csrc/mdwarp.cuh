@@ -294,7 +294,7 @@ __device__ __forceinline__ void md_load_prim(const T* __restrict__ base, long lo
   pr.invp = base[BRA_INVP * npp + idx];
 #pragma unroll
   for (int x = 0; x < 3; ++x) {
-    pr.P[x] = base[(BRA_PX + x) * npp + idx];
+    if constexpr (!std::is_same<T, ff>::value) pr.P[x] = base[(BRA_PX + x) * npp + idx];
     pr.PA[x] = base[(BRA_PAX + x) * npp + idx];
     pr.PB[x] = base[(BRA_PBX + x) * npp + idx];
   }
@@ -308,11 +308,31 @@ __device__ __forceinline__ void md_row_prim(const T* __restrict__ row, MDPrim<T>
   pr.invp = row[BRA_INVP];
 #pragma unroll
   for (int x = 0; x < 3; ++x) {
-    pr.P[x] = row[BRA_PX + x];
+    if constexpr (!std::is_same<T, ff>::value) pr.P[x] = row[BRA_PX + x];
     pr.PA[x] = row[BRA_PAX + x];
     pr.PB[x] = row[BRA_PBX + x];
   }
   pr.K = row[BRA_K];
+}
+
+// Two-float values: both centres of a primitive quartet relative to the bra's
+// first centre A, P - A and Q - A = (Q - C) - (A - C).
+__device__ __forceinline__ void md_centre(const float4* __restrict__ cen, int A, int C, ff* AC) {
+  const float4 a0 = cen[3 * A], a1 = cen[3 * A + 1], a2 = cen[3 * A + 2];
+  const float4 c0 = cen[3 * C], c1 = cen[3 * C + 1], c2 = cen[3 * C + 2];
+  AC[0] = diff3(a0.x, a1.x, a2.x, c0.x, c1.x, c2.x);
+  AC[1] = diff3(a0.y, a1.y, a2.y, c0.y, c1.y, c2.y);
+  AC[2] = diff3(a0.z, a1.z, a2.z, c0.z, c1.z, c2.z);
+}
+template <typename T>
+__device__ __forceinline__ void md_shift(MDPrim<T>& bp, MDPrim<T>& kp, const ff* AC) {
+  if constexpr (std::is_same<T, ff>::value) {
+#pragma unroll
+    for (int x = 0; x < 3; ++x) {
+      bp.P[x] = bp.PA[x];
+      kp.P[x] = nrm(kp.PA[x] - AC[x]);
+    }
+  }
 }
 
 }  // namespace gbhf

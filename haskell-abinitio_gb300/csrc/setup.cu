@@ -253,6 +253,41 @@ static BoysHostTables build_boys_host_tables() {
   return bt;
 }
 
+// The two-float Horner table (BOYSFF_*), built and uploaded when a basis first
+// uses it: small molecules never do.
+static std::vector<float> build_boys_ff_table() {
+  std::vector<float> hff((size_t)(BOYSH_LMAX + 1) * BOYSFF_NROW * BOYSFF_STRIDE, 0.0f);
+  for (int j = 0; j < BOYSFF_NROW; ++j) {
+    double f[BOYS_NCOL];
+    const double tj = (double)j * BOYSFF_H;
+    boys_row_host(tj, f);
+    for (int L = 0; L <= BOYSH_LMAX; ++L) {
+      float* row = hff.data() + ((size_t)L * BOYSFF_NROW + j) * BOYSFF_STRIDE;
+      auto split = [](double x, float* o) {
+        o[0] = (float)x;
+        o[1] = (float)(x - (double)o[0]);
+      };
+      double fact = 1.0;
+      for (int k = 0; k < 4; ++k) {
+        if (k > 0) fact *= k;
+        split(f[L + k] / fact, row + 2 * k);
+      }
+      row[8] = (float)(f[L + 4] / 24.0);
+      row[9] = (float)(f[L + 5] / 120.0);
+      split(std::exp(-tj), row + 10);
+    }
+  }
+  return hff;
+}
+
+static gbhf_status ensure_boys_ff(gbhf_ctx* c) {
+  if (c->boyshff.p) return GBHF_OK;
+  static const std::vector<float> hff = build_boys_ff_table();   // once per process, thread-safe
+  GBHF_CUDA(c, c->boyshff.alloc(hff.size() / 4));
+  GBHF_CUDA(c, cudaMemcpyAsync(c->boyshff.p, hff.data(), hff.size() * sizeof(float), cudaMemcpyHostToDevice, c->stream));
+  return GBHF_OK;
+}
+
 static const BoysHostTables& boys_host_tables() {
   static const BoysHostTables bt = build_boys_host_tables();   // thread-safe one-time initialisation
   return bt;
@@ -330,7 +365,8 @@ __global__ void k_pair_layouts(int np, const int* __restrict__ pA, const int* __
                                const int4* __restrict__ seg, const int4* __restrict__ sh,
                                const double* __restrict__ xyz, const double* __restrict__ coef,
                                const double* __restrict__ expo, long long npp, double* __restrict__ bra64,
-                               double* __restrict__ ket64, float* __restrict__ bra32, float* __restrict__ ket32) {
+                               double* __restrict__ ket64, float* __restrict__ bra32, float* __restrict__ ket32,
+                               ff* __restrict__ braff, ff* __restrict__ ketff) {
   const int t = blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= np) return;
   const int A = pA[t], B = pB[t];
@@ -347,7 +383,44 @@ __global__ void k_pair_layouts(int np, const int* __restrict__ pA, const int* __
       bra32[(long long)fl * npp + bi] = (float)f[fl];
       ket32[(long long)fl * npp + ki] = (float)f[fl];
     }
+    if (!braff) continue;
+    // two-float values, with P - A = (b/p)(B - A) and P - B = (a/p)(A - B), whose
+    // errors scale with their size (P itself is not used there)
+    const double fb = (f[BRA_P] - f[BRA_AEXP]) * f[BRA_INVP], fa = f[BRA_AEXP] * f[BRA_INVP];
+    for (int x = 0; x < 3; ++x) {
+      const double ab = xyz[3 * sh[A].x + x] - xyz[3 * sh[B].x + x];
+      f[BRA_PAX + x] = -fb * ab;
+      f[BRA_PBX + x] = fa * ab;
+    }
+    for (int fl = 0; fl < BRA_NFIELD; ++fl) {
+      braff[(long long)fl * npp + bi] = ff(f[fl]);
+      ketff[(long long)fl * npp + ki] = ff(f[fl]);
+    }
   }
+}
+
+// Per molecule the Schwarz product Q_ab Q_cd below which a quartet runs in two
+// floats also where FP64 is asked for: 2^-5 of the molecule's largest.  There the
+// two-float error, 2^-45 of the quartet, is 2^-50 of the largest quartet, the size
+// of the FP64 rounding (2^-53 a term) and Boys remainder (5e-15) of the large
+// ones that stay in FP64.  0 (never) below 512 primitive pairs, where a build is
+// a handful of tasks and the extra launches cost more than the arithmetic saves
+// (SCF + gradient of a water, 250 pairs: 11.0 -> 11.5 ms with the two-float
+// lists; the dimer's Fock build, 1000 pairs: 377 -> 188 us), and when an exponent, a coefficient or a
+// coordinate is outside the range that FP32 exponents leave for the products.
+static std::vector<double> ff_limits(const Basis& b, const PairData& P) {
+  bool range = true;
+  for (double e : b.prim_exp) range &= e >= 1e-8 && e <= 1e8;
+  for (double k : b.prim_coef) range &= std::fabs(k) <= 1e8;
+  for (double x : b.xyz) range &= std::fabs(x) <= 1e5;
+  std::vector<double> lim(b.nmol, 0.0);
+  if (!range || P.nprim_pairs < 512) return lim;
+  for (int t = 0; t < P.npairs; ++t) {
+    double& q = lim[b.shells[P.hA[t]].mol];
+    q = std::max(q, P.hQ[t]);
+  }
+  for (double& q : lim) q = q * q / 32;
+  return lim;
 }
 
 gbhf_status ensure_pairs(gbhf_ctx* c) {
@@ -554,6 +627,13 @@ gbhf_status ensure_pairs(gbhf_ctx* c) {
   GBHF_CUDA(c, P.ket64.alloc(nf));
   GBHF_CUDA(c, P.bra32.alloc(nf));
   GBHF_CUDA(c, P.ket32.alloc(nf));
+  const std::vector<double> ffq = ff_limits(b, P);
+  const bool use_ff = *std::max_element(ffq.begin(), ffq.end()) > 0;
+  if (use_ff) {
+    GBHF_TRY(ensure_boys_ff(c));
+    GBHF_CUDA(c, P.braff.alloc(nf));
+    GBHF_CUDA(c, P.ketff.alloc(nf));
+  }
   auto up = [&](void* d, const void* h, size_t bytes) {
     return cudaMemcpyAsync(d, h, bytes, cudaMemcpyHostToDevice, c->stream);
   };
@@ -566,13 +646,16 @@ gbhf_status ensure_pairs(gbhf_ctx* c) {
   std::vector<float> qf(P.hQ.begin(), P.hQ.end());
   GBHF_CUDA(c, P.Qf.alloc(std::max(np, 1)));
   GBHF_CUDA(c, up(P.Qf.p, qf.data(), np * sizeof(float)));
+  GBHF_CUDA(c, P.ffq.alloc(ffq.size()));
+  GBHF_CUDA(c, up(P.ffq.p, ffq.data(), ffq.size() * sizeof(double)));
   GBHF_CUDA(c, up(P.seg_info.p, seginfo.data(), seginfo.size() * sizeof(int4)));
   GBHF_CUDA(c, up(P.mol.p, pmol.data(), np * sizeof(int)));
   GBHF_CUDA(c, up(P.mseg.p, P.hmseg.data(), P.hmseg.size() * sizeof(int)));
   if (np > 0) {
     k_pair_layouts<<<(np + 127) / 128, 128, 0, c->stream>>>(np, P.A.p, P.B.p, P.poff.p, P.kseg.p, P.seg_info.p, dsh.p,
                                                             c->d_xyz.p, c->d_coef.p, c->d_exp.p, (long long)npp,
-                                                            P.bra64.p, P.ket64.p, P.bra32.p, P.ket32.p);
+                                                            P.bra64.p, P.ket64.p, P.bra32.p, P.ket32.p, use_ff ? P.braff.p : nullptr,
+                                                            use_ff ? P.ketff.p : nullptr);
     count_launch(c);
     GBHF_CUDA(c, cudaGetLastError());
   }

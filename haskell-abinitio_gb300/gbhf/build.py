@@ -17,11 +17,12 @@ CSRC = PKG.parent / "csrc"
 BUILD = PKG / "_build"
 LIB = BUILD / "libgbhf.so"
 ARCH = ["-gencode", "arch=compute_103a,code=sm_103a"]
-SOURCES = ["api.cu", "setup.cu", "eri_canon.cu", "jk.cu", "linalg.cu", "scf.cu", "measure.cu", "noalloc.cu", "grad.cu", "batch.cu",
-           "sad.cu", "bscf.cu", "jkd.cu", "gradd.cu", "uhf.cu",
+SOURCES = ["jk.cu", "grad_ff.cu", "jk_ff.cu", "grad.cu", "jkd.cu", "gradd.cu", "api.cu", "setup.cu", "eri_canon.cu", "linalg.cu", "scf.cu", "measure.cu", "noalloc.cu", "batch.cu",
+           "sad.cu", "bscf.cu", "uhf.cu",
            "tune.cu", "tridiag.cu"]
-HEADERS = ["gbhf_common.cuh", "gbhf_internal.h", "gbhf_md.cuh", "eri_gen.cuh", "grad_gen.cuh", "jacobi.cuh",
-           "dense.cuh", "mdwarp.cuh"]
+HEADERS = ["gbhf_common.cuh", "gbhf_ff.cuh", "gbhf_internal.h", "gbhf_md.cuh", "eri_gen.cuh", "grad_gen.cuh", "jacobi.cuh",
+           "dense.cuh", "mdwarp.cuh", "jk_kern.cuh",
+           "grad_kern.cuh"]
 
 
 def nvcc():
