@@ -84,9 +84,7 @@ gbhf_status gbhf_create(gbhf_ctx** out, int device) {
     return GBHF_ERR_CUDA;
   }
   for (auto& e : c->ev) cudaEventCreate(&e);
-  for (auto& e : c->evc) cudaEventCreate(&e);
   for (auto& e : c->evu) cudaEventCreate(&e);
-  for (auto& e : c->evg) cudaEventCreate(&e);
   for (auto& e : c->evp) cudaEventCreate(&e);
   default_budgets(c, 0);
   default_budgets(c, 1);
@@ -613,8 +611,20 @@ gbhf_status gbhf_autotune(gbhf_ctx* c, int which, int precision, double schwarz_
   return autotune_dev(c, which, D, precision, schwarz_cutoff, mc, repeats, class_ms);
 }
 
+namespace gbhf {
+// The launch boundaries of the profiling builds, created with the first of them.
+gbhf_status ensure_profile_events(gbhf_ctx* c) {
+  for (auto& e : c->evc)
+    if (!e) GBHF_CUDA(c, cudaEventCreate(&e));
+  for (auto& e : c->evg)
+    if (!e) GBHF_CUDA(c, cudaEventCreate(&e));
+  return GBHF_OK;
+}
+}  // namespace gbhf
+
 gbhf_status gbhf_profile_reset(gbhf_ctx* c, int enable_events) {
   CTX_CHECK(c);
+  if (enable_events) GBHF_TRY(ensure_profile_events(c));
   GBHF_TRY(flush_jk_stats(c));   // counts of earlier builds go with the old profile
   c->prof = Profile();
   c->prof.events = enable_events != 0;

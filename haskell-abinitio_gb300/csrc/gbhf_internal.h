@@ -170,6 +170,9 @@ constexpr int GRAD_COMBO_KET[NCOMBO_MAX] = {0, 1, 2, 0, 1, 2, 0, 1, 2, 3, 4, 5, 
 // precision) and two-float (gbhf_ff.cuh; the part of the FP64 work whose bound
 // allows it).
 constexpr int NTIER = 3;
+// Below this many primitive pairs a build is a handful of tasks: its time is
+// launches, so it runs without two-float lists and density screening.
+constexpr size_t SMALL_PRIM_PAIRS = 512;
 constexpr int TIER_64 = 0, TIER_32 = 1, TIER_FF = 2;
 
 struct Segment {
@@ -208,7 +211,8 @@ struct PairData {
   std::vector<double> hQ;
   DBuf<int> A, B, K, poff, kseg;             // kseg: segment index (global list)
   DBuf<double> Q;
-  DBuf<float> Qf;                  // Q in FP32 (the FP32 kernels' per-quartet density test)
+  DBuf<float> Qf;                  // Q rounded up to FP32 (the per-quartet density test)
+  DBuf<int4> pinfo;                // per pair: shells A, B and their first functions within the molecule
   DBuf<int4> seg_info;                       // (start, end, K, data_off) per segment, all classes
   int nseg_total = 0;
   int seg_cls_start[NPCLS + 1] = {};
@@ -223,6 +227,7 @@ struct PairData {
   DBuf<float> bra32, ket32;
   DBuf<ff> braff, ketff;       // two-float values; Px, Py, Pz unused (P - A stands for P)
   DBuf<double> ffq;            // per molecule: two-float below this Q_ab Q_cd (0: never)
+  bool use_ff = false;         // some molecule's limit is above 0
   size_t nprim_pairs = 0;
 };
 
@@ -254,6 +259,11 @@ struct TaskLists {
   DBuf<int> amol;                      // per atom: molecule
   DBuf<int> mfo, mao;                  // per molecule: first function, first atom (nmol+1)
   DBuf<double> row, pw, pb, sw;        // density weights (incremental builds, gradient)
+  DBuf<float> Ds, pbf;                 // largest |D| per shell block and per pair (per-quartet screening)
+  bool screened = false;               // they belong to the current build's density
+  DBuf<int> ms0;                       // per molecule: first shell (nmol+1)
+  DBuf<long long> soff;                // per molecule: offset of its ns_m x ns_m block in Ds
+  size_t ds_size = 0;
   long f0_gen = -1;                    // basis generation f0 was uploaded for
 };
 
@@ -345,7 +355,6 @@ struct gbhf_ctx {
   gbhf::DBuf<float> dfloat;
   gbhf::DBuf<gbhf::ff> dff;         // density of the two-float kernels, scaled by 2^-e
   gbhf::DBuf<int> dff_exp;          // e
-  gbhf::DBuf<double> dff_max;       // max |D| of it
   gbhf::DBuf<int> dev_status;
   int purify_grid = 0;              // co-resident blocks of the fused purification kernel
   int tc2_grid = 0;                 // co-resident blocks of the one-barrier TC2 kernel
@@ -542,6 +551,7 @@ gbhf_status sad_density(gbhf_ctx* c, double* d_D);
 // autotuner, and the two-electron gradient alone (for the autotuner).
 void default_budgets(gbhf_ctx* c, int which);
 bool lane_per_ket(int which, int k);
+gbhf_status ensure_profile_events(gbhf_ctx* c);   // api.cu
 gbhf_status autotune_dev(gbhf_ctx* c, int which, const double* d_D, int precision, double schwarz,
                          double mixed_cutoff, int reps, double* class_ms);
 gbhf_status gradient_uhf_dev(gbhf_ctx* c, const double* d_Da, const double* d_Db, const double* d_W, double schwarz,
@@ -569,8 +579,6 @@ constexpr int PURIFY_REC = 12;
 gbhf_status purify_finish(gbhf_ctx* c, const double* rec);
 gbhf_status purify_flush(gbhf_ctx* c);
 gbhf_status max_abs_dev(gbhf_ctx* c, size_t n, const double* d_x, double* d_out);   // into device memory
-gbhf_status to_float(gbhf_ctx* c, size_t n, const double* d_x, float* d_y);
-gbhf_status to_ff(gbhf_ctx* c, size_t n, const double* d_x);   // into c->dff, c->dff_exp
 
 // Primitive-pair data and Boys table of a kernel's value type.
 template <typename T> inline const T* pair_bra(const PairData& P) {

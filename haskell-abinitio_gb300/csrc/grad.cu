@@ -43,20 +43,10 @@ gbhf_status grad_2e(gbhf_ctx* c, const double* d_D, double schwarz, double mixed
   GBHF_TRY(build_grad_tasks(c, d_D, schwarz, mixed_cutoff, precision));
   TaskLists& gt = c->gtasks;
   gt.thr_exact = schwarz;   // per-quartet Gamma test in the kernels
-  const size_t nst = (size_t)c->basis.stacked;
   int nts[NCOMBO_MAX][NTIER];
-  bool any[NTIER] = {};
   for (int k = 0; k < NCOMBO_MAX; ++k)
-    for (int t = 0; t < NTIER; ++t) {
+    for (int t = 0; t < NTIER; ++t)
       nts[k][t] = gt.hranges[2 * (NTIER * k + t) + 1] - gt.hranges[2 * (NTIER * k + t)];
-      any[t] |= nts[k][t] > 0;
-    }
-  if (any[TIER_32]) {
-    GBHF_CUDA(c, c->dfloat.alloc(nst));
-    GBHF_TRY(to_float(c, nst, d_D, c->dfloat.p));
-  }
-  if (any[TIER_FF]) GBHF_TRY(to_ff(c, nst, d_D));
-  GBHF_CUDA(c, cudaMemsetAsync(gt.counters.p, 0, NTIER * NCOMBO_MAX * sizeof(int), c->stream));
   const bool ev = c->prof.events;
   int ne = 0, ev_combo[NTIER * NCOMBO_MAX], ev_prec[NTIER * NCOMBO_MAX];
   if (ev) {

@@ -314,21 +314,30 @@ __global__ void k_ranges(int ncombo, int n, const int* item_combo_start, const i
   }
 }
 
-// Density weights for incremental builds and the gradient: per shell its row
-// maximum of |D| over its molecule's functions, per pair w = max(block max of
-// the pair, row A, row B) and the block max alone, per ket segment the largest
-// block max of its pairs.
-__global__ void k_shell_rowmax(int ns, const int* __restrict__ f0, const int* __restrict__ nc,
-                               const int* __restrict__ smol, const int* __restrict__ mn,
-                               const long long* __restrict__ moff, const double* __restrict__ D,
-                               double* __restrict__ row) {
+// Density maxima.  Per shell block the largest |D| (Ds, rounded up to FP32, for
+// the per-quartet screening), per shell its row maximum over the molecule's
+// functions; per pair the block maximum (FP32 for the screening) and, for the
+// task lists of incremental builds and the gradient, w = max(block, row A, row
+// B) and the block maximum, and per ket segment the largest block maximum.
+__global__ void k_shell_dmax(int ns, const int* __restrict__ f0, const int* __restrict__ nc,
+                             const int* __restrict__ smol, const int* __restrict__ mn,
+                             const long long* __restrict__ moff, const int* __restrict__ ms0,
+                             const long long* __restrict__ soff, const double* __restrict__ D,
+                             double* __restrict__ row, float* __restrict__ Ds) {
   const int s = blockIdx.x;
   if (s >= ns) return;
-  const int m = smol[s], n = mn[m];
-  const double* Dm = D + moff[m];
+  const int m = smol[s], n = mn[m], s0 = ms0[m], nsm = ms0[m + 1] - s0;
+  const double* Dm = D + moff[m] + (long long)f0[s] * n;
+  float* out = Ds + soff[m] + (long long)(s - s0) * nsm;
   double v = 0;
-  for (int a = 0; a < nc[s]; ++a)
-    for (int j = threadIdx.x; j < n; j += blockDim.x) v = fmax(v, fabs(Dm[(long)(f0[s] + a) * n + j]));
+  for (int j = threadIdx.x; j < nsm; j += blockDim.x) {
+    const int g = f0[s0 + j], w = nc[s0 + j];
+    double x = 0;
+    for (int a = 0; a < nc[s]; ++a)
+      for (int b = 0; b < w; ++b) x = fmax(x, fabs(Dm[(long long)a * n + g + b]));
+    out[j] = __double2float_ru(x);
+    v = fmax(v, x);
+  }
   __shared__ double sh[32];
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) v = fmax(v, __shfl_xor_sync(0xffffffffu, v, o));
@@ -343,20 +352,58 @@ __global__ void k_shell_rowmax(int ns, const int* __restrict__ f0, const int* __
 // A quartet (AB|CD) feeds J_AB (dD_CD), J_CD (dD_AB) and K_AC, K_AD, K_BC, K_BD
 // (dD_BD, dD_BC, dD_AD, dD_AC); every exchange block holds a bra shell, so
 // max(pw[bra], pb[ket]) bounds all six density factors.
-__global__ void k_pair_weight(int np, const int* __restrict__ pA, const int* __restrict__ pB,
-                              const int* __restrict__ pmol, const int* __restrict__ f0, const int* __restrict__ nc,
-                              const int* __restrict__ mn, const long long* __restrict__ moff,
-                              const double* __restrict__ D, const double* __restrict__ row, double* __restrict__ pw,
-                              double* __restrict__ pb) {
-  const int p = blockIdx.x * blockDim.x + threadIdx.x;
-  if (p >= np) return;
-  const int A = pA[p], B = pB[p], m = pmol[p], n = mn[m];
-  const double* Dm = D + moff[m];
-  double b = 0;
-  for (int x = 0; x < nc[A]; ++x)
-    for (int y = 0; y < nc[B]; ++y) b = fmax(b, fabs(Dm[(long)(f0[A] + x) * n + f0[B] + y]));
-  pw[p] = fmax(b, fmax(row[A], row[B]));
-  pb[p] = b;
+// One launch also makes the kernels' copies of the density, where asked for:
+// FP32 (d32) and two-float (dff), the latter scaled by 2^-e with e the exponent
+// of max |D| (clamped to +-400; 0 when the maximum is 0 or not finite), so that
+// any density an FP64 build takes stays inside the FP32 exponent range; and it
+// zeroes the work-queue heads.
+struct PrepArgs {
+  int np, ns;
+  const int *pA, *pB, *pmol, *f0, *nc, *mn;
+  const long long* moff;
+  const double* D;
+  const double* row;
+  double *pw, *pb;
+  float* pbf;
+  size_t nn;
+  float* d32;
+  ff* dff;
+  int* dexp;
+  int* counters;
+  int ncounters;
+};
+__global__ void __launch_bounds__(128) k_density_prep(PrepArgs a) {
+  const size_t i0 = blockIdx.x * (size_t)blockDim.x + threadIdx.x, step = (size_t)gridDim.x * blockDim.x;
+  if (i0 < (size_t)a.ncounters) a.counters[i0] = 0;
+  for (size_t p = i0; p < (size_t)a.np; p += step) {
+    const int A = a.pA[p], B = a.pB[p], m = a.pmol[p], n = a.mn[m];
+    const double* Dm = a.D + a.moff[m];
+    double b = 0;
+    for (int x = 0; x < a.nc[A]; ++x)
+      for (int y = 0; y < a.nc[B]; ++y) b = fmax(b, fabs(Dm[(long)(a.f0[A] + x) * n + a.f0[B] + y]));
+    a.pw[p] = fmax(b, fmax(a.row[A], a.row[B]));
+    a.pb[p] = b;
+    a.pbf[p] = __double2float_ru(b);
+  }
+  if (a.d32)
+    for (size_t i = i0; i < a.nn; i += step) a.d32[i] = (float)a.D[i];
+  if (!a.dff) return;
+  double mx = 0;
+  for (int s = threadIdx.x; s < a.ns; s += blockDim.x) mx = fmax(mx, a.row[s]);
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) mx = fmax(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+  __shared__ double sh[4];
+  if ((threadIdx.x & 31) == 0) sh[threadIdx.x >> 5] = mx;
+  __syncthreads();
+  mx = fmax(fmax(sh[0], sh[1]), fmax(sh[2], sh[3]));
+  const int e = mx > 0 && mx <= 1.7976931348623157e308 ? min(400, max(-400, ilogb(mx))) : 0;
+  const double sc = scalbn(1.0, -e);
+  if (i0 == 0) *a.dexp = e;
+  for (size_t i = i0; i < a.nn; i += step) {
+    const double v = a.D[i] * sc;
+    const float h = (float)v;
+    a.dff[i] = ff(h, (float)(v - (double)h));
+  }
 }
 
 __global__ void k_seg_max(int nseg, const int4* __restrict__ seg, const double* __restrict__ pw, double* __restrict__ sw) {
@@ -376,20 +423,54 @@ __global__ void k_seg_max(int nseg, const int4* __restrict__ seg, const double* 
   }
 }
 
-static gbhf_status density_weights(gbhf_ctx* c, TaskLists& st, const double* d_dD) {
+__global__ void k_to_float(size_t n, const double* __restrict__ x, float* __restrict__ y) {
+  for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x)
+    y[i] = (float)x[i];
+}
+static gbhf_status to_float(gbhf_ctx* c, size_t n, const double* d_x, float* d_y) {
+  const int blocks = (int)std::min<size_t>((n + 255) / 256, (size_t)c->nsm * 4);
+  k_to_float<<<std::max(blocks, 1), 256, 0, c->stream>>>(n, d_x, d_y);
+  count_launch(c);
+  GBHF_CUDA(c, cudaGetLastError());
+  return GBHF_OK;
+}
+
+// Everything the kernels of the next build need of its density d_dD: maxima for
+// the screening (c->tasks.Ds, pbf), FP32 and two-float copies, zeroed work-queue
+// heads of st (ncounters) and, with `segments`, the segment maxima of the weighted
+// task lists.
+static gbhf_status density_prep(gbhf_ctx* c, TaskLists& st, const double* d_dD, int precision, int ncounters,
+                                bool segments) {
   PairData& P = c->pairs;
-  const TaskLists& sh = c->tasks;   // per-shell and per-molecule arrays
+  TaskLists& sh = c->tasks;   // per-shell and per-molecule arrays
   const int ns = (int)c->basis.shells.size();
+  const size_t nst = (size_t)c->basis.stacked;   // all molecules' blocks
   GBHF_CUDA(c, st.row.alloc(ns));
   GBHF_CUDA(c, st.pw.alloc(std::max(P.npairs, 1)));
   GBHF_CUDA(c, st.pb.alloc(std::max(P.npairs, 1)));
   GBHF_CUDA(c, st.sw.alloc(std::max(P.nseg_total, 1)));
-  k_shell_rowmax<<<ns, 128, 0, c->stream>>>(ns, sh.f0.p, sh.nc.p, sh.smol.p, sh.mn.p, sh.moff.p, d_dD, st.row.p);
-  k_pair_weight<<<(P.npairs + 127) / 128, 128, 0, c->stream>>>(P.npairs, P.A.p, P.B.p, P.mol.p, sh.f0.p, sh.nc.p,
-                                                               sh.mn.p, sh.moff.p, d_dD, st.row.p, st.pw.p, st.pb.p);
-  if (P.nseg_total > 0) k_seg_max<<<P.nseg_total, 256, 0, c->stream>>>(P.nseg_total, P.seg_info.p, st.pb.p, st.sw.p);
-  count_launch(c, 3);
+  GBHF_CUDA(c, st.counters.alloc(ncounters));
+  GBHF_CUDA(c, sh.pbf.alloc(std::max(P.npairs, 1)));
+  GBHF_CUDA(c, sh.Ds.alloc(std::max<size_t>(sh.ds_size, 1)));
+  if (precision != GBHF_PREC_FP64) GBHF_CUDA(c, c->dfloat.alloc(nst));
+  if (P.use_ff) {
+    GBHF_CUDA(c, c->dff.alloc(nst));
+    GBHF_CUDA(c, c->dff_exp.alloc(1));
+  }
+  k_shell_dmax<<<ns, 128, 0, c->stream>>>(ns, sh.f0.p, sh.nc.p, sh.smol.p, sh.mn.p, sh.moff.p, sh.ms0.p, sh.soff.p, d_dD,
+                                          st.row.p, sh.Ds.p);
+  const PrepArgs a{P.npairs,   ns,          P.A.p, P.B.p,  P.mol.p, sh.f0.p, sh.nc.p, sh.mn.p, sh.moff.p, d_dD, st.row.p,
+                   st.pw.p,    st.pb.p,     sh.pbf.p, nst, precision != GBHF_PREC_FP64 ? c->dfloat.p : nullptr,
+                   P.use_ff ? c->dff.p : nullptr, c->dff_exp.p, st.counters.p, ncounters};
+  const int blocks = (int)std::min<size_t>((std::max<size_t>(P.npairs, nst) + 127) / 128, (size_t)c->nsm * 8);
+  k_density_prep<<<std::max(blocks, 1), 128, 0, c->stream>>>(a);
+  if (segments && P.nseg_total > 0) {
+    k_seg_max<<<P.nseg_total, 256, 0, c->stream>>>(P.nseg_total, P.seg_info.p, st.pb.p, st.sw.p);
+    count_launch(c);
+  }
+  count_launch(c, 2);
   GBHF_CUDA(c, cudaGetLastError());
+  sh.screened = true;
   return GBHF_OK;
 }
 
@@ -421,8 +502,12 @@ static gbhf_status build_task_lists(gbhf_ctx* c, TaskLists& TL, int ncombo, cons
   GBHF_CUDA(c, TL.item_count.alloc(NTIER * (size_t)std::max(ni, 1)));
   GBHF_CUDA(c, TL.item_off.alloc(NTIER * ((size_t)ni + 1)));
   GBHF_CUDA(c, TL.ranges.alloc(2 * NTIER * ncombo));
-  GBHF_CUDA(c, TL.counters.alloc(NTIER * ncombo));
   GBHF_CUDA(c, TL.stats.alloc(3 * NTIER * ncombo));
+  // 32-ket groups that a task of the s/p J/K kernels scans: the queue of survivors
+  // then fills whole batches, and the bra is staged once for all of them, while
+  // there are tasks enough for every warp ((H2O)64 mixed build in order: 65.9 ms
+  // at 1, 57.3 at 4, 56.2 at 8, 55.8 at 16; (H2O)16 mixed SCF 40.4, 39.3, 39.6, 40.3)
+  const int scan = P.npairs >= 65536 ? 8 : 4;
   TaskGenArgs g;
   g.nitems = ni;
   g.ncombo = ncombo;
@@ -431,6 +516,8 @@ static gbhf_status build_task_lists(gbhf_ctx* c, TaskLists& TL, int ncombo, cons
     g.cket[k] = k < ncombo ? cket[k] : 0;
     g.lane_prims[k] = k < ncombo ? std::max(1, lane_prims[k]) : 1;
     g.task_kets[k] = k < ncombo ? std::min(32, std::max(1, task_kets[k])) : 32;
+    // (the s/p kernels only)
+    if (k < (all_pairs ? NGCOMBO_SP : NCOMBO_SP) && g.task_kets[k] == 32) g.task_kets[k] *= scan;
     // the (ss|ss) and (ps|ps) quartets with the bra of more primitives: the
     // FP32 launches gain 13-14% (fewer ket-field loads per primitive
     // quartet); (pp|pp) FP64 lost 18% that way (its launch is tail-bound)
@@ -575,6 +662,17 @@ gbhf_status ensure_shell_arrays(gbhf_ctx* c) {
   }
   GBHF_CUDA(c, st.f0.alloc(ns));
   GBHF_CUDA(c, st.sscale.alloc(sc.size()));
+  // shells of each molecule (contiguous: shells follow the functions)
+  std::vector<int> ms0(b.nmol + 1, (int)ns);
+  std::vector<long long> soff(b.nmol + 1, 0);
+  for (size_t s = ns; s-- > 0;) ms0[sm[s]] = (int)s;
+  for (int m = 0; m < b.nmol; ++m) soff[m + 1] = soff[m] + (long long)(ms0[m + 1] - ms0[m]) * (ms0[m + 1] - ms0[m]);
+  st.ds_size = (size_t)soff[b.nmol];
+  GBHF_CUDA(c, st.ms0.alloc(b.nmol + 1));
+  GBHF_CUDA(c, st.soff.alloc(b.nmol + 1));
+  GBHF_CUDA(c, cudaMemcpyAsync(st.ms0.p, ms0.data(), (b.nmol + 1) * sizeof(int), cudaMemcpyHostToDevice, c->stream));
+  GBHF_CUDA(c, cudaMemcpyAsync(st.soff.p, soff.data(), (b.nmol + 1) * sizeof(long long), cudaMemcpyHostToDevice,
+                               c->stream));
   GBHF_CUDA(c, st.cen.alloc(3 * std::max<size_t>(ns, 1)));
   GBHF_CUDA(c, cudaMemcpyAsync(st.cen.p, cen.data(), cen.size() * sizeof(float), cudaMemcpyHostToDevice, c->stream));
   GBHF_CUDA(c, st.nc.alloc(ns));
@@ -613,8 +711,10 @@ gbhf_status build_grad_tasks(gbhf_ctx* c, const double* d_D, double cutoff, doub
   GBHF_TRY(ensure_pairs(c));
   GBHF_TRY(ensure_shell_arrays(c));
   TaskLists& gt = c->gtasks;
-  GBHF_TRY(density_weights(c, gt, d_D));
-  const double t64 = precision == GBHF_PREC_FP64 ? 0.0 : mixed_cutoff;
+  GBHF_TRY(density_prep(c, gt, d_D, precision, NTIER * NCOMBO_MAX, true));
+  // FP32 up to the cutoff, but never above a bound of 1/8: two floats take the
+  // rest of what a larger cutoff gives to FP32
+  const double t64 = precision == GBHF_PREC_FP64 ? 0.0 : std::min(mixed_cutoff, 0.125);
   GBHF_TRY(build_task_lists(c, gt, NCOMBO_MAX, GRAD_COMBO_BRA, GRAD_COMBO_KET, c->gr_lp, c->gr_tk, true, true,
                             cutoff, t64, ff_weighted_limit(precision, t64), gt.pw.p, gt.sw.p));
   return GBHF_OK;
@@ -625,12 +725,22 @@ gbhf_status jk_build(gbhf_ctx* c, const double* d_Dsq, double* d_G, int precisio
   const int wj = with_j ? 1 : 0;
   c->tasks.thr_exact = schwarz;   // per-quartet test in the kernels, on the density passed here
   GBHF_TRY(ensure_pairs(c));
-  const int n = c->basis.nbf;
+  const PairData& P = c->pairs;
   TaskLists& st = c->tasks;
   GBHF_TRY(ensure_shell_arrays(c));
+  if (local_weights || P.nprim_pairs >= SMALL_PRIM_PAIRS) {
+    GBHF_TRY(density_prep(c, st, d_Dsq, precision, NTIER * NCOMBO, local_weights));
+  } else {
+    st.screened = false;
+    GBHF_CUDA(c, st.counters.alloc(NTIER * NCOMBO));
+    GBHF_CUDA(c, cudaMemsetAsync(st.counters.p, 0, NTIER * NCOMBO * sizeof(int), c->stream));
+    if (precision != GBHF_PREC_FP64) {
+      GBHF_CUDA(c, c->dfloat.alloc((size_t)c->basis.stacked));
+      GBHF_TRY(to_float(c, (size_t)c->basis.stacked, d_Dsq, c->dfloat.p));
+    }
+  }
   if (local_weights) {
     // incremental build: bounds weighted by the local size of the density change
-    GBHF_TRY(density_weights(c, st, d_Dsq));
     const double t64 = precision == GBHF_PREC_FP64 ? 0.0 : mixed_cutoff;
     GBHF_TRY(build_tasks(c, precision, schwarz, t64, st.pw.p, st.sw.p));
     st.thr_all = -1;   // lists no longer match a uniform weight
@@ -645,24 +755,17 @@ gbhf_status jk_build(gbhf_ctx* c, const double* d_Dsq, double* d_G, int precisio
       st.thr64 = thr64;
     }
   }
-  GBHF_CUDA(c, cudaMemsetAsync(c->tasks.counters.p, 0, NTIER * NCOMBO * sizeof(int), c->stream));
   if (!st.stats_pending) {   // the counters add up over builds until flush_jk_stats reads them
     GBHF_CUDA(c, cudaMemsetAsync(c->tasks.stats.p, 0, 3 * NTIER * NCOMBO * sizeof(unsigned long long), c->stream));
     st.stats_pending = true;
   }
   int nt[NCOMBO][NTIER];
-  bool any[NTIER] = {};
+  long total = 0;
   for (int k = 0; k < NCOMBO; ++k)
     for (int t = 0; t < NTIER; ++t) {
       nt[k][t] = st.hranges[2 * (NTIER * k + t) + 1] - st.hranges[2 * (NTIER * k + t)];
-      any[t] |= nt[k][t] > 0;
+      total += nt[k][t];
     }
-  const size_t nst = (size_t)c->basis.stacked;   // all molecules' blocks
-  if (any[TIER_32]) {
-    GBHF_CUDA(c, c->dfloat.alloc(nst));
-    GBHF_TRY(to_float(c, nst, d_Dsq, c->dfloat.p));
-  }
-  if (any[TIER_FF]) GBHF_TRY(to_ff(c, nst, d_Dsq));
   const bool ev = c->prof.events;
   // FP64 lists, then two-float, then FP32, each heaviest class first.  Without
   // per-class profiling events the launches go round-robin to the side streams:
@@ -671,6 +774,11 @@ gbhf_status jk_build(gbhf_ctx* c, const double* d_Dsq, double* d_G, int precisio
   // order on the context stream so that each launch is timed alone.
   static const int order[NCOMBO] = {20, 19, 18, 17, 16, 15, 14, 13, 12, 11, 10, 9, 8, 7, 6, 5, 4, 3, 2, 1, 0};
   static const int tiers[NTIER] = {TIER_64, TIER_FF, TIER_32};
+  // with a million tasks the launches are long against their tails, and classes
+  // that share an SM only push each other's Boys rows out of L1: one stream
+  // ((H2O)64 mixed, 3.1 million tasks: 56.2 ms in order, 61.8 on eight streams;
+  // (H2O)16, 170 thousand: 42.7 against 39.4 ms per SCF)
+  const int nside = total >= (1l << 20) ? 1 : gbhf_ctx::NSIDE;
   int ne = 0, nl = 0;
   int ev_combo[NTIER * NCOMBO], ev_prec[NTIER * NCOMBO];
   if (ev) GBHF_CUDA(c, cudaEventRecord(c->evc[ne], c->stream));
@@ -682,7 +790,7 @@ gbhf_status jk_build(gbhf_ctx* c, const double* d_Dsq, double* d_G, int precisio
     for (int oi = 0; oi < NCOMBO; ++oi) {
       const int k = order[oi];
       if (nt[k][tier] <= 0) continue;
-      cudaStream_t strm = ev ? c->stream : c->side[nl % gbhf_ctx::NSIDE];
+      cudaStream_t strm = ev ? c->stream : c->side[nl % nside];
       ++nl;
       if (k >= NCOMBO_SP && !gen_dclass(k)) GBHF_TRY(launch_jk_dclass(c, strm, k, tier, d_Dsq, d_G, nt[k][tier], wj));
       else if (tier == TIER_64) GBHF_TRY(launch_combo<double>(c, strm, k, tier, d_Dsq, d_G, nt[k][tier], wj));

@@ -369,46 +369,6 @@ __global__ void k_antisym(int n, const double* __restrict__ M, double* __restric
   e[(long)i * n + j] = M[(long)i * n + j] - M[(long)j * n + i];
 }
 
-__global__ void k_to_float(size_t n, const double* __restrict__ x, float* __restrict__ y) {
-  for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x)
-    y[i] = (float)x[i];
-}
-
-gbhf_status to_float(gbhf_ctx* c, size_t n, const double* d_x, float* d_y) {
-  int blocks = (int)std::min<size_t>((n + 255) / 256, (size_t)c->nsm * 8);
-  k_to_float<<<std::max(blocks, 1), 256, 0, c->stream>>>(n, d_x, d_y);
-  count_launch(c);
-  GBHF_CUDA(c, cudaGetLastError());
-  return GBHF_OK;
-}
-
-// Density of the two-float kernels: 2^-e x as two FP32 parts, with e the
-// exponent of max |x| (clamped to +-400; 0 when the maximum is 0 or not finite),
-// so that any density an FP64 build takes stays inside the FP32 exponent range.
-__global__ void k_to_ff(size_t n, const double* __restrict__ x, const double* __restrict__ mx, ff* __restrict__ y,
-                        int* __restrict__ e_out) {
-  const double m = *mx;
-  const int e = m > 0 && m <= 1.7976931348623157e308 ? min(400, max(-400, ilogb(m))) : 0;
-  const double s = scalbn(1.0, -e);
-  if (blockIdx.x == 0 && threadIdx.x == 0) *e_out = e;
-  for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) {
-    const double v = x[i] * s;
-    const float h = (float)v;
-    y[i] = ff(h, (float)(v - (double)h));
-  }
-}
-gbhf_status to_ff(gbhf_ctx* c, size_t n, const double* d_x) {
-  GBHF_CUDA(c, c->dff.alloc(n));
-  GBHF_CUDA(c, c->dff_exp.alloc(1));
-  GBHF_CUDA(c, c->dff_max.alloc(1));
-  GBHF_TRY(max_abs_dev(c, n, d_x, c->dff_max.p));
-  const int blocks = (int)std::min<size_t>((n + 255) / 256, (size_t)c->nsm * 4);
-  k_to_ff<<<std::max(blocks, 1), 256, 0, c->stream>>>(n, d_x, c->dff_max.p, c->dff.p, c->dff_exp.p);
-  count_launch(c);
-  GBHF_CUDA(c, cudaGetLastError());
-  return GBHF_OK;
-}
-
 // Block reduction helper (sum or max) into a double.
 
 // out[0] = max|e|, out[1] = 1/2 sum Dnew(H+F) (when H,F given), out[2] = sum (Dnew-Dold)^2,

@@ -414,7 +414,7 @@ static std::vector<double> ff_limits(const Basis& b, const PairData& P) {
   for (double k : b.prim_coef) range &= std::fabs(k) <= 1e8;
   for (double x : b.xyz) range &= std::fabs(x) <= 1e5;
   std::vector<double> lim(b.nmol, 0.0);
-  if (!range || P.nprim_pairs < 512) return lim;
+  if (!range || P.nprim_pairs < SMALL_PRIM_PAIRS) return lim;
   for (int t = 0; t < P.npairs; ++t) {
     double& q = lim[b.shells[P.hA[t]].mol];
     q = std::max(q, P.hQ[t]);
@@ -628,7 +628,7 @@ gbhf_status ensure_pairs(gbhf_ctx* c) {
   GBHF_CUDA(c, P.bra32.alloc(nf));
   GBHF_CUDA(c, P.ket32.alloc(nf));
   const std::vector<double> ffq = ff_limits(b, P);
-  const bool use_ff = *std::max_element(ffq.begin(), ffq.end()) > 0;
+  const bool use_ff = P.use_ff = *std::max_element(ffq.begin(), ffq.end()) > 0;
   if (use_ff) {
     GBHF_TRY(ensure_boys_ff(c));
     GBHF_CUDA(c, P.braff.alloc(nf));
@@ -643,7 +643,16 @@ gbhf_status ensure_pairs(gbhf_ctx* c) {
   GBHF_CUDA(c, up(P.poff.p, P.hPoff.data(), np * sizeof(int)));
   GBHF_CUDA(c, up(P.kseg.p, P.hSeg.data(), np * sizeof(int)));
   GBHF_CUDA(c, up(P.Q.p, P.hQ.data(), np * sizeof(double)));
-  std::vector<float> qf(P.hQ.begin(), P.hQ.end());
+  std::vector<float> qf(np);
+  std::vector<int4> pinfo(std::max(np, 1));
+  for (int t = 0; t < np; ++t) {
+    qf[t] = (float)P.hQ[t];
+    if ((double)qf[t] < P.hQ[t]) qf[t] = std::nextafter(qf[t], INFINITY);
+    const Shell &sa = b.shells[P.hA[t]], &sb = b.shells[P.hB[t]];
+    pinfo[t] = make_int4(P.hA[t], P.hB[t], sa.f0 - b.mol_fn_off[sa.mol], sb.f0 - b.mol_fn_off[sb.mol]);
+  }
+  GBHF_CUDA(c, P.pinfo.alloc(std::max(np, 1)));
+  GBHF_CUDA(c, up(P.pinfo.p, pinfo.data(), np * sizeof(int4)));
   GBHF_CUDA(c, P.Qf.alloc(std::max(np, 1)));
   GBHF_CUDA(c, up(P.Qf.p, qf.data(), np * sizeof(float)));
   GBHF_CUDA(c, P.ffq.alloc(ffq.size()));

@@ -89,6 +89,7 @@ gbhf_status autotune_dev(gbhf_ctx* c, int which, const double* d_D, int precisio
                which == 0 ? c->jk_tk : c->gr_tk};
   reps = std::max(1, reps);
   const Profile saved = c->prof;
+  GBHF_TRY(ensure_profile_events(c));
   c->prof.events = true;
   DBuf<double> out;
   const size_t nout = which == 0 ? (size_t)c->basis.stacked : 3 * (size_t)std::max(c->basis.natoms, 1);

@@ -95,3 +95,45 @@ def test_exponents_outside_the_fp32_range_stay_in_fp64(ctx):
     ref = O.fock_canonical(h, d, ob.eri_canonical(False))
     got = ctx.fock(h, d, _lib.MODE_EXACT, _lib.PREC_FP64, 0.0, 0.0)
     np.testing.assert_allclose(got, ref, rtol=0, atol=1e-13 * np.abs(ref).max())
+
+
+def _one_atom_pair(shells):
+    """Two atoms with one-primitive shells of the given angular momenta."""
+    lab = {0: ("S",), 1: ("Px", "Py", "Pz"), 2: ("Dxx", "Dxy", "Dxz", "Dyy", "Dyz", "Dzz")}
+    fns = [B.CGF(((1.0, 0.7 + 0.4 * i),), t) for i, l in enumerate(shells) for t in lab[l]]
+    return B.flatten([B.AtomData((0.0, 0.0, 0.0), fns, 8.0), B.AtomData((0.0, 0.3, 1.9), fns, 8.0)])
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("shells", [(0,), (0, 0), (1, 0), (2,), (2, 0), (2, 0, 0), (2, 1), (2, 2, 0, 0), (2, 1, 0)],
+                         ids=lambda s: "".join("spd"[l] for l in s))
+def test_every_class_alone_and_with_zero_density(ctx, shells):
+    """Unscreened builds over few shells: a zero density gives exactly the core
+    matrix, a random one the stored-integral Fock matrix (1e-12: sums of a few
+    hundred rounding errors of elements of order one to ten)."""
+    fb = _one_atom_pair(shells)
+    ctx.set_basis(fb)
+    ntri = fb.n_cgf * (fb.n_cgf + 1) // 2
+    h = np.arange(ntri, dtype=float)
+    np.testing.assert_array_equal(ctx.fock(h, np.zeros(ntri), _lib.MODE_EXACT, _lib.PREC_FP64, 0.0, 0.0), h)
+    d = np.random.default_rng(1).standard_normal(ntri)
+    ref = O.fock_canonical(np.zeros(ntri), d, O.OracleBasis(fb).eri_canonical(False))
+    got = ctx.fock(np.zeros(ntri), d, _lib.MODE_EXACT, _lib.PREC_FP64, 0.0, 0.0)
+    np.testing.assert_allclose(got, ref, rtol=0, atol=1e-12)
+
+
+@pytest.mark.gpu
+def test_queued_batches_of_a_large_system(ctx):
+    """(H2O)10/6-31G: 4 095 pairs, ket ranges longer than a batch and batches cut by
+    the density screening; FP64 against the oracle's screened build and mixed
+    against FP64 (the bounds of the library's own Fock tests)."""
+    xyz = M.water_cluster(10, np.random.default_rng(10))
+    fb = B.flatten(B.make_atoms(M.water_labels(10), xyz, "6-31g"))
+    ob = O.OracleBasis(fb)
+    ctx.set_basis(fb)
+    h, d = ob.hcore(False), _density(fb, 10)
+    ref, _ = ob.fock_direct(h, d, 1e-12)
+    got = ctx.fock(h, d, _lib.MODE_EXACT, _lib.PREC_FP64, 1e-12, 0.0)
+    np.testing.assert_allclose(got, ref, rtol=0, atol=1e-10)
+    mix = ctx.fock(h, d, _lib.MODE_EXACT, _lib.PREC_MIXED, 1e-12, 1e-4)
+    assert 0 < np.max(np.abs(mix - got)) < 1e-6
