@@ -54,6 +54,17 @@ bool need_basis(gbhf_ctx* c) {
 
 }  // namespace
 
+namespace gbhf {
+// The launch boundaries of the profiling builds, created with the first of them.
+gbhf_status ensure_profile_events(gbhf_ctx* c) {
+  for (auto& e : c->evc)
+    if (!e) GBHF_CUDA(c, cudaEventCreate(&e));
+  for (auto& e : c->evg)
+    if (!e) GBHF_CUDA(c, cudaEventCreate(&e));
+  return GBHF_OK;
+}
+}  // namespace gbhf
+
 extern "C" {
 
 int gbhf_version(void) { return 1; }
@@ -610,17 +621,6 @@ gbhf_status gbhf_autotune(gbhf_ctx* c, int which, int precision, double schwarz_
   const double mc = precision == GBHF_PREC_FP64 ? 0.0 : mixed_cutoff;
   return autotune_dev(c, which, D, precision, schwarz_cutoff, mc, repeats, class_ms);
 }
-
-namespace gbhf {
-// The launch boundaries of the profiling builds, created with the first of them.
-gbhf_status ensure_profile_events(gbhf_ctx* c) {
-  for (auto& e : c->evc)
-    if (!e) GBHF_CUDA(c, cudaEventCreate(&e));
-  for (auto& e : c->evg)
-    if (!e) GBHF_CUDA(c, cudaEventCreate(&e));
-  return GBHF_OK;
-}
-}  // namespace gbhf
 
 gbhf_status gbhf_profile_reset(gbhf_ctx* c, int enable_events) {
   CTX_CHECK(c);
