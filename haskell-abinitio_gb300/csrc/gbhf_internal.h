@@ -282,8 +282,10 @@ struct TridiagWork {
   DBuf<int> blk, rank;
 };
 // Largest n of the tridiagonal path: the packed lower triangle of A plus two
-// vectors in one CTA's shared memory (232: 215 KiB).  Larger n use Jacobi.
+// vectors in one CTA's shared memory (232: 215 KiB).
 constexpr int TRIDIAG_MAX_N = 232;
+// With the rows in the shared memory of a 16-CTA cluster (608: 222 KiB each).
+constexpr int TRIDIAG_WIDE_MAX_N = 608;
 
 struct Profile {
   bool events = false;
@@ -335,7 +337,7 @@ struct gbhf_ctx {
   size_t smem_optin = 0;          // largest dynamic shared memory per block (opt-in)
   bool force_jacobi = false;      // GBHF_EIGEN=jacobi at gbhf_create: every eigen-solve by Jacobi
   bool force_sytrd_single = false; // GBHF_EIGEN=single-cta: tridiagonalisation in one CTA
-  int sytrd_cluster = 0;          // 1: the cluster tridiagonalisation runs here, -1: it does not, 0: not checked
+  bool sytrd_checked = false, sytrd8 = false, sytrd16 = false;   // the cluster tridiagonalisations that run here
   // state of the last SCF (for the gradient): density, Fock matrix, occupation
   gbhf::DBuf<double> last_D, last_F;
   // state of the last converged UHF SCF: alpha and beta densities, energy-weighted density
@@ -522,9 +524,9 @@ gbhf_status launch_grad_dclass(gbhf_ctx* c, cudaStream_t strm, int combo, int ti
 gbhf_status gemm(gbhf_ctx* c, bool ta, bool tb, int m, int n, int k, double alpha, const double* A, int lda,
                  const double* B, int ldb, double beta, double* C, int ldc, bool sym = false);
 gbhf_status eigh(gbhf_ctx* c, int n, const double* d_A, double* d_evals, double* d_evecs, const double* d_V0);
-// tridiag.cu: Householder + bisection + inverse iteration, n <= TRIDIAG_MAX_N
+// tridiag.cu: Householder + bisection + inverse iteration, for the n that tridiag_takes
+bool tridiag_takes(gbhf_ctx* c, int n);
 gbhf_status eigh_tridiag(gbhf_ctx* c, int n, const double* d_A, double* d_evals, double* d_evecs);
-size_t tridiag_smem_bytes(int n);
 gbhf_status flat_to_square(gbhf_ctx* c, int n, const double* d_flat, double* d_sq);
 gbhf_status square_to_flat(gbhf_ctx* c, int n, const double* d_sq, double* d_flat);
 gbhf_status symm_ortho_dev(gbhf_ctx* c, int n, const double* d_S, double* d_X);

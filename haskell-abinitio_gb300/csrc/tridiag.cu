@@ -4,11 +4,11 @@
 // eigenvalues with the eigenvectors as columns (sortEigenData,
 // NumericalTools/VectorTools.hs:27-31).
 //
-// 1. k_sytrd_cluster: an 8-CTA thread-block cluster reduces A to tridiagonal
-//    T = Q^T A Q with the packed lower triangle of A spread over the CTAs'
-//    shared memory (k_sytrd: the same in one CTA, where clusters are not
-//    available), n - 2 Householder reflectors H_k = I - tau_k v_k v_k^T
-//    (v_k[k+1] = 1); n <= TRIDIAG_MAX_N.
+// 1. k_sytrd_cluster: a thread-block cluster of 8 or 16 CTAs reduces A to
+//    tridiagonal T = Q^T A Q with the rows of A spread over the CTAs' shared
+//    memory (k_sytrd: the packed triangle in one CTA, for the smallest n and where
+//    clusters are not available), n - 2 Householder reflectors H_k = I - tau_k v_k v_k^T
+//    (v_k[k+1] = 1); n <= TRIDIAG_WIDE_MAX_N.
 // 2. k_tri_prep: split T into unreduced blocks at negligible off-diagonals.
 // 3. k_tri_vec: one warp per eigenvalue: 32-point multisection with Sturm
 //    counts on its block, then inverse iteration (LU with partial pivoting of
@@ -150,179 +150,192 @@ __global__ void __launch_bounds__(1024) k_sytrd(int n, const double* __restrict_
   }
 }
 
-// The same reduction by one thread-block cluster of SY_CS CTAs: CTA r owns
-// the rows i = r (mod SY_CS) of the packed lower triangle in its shared memory,
-// so the FP64 work of a step is split SY_CS ways.  Per step k, two cluster
-// barriers:
-//   A. every CTA pushes its entries x_i = A_ik (i > k) into every CTA's copy of
-//      the Householder vector and its partial |x|^2 into its own slot; after
-//      the barrier each CTA sums the partials in rank order (all CTAs get the
-//      same bits), forms tau and scales its copy into v;
-//   B. p_part[j] = sum over its own rows i > j of A_ij v_i (+ the row dot
-//      sum_(l <= j) A_jl v_l for its own rows j); after the barrier every CTA
-//      sums p_j over the ranks (rank order), forms p.v and w = p - (tau/2)(p.v) v
-//      for all j, and updates its own rows A_il -= v_i w_l + w_i v_l.
-// The Householder vector and the partial slots alternate between two buffers
-// by step parity (a CTA writes step k + 1's values into another CTA's memory
-// while that CTA may still read step k's).  Outputs as k_sytrd.
-constexpr int SY_CS = 8, SY_THREADS = 512;
+// The same reduction by one thread-block cluster of CS CTAs: CTA r holds the
+// full rows i = r (mod CS) of A in its shared memory, so that a row's product
+// with the Householder vector needs no other CTA and the FP64 work of a step is
+// split CS ways.  The rank-2 update of step k - 1 is applied in the same pass
+// that forms the products of step k (one read and one write of A per step).
+// Per step two cluster barriers:
+//   A. every CTA forms its entries x_i of column k (with the pending update) and
+//      writes them into every CTA's copy of x;
+//   B. after the barrier one warp forms tau and the scale from x (the same bits in
+//      every CTA), all form v; each warp updates own rows, A_il -= v'_i w'_l +
+//      w'_i v'_l with the last step's v' and w', takes their products with v and
+//      writes p_i = tau A_i v into every CTA's copy of p;
+//   after the barrier w = p - (tau/2)(p.v) v, for all entries in every CTA.
+// x is rewritten only after barrier B of its step and p only after barrier A of
+// the next one, so one buffer of each is enough.  Outputs as k_sytrd.
+//
+// Bound: the two barriers and the serial scalar part of a step (2-3 us) and, from
+// n of about 300 on, FP64 throughput (3 FMAs per element and step, 2 per cycle and
+// SM): 16 CTAs above SY_WIDE_N (8 CTAs 3.67 ms at n = 256 for the whole solve, 16
+// CTAs 3.46 at 257).  The solve at n = 208: 4.60 ms with the packed triangle spread
+// over 8 CTAs (partial products summed over the CTAs, four block reductions a
+// step) and the kernels below as they were, 2.73 now; at 333: 59.5 ms by Jacobi,
+// 4.9 now.
+constexpr int SY_THREADS = 512, SY_WARPS = SY_THREADS / 32;
+constexpr int SY_WIDE_N = 256;
 
-__host__ __device__ __forceinline__ long sy_off(int r, int q) {   // start of local row q of rank r
-  return (long)q * (r + 1) + (long)SY_CS * q * (q - 1) / 2;
-}
-__host__ __device__ __forceinline__ long sy_local_doubles(int n, int r) {
-  const int nq = n > r ? (n - r + SY_CS - 1) / SY_CS : 0;
-  return sy_off(r, nq);
+__host__ __device__ __forceinline__ int sy_ld(int n) { return n | 1; }
+inline size_t sy_smem_bytes(int n, int cs) {
+  return ((size_t)((n + cs - 1) / cs) * sy_ld(n) + 5 * (size_t)n) * sizeof(double);
 }
 
-__global__ void __cluster_dims__(SY_CS, 1, 1) __launch_bounds__(SY_THREADS)
+template <int CS>
+__global__ void __launch_bounds__(SY_THREADS)
     k_sytrd_cluster(int n, const double* __restrict__ A, double* __restrict__ d, double* __restrict__ e,
                     double* __restrict__ tau, double* __restrict__ Vt) {
   namespace cg = cooperative_groups;
   cg::cluster_group cluster = cg::this_cluster();
   extern __shared__ double sm[];
-  const int r = (int)cluster.block_rank(), tid = threadIdx.x, nt = blockDim.x;
-  const int nq = n > r ? (n - r + SY_CS - 1) / SY_CS : 0;   // rows owned
-  // The buffers other CTAs reach come first, at the same offsets in every CTA
-  // (a remote address is the local offset mapped into the other CTA's window);
-  // the owned rows, whose size depends on the rank, follow them.
-  double* sv = sm;                   // 2 x n: Householder vector, by step parity
-  double* sw = sv + 2 * n;           // n: p, then w
-  double* pp = sw + n;               // n: this CTA's partial p
-  double* red = pp + n;              // 2 x 4: partial |x|^2 by step parity
-  double* P = red + 8;               // owned rows, packed
-  __shared__ double s_bc[4];
-  __shared__ double s_red[SY_THREADS / 32];
-  auto row_of = [&](int q) { return r + SY_CS * q; };
-  auto bsum = [&](double v) -> double {   // block sum, valid in every thread
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-    __syncthreads();
-    if ((tid & 31) == 0) s_red[tid >> 5] = v;
-    __syncthreads();
-    double t = 0.0;
-    for (int w = 0; w < nt / 32; ++w) t += s_red[w];
-    return t;
-  };
-  for (int q = 0; q < nq; ++q) {
-    const int i = row_of(q);
-    for (int j = tid; j <= i; j += nt) P[sy_off(r, q) + j] = A[(long)i * n + j];
-  }
+  __shared__ double s_bc[3];
+  const int r = (int)cluster.block_rank(), tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int nq = n > r ? (n - r + CS - 1) / CS : 0;   // rows owned: r + CS q
+  const int ld = sy_ld(n);
+  // the buffers that other CTAs write come first, at the same offsets in every CTA
+  double* x = sm;
+  double* p = x + n;
+  double* v = p + n;        // this step's Householder vector
+  double* vp = v + n;       // the last step's v and w
+  double* wp = vp + n;
+  double* P = wp + n;       // owned rows
+  for (int q = warp; q < nq; q += SY_WARPS)
+    for (int j = lane; j < n; j += 32) {   // the lower triangle is what counts
+      const int i = r + CS * q;
+      P[q * ld + j] = j <= i ? A[(long)i * n + j] : A[(long)j * n + i];
+    }
+  for (int i = tid; i < n; i += SY_THREADS) vp[i] = wp[i] = 0.0;
   cluster.sync();
   for (int k = 0; k + 2 < n; ++k) {
-    const int par = k & 1;
-    double* v = sv + par * n;
-    // A: push x_i = A_ik (i > k) of own rows into every CTA's copy; partial |x|^2 (i > k + 1)
-    const int q0 = (k + 1 - r + SY_CS - 1) / SY_CS > 0 ? (k + 1 - r + SY_CS - 1) / SY_CS : 0;   // first own row > k
-    double s = 0.0;
-    for (int idx = tid; idx < (nq - q0) * SY_CS; idx += nt) {
-      const int q = q0 + idx / SY_CS, dst = idx % SY_CS;
-      const int i = row_of(q);
-      const double x = P[sy_off(r, q) + k];
-      double* rv = cluster.map_shared_rank(v, dst);
-      rv[i] = x;
-      if (dst == 0 && i > k + 1) s += x * x;
+    const int q0 = k >= r ? (k - r) / CS + 1 : 0;   // first own row > k
+    // A: column k of own rows > k, to every CTA
+    {
+      const double wk = wp[k], vk = vp[k];
+      for (int idx = tid; idx < (nq - q0) * CS; idx += SY_THREADS) {
+        const int q = q0 + idx / CS, dst = idx % CS, i = r + CS * q;
+        const double xi = fma(-wp[i], vk, fma(-vp[i], wk, P[q * ld + k]));
+        cluster.map_shared_rank(x, dst)[i] = xi;
+      }
+      if (k % CS == r && tid == 0) d[k] = fma(-2.0 * vk, wk, P[(k / CS) * ld + k]);
     }
-    s = bsum(s);
-    if (tid == 0) red[par * 4] = s;
-    if (k % SY_CS == r && tid == 0) d[k] = P[sy_off(r, k / SY_CS) + k];
     cluster.sync();
-    if (tid < 32) {
-      // the SY_CS partials read at once (one remote latency), summed in rank order
-      const double part = tid < SY_CS ? *cluster.map_shared_rank(red + par * 4, tid) : 0.0;
-      double tot = 0.0;
+    if (warp == 0) {
+      double s = 0.0;
+      for (int i = k + 2 + lane; i < n; i += 32) s = fma(x[i], x[i], s);
 #pragma unroll
-      for (int rr = 0; rr < SY_CS; ++rr) tot += __shfl_sync(0xffffffffu, part, rr);
-      const double alpha = v[k + 1];
-      double beta = alpha, t = 0.0, scale = 0.0;
-      if (tot > 0.0) {
-        beta = -copysign(sqrt(alpha * alpha + tot), alpha);
-        t = (beta - alpha) / beta;
-        scale = 1.0 / (alpha - beta);
-      }
-      if (r == 0 && tid == 0) {
-        e[k] = beta;
-        tau[k] = t;
-      }
-      if (tid == 0) {
+      for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+      if (lane == 0) {
+        const double alpha = x[k + 1];
+        double beta = alpha, t = 0.0, scale = 0.0;
+        if (s > 0.0) {
+          beta = -copysign(sqrt(fma(alpha, alpha, s)), alpha);
+          t = (beta - alpha) / beta;
+          scale = 1.0 / (alpha - beta);
+        }
         s_bc[0] = t;
         s_bc[1] = scale;
+        if (r == 0) {
+          e[k] = beta;
+          tau[k] = t;
+        }
       }
     }
     __syncthreads();
     const double t = s_bc[0], scale = s_bc[1];
-    for (int i = k + 1 + tid; i < n; i += nt) v[i] = i == k + 1 ? 1.0 : v[i] * scale;
+    for (int i = k + 1 + tid; i < n; i += SY_THREADS) v[i] = i == k + 1 ? 1.0 : x[i] * scale;
     __syncthreads();
-    for (int q = tid; q < nq; q += nt) {   // own entries of Vt row k
-      const int i = row_of(q);
-      Vt[(long)k * n + i] = i <= k ? 0.0 : v[i];
-    }
-    // (with t = 0 the steps below leave A unchanged; they still run, so that
-    // every CTA passes the same barriers whatever its data)
-    // B: partial p (column part over own rows i > j, then the row dots of own rows)
-    for (int j = k + 1 + tid; j < n; j += nt) {
+    for (int i = r + CS * tid; i < n; i += CS * SY_THREADS) Vt[(long)k * n + i] = i <= k ? 0.0 : v[i];
+    // B: pending update of own rows and their products with v
+    for (int q = q0 + warp; q < nq; q += SY_WARPS) {
+      const int i = r + CS * q;
+      double* row = P + q * ld;
+      const double vi = vp[i], wi = wp[i];
       double acc = 0.0;
-      for (int q = (j + 1 - r + SY_CS - 1) / SY_CS > 0 ? (j + 1 - r + SY_CS - 1) / SY_CS : 0; q < nq; ++q)
-        acc += P[sy_off(r, q) + j] * v[row_of(q)];
-      pp[j] = acc;
-    }
-    __syncthreads();
-    {
-      const int nown = nq - q0;                 // own rows > k
-      int G = 32;
-      while (G > 1 && G * nown > nt) G >>= 1;
-      const int qi = q0 + tid / G, g = tid % G;
-      double acc = 0.0;
-      if (tid / G < nown) {
-        const long off = sy_off(r, qi);
-        for (int l = k + 1 + g; l <= row_of(qi); l += G) acc += P[off + l] * v[l];
+      for (int l = k + 1 + lane; l < n; l += 32) {
+        const double a = fma(-wi, vp[l], fma(-vi, wp[l], row[l]));
+        row[l] = a;
+        acc = fma(a, v[l], acc);
       }
-      for (int o = G >> 1; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
-      if (tid / G < nown && g == 0) pp[row_of(qi)] += acc;
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
+      if (lane < CS) cluster.map_shared_rank(p, lane)[i] = t * acc;
     }
     cluster.sync();
-    // p_j = t sum_r pp_r[j] for every j; p.v; w
-    double pv = 0.0;
-    for (int j = k + 1 + tid; j < n; j += nt) {
-      double part[SY_CS];
+    if (warp == 0) {
+      double pv = 0.0;
+      for (int i = k + 1 + lane; i < n; i += 32) pv = fma(p[i], v[i], pv);
 #pragma unroll
-      for (int rr = 0; rr < SY_CS; ++rr) part[rr] = cluster.map_shared_rank(pp, rr)[j];
-      double acc = 0.0;
-#pragma unroll
-      for (int rr = 0; rr < SY_CS; ++rr) acc += part[rr];
-      const double p = t * acc;
-      sw[j] = p;
-      pv += p * v[j];
+      for (int o = 16; o > 0; o >>= 1) pv += __shfl_xor_sync(0xffffffffu, pv, o);
+      if (lane == 0) s_bc[2] = -0.5 * t * pv;
     }
-    pv = bsum(pv);
-    const double c2 = -0.5 * t * pv;
-    for (int j = k + 1 + tid; j < n; j += nt) sw[j] += c2 * v[j];
     __syncthreads();
-    // own rows: A_il -= v_i w_l + w_i v_l, l in (k, i]
-    {
-      const int nown = nq - q0;
-      int G = 32;
-      while (G > 1 && G * nown > nt) G >>= 1;
-      const int qi = q0 + tid / G, g = tid % G;
-      if (tid / G < nown) {
-        const int i = row_of(qi);
-        const long off = sy_off(r, qi);
-        const double vi = v[i], wi = sw[i];
-        for (int l = k + 1 + g; l <= i; l += G) P[off + l] -= vi * sw[l] + wi * v[l];
-      }
+    const double c2 = s_bc[2];
+    for (int i = k + 1 + tid; i < n; i += SY_THREADS) {
+      const double vi = v[i];
+      vp[i] = vi;
+      wp[i] = fma(c2, vi, p[i]);
     }
     __syncthreads();
   }
+  // the last 2 x 2 block, with the pending update
   if (tid == 0) {
+    const int i1 = n - 1, i2 = n - 2;
     if (n >= 2) {
-      if ((n - 2) % SY_CS == r) d[n - 2] = P[sy_off(r, (n - 2) / SY_CS) + (n - 2)];
-      if ((n - 1) % SY_CS == r) e[n - 2] = P[sy_off(r, (n - 1) / SY_CS) + (n - 2)];
-      if (r == 0) tau[n - 2] = 0.0;
+      if (i2 % CS == r) d[i2] = fma(-2.0 * vp[i2], wp[i2], P[(i2 / CS) * ld + i2]);
+      if (i1 % CS == r) e[i2] = fma(-wp[i1], vp[i2], fma(-vp[i1], wp[i2], P[(i1 / CS) * ld + i2]));
+      if (r == 0) tau[i2] = 0.0;
     }
-    if ((n - 1) % SY_CS == r) d[n - 1] = P[sy_off(r, (n - 1) / SY_CS) + (n - 1)];
-    if (r == 0) tau[n - 1] = 0.0;
+    if (i1 % CS == r) d[i1] = fma(-2.0 * vp[i1], wp[i1], P[(i1 / CS) * ld + i1]);
+    if (r == 0) tau[i1] = 0.0;
   }
-  cluster.sync();   // no CTA leaves while another may still read its shared memory
+  cluster.sync();   // no CTA leaves while another may still write into its shared memory
+}
+
+template <int CS>
+gbhf_status sytrd_config(gbhf_ctx* c, int n, cudaLaunchConfig_t& cfg, cudaLaunchAttribute& attr) {
+  cfg = {};
+  cfg.gridDim = dim3(CS);
+  cfg.blockDim = dim3(SY_THREADS);
+  cfg.dynamicSmemBytes = sy_smem_bytes(n, CS);
+  cfg.stream = c->stream;
+  attr = {};
+  attr.id = cudaLaunchAttributeClusterDimension;
+  attr.val.clusterDim.x = CS;
+  attr.val.clusterDim.y = 1;
+  attr.val.clusterDim.z = 1;
+  cfg.attrs = &attr;
+  cfg.numAttrs = 1;
+  return GBHF_OK;
+}
+
+// Whether this device runs the cluster kernel at its largest size (checked once per context).
+template <int CS>
+bool sytrd_runs(gbhf_ctx* c, int max_n) {
+  // the attributes belong to the kernel (per device, for the whole process): always
+  // the largest size, so that no context lowers it under another's launch
+  bool ok = cudaFuncSetAttribute(k_sytrd_cluster<CS>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 (int)sy_smem_bytes(max_n, CS)) == cudaSuccess;
+  if (CS > 8)
+    ok = ok && cudaFuncSetAttribute(k_sytrd_cluster<CS>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess;
+  if (ok) {
+    cudaLaunchConfig_t cfg;
+    cudaLaunchAttribute attr;
+    sytrd_config<CS>(c, max_n, cfg, attr);
+    int ncl = 0;
+    ok = cudaOccupancyMaxActiveClusters(&ncl, k_sytrd_cluster<CS>, &cfg) == cudaSuccess && ncl >= 1;
+  }
+  (void)cudaGetLastError();   // a refused query leaves no error behind
+  return ok;
+}
+
+template <int CS>
+gbhf_status launch_sytrd(gbhf_ctx* c, int n, const double* d_A, TridiagWork& w) {
+  cudaLaunchConfig_t cfg;
+  cudaLaunchAttribute attr;
+  GBHF_TRY(sytrd_config<CS>(c, n, cfg, attr));
+  GBHF_CUDA(c, cudaLaunchKernelEx(&cfg, k_sytrd_cluster<CS>, n, d_A, w.d.p, w.e.p, w.tau.p, w.Vt.p));
+  count_launch(c);
+  return GBHF_OK;
 }
 
 // Unreduced blocks: e_i is dropped when e_i^2 <= eps^2 |d_i d_(i+1)| (or is
@@ -333,8 +346,9 @@ __global__ void __cluster_dims__(SY_CS, 1, 1) __launch_bounds__(SY_THREADS)
 __global__ void __launch_bounds__(256) k_tri_prep(int n, const double* __restrict__ d, double* __restrict__ e,
                                                   int* __restrict__ blk, double* __restrict__ e2,
                                                   float* __restrict__ df, float* __restrict__ e2f,
-                                                  double* __restrict__ scal) {
-  __shared__ double sd[1024], se[1024];
+                                                  double* __restrict__ scal, int* __restrict__ status) {
+  __shared__ double sd[1025], se[1025];
+  __shared__ bool cut[1024];
   __shared__ double s_red[8];
   const int tid = threadIdx.x;
   for (int i = tid; i < n; i += blockDim.x) {
@@ -347,38 +361,41 @@ __global__ void __launch_bounds__(256) k_tri_prep(int n, const double* __restric
     double r = fabs(sd[i]);
     if (i > 0) r += fabs(se[i - 1]);
     if (i + 1 < n) r += fabs(se[i]);
+    if (status && !(r <= DBL_MAX)) atomicOr(status, GBHF_DEV_ERR_NOTCONV);
     tn = fmax(tn, r);
   }
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) tn = fmax(tn, __shfl_xor_sync(0xffffffffu, tn, o));
   if ((tid & 31) == 0) s_red[tid >> 5] = tn;
   __syncthreads();
+  __syncthreads();
+  for (int w = 0; w < (int)(blockDim.x >> 5); ++w) tn = fmax(tn, s_red[w]);
+  // a row ends its block where the next off-diagonal is negligible
+  double emax2 = 0.0;
+  for (int i = tid; i < n; i += blockDim.x) {
+    const double ee = se[i] * se[i];
+    const bool split = i + 1 == n || se[i] == 0.0 || ee <= kEps * kEps * fabs(sd[i] * sd[i + 1]);
+    cut[i] = split;
+    if (!split) emax2 = fmax(emax2, ee);
+  }
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) emax2 = fmax(emax2, __shfl_xor_sync(0xffffffffu, emax2, o));
+  __syncthreads();   // s_red read above
+  if ((tid & 31) == 0) s_red[tid >> 5] = emax2;
+  __syncthreads();
   if (tid == 0) {
-    for (int w = 1; w < (int)(blockDim.x >> 5); ++w) tn = fmax(tn, s_red[w]);
-    double emax2 = 0.0;
-    int s0 = 0;
-    for (int i = 0; i < n; ++i) {
-      bool split = (i + 1 == n);
-      if (!split) {
-        const double ee = se[i] * se[i];
-        if (se[i] == 0.0 || ee <= kEps * kEps * fabs(sd[i] * sd[i + 1])) {
-          se[i] = 0.0;
-          split = true;
-        } else {
-          emax2 = fmax(emax2, ee);
-        }
-      }
-      if (split) {
-        for (int r = s0; r <= i; ++r) {
-          blk[r] = s0;
-          blk[n + r] = i;
-        }
-        s0 = i + 1;
-      }
-    }
+    for (int w = 1; w < (int)(blockDim.x >> 5); ++w) emax2 = fmax(emax2, s_red[w]);
     scal[0] = fmax(tn, DBL_MIN);
     scal[1] = DBL_MIN * fmax(1.0, emax2);
     scal[2] = (double)FLT_MIN * fmax(1.0, emax2);
+  }
+  for (int i = tid; i < n; i += blockDim.x) {
+    int lo = i, hi = i;
+    while (lo > 0 && !cut[lo - 1]) --lo;
+    while (!cut[hi]) ++hi;
+    blk[i] = lo;
+    blk[n + i] = hi;
+    if (cut[i]) se[i] = 0.0;
   }
   __syncthreads();
   for (int i = tid; i < n; i += blockDim.x) {
@@ -390,27 +407,37 @@ __global__ void __launch_bounds__(256) k_tri_prep(int n, const double* __restric
   }
 }
 
-// 1/q by one Newton-Raphson step, r1 = r0 + r0 (1 - q r0), from the
-// single-precision reciprocal (relative error ~2^-46); outside the single-
-// precision range the plain quotient.  Only the sign of each pivot of a Sturm
-// sequence matters, so this accuracy is ample.
+// 1/q to about an ulp with three FP64 instructions: the single-precision
+// estimate of the truncated q (exponents moved with integer operations), then
+// r0 (1 + h + h^2), h = 1 - q r0 (the neglected h^3 is below 2^-63); outside the
+// single-precision range the plain quotient.
 __device__ __forceinline__ double recip_nr(double q) {
-  const double aq = fabs(q);
-  if (!(aq > 1e-30 && aq < 1e30)) return 1.0 / q;
-  const double r0 = (double)__frcp_rn((float)q);
-  return fma(r0, fma(-q, r0, 1.0), r0);
+  const int hi = __double2hiint(q), ahi = hi & 0x7fffffff;
+  if ((unsigned)(ahi - 0x39b00000) >= 0x0c800000u) return 1.0 / q;   // |q| outside [2^-100, 2^100)
+  const float xf = __int_as_float((ahi - 0x38000000) << 3);
+  float yf;
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(yf) : "f"(xf));
+  const int yb = __float_as_int(yf);
+  const double r0 = __hiloint2double(((yb >> 3) + 0x38000000) | (hi & 0x80000000), yb << 29);
+  const double h = fma(-q, r0, 1.0);
+  return fma(r0, fma(h, h, h), r0);
 }
 
 // Eigenvalues of T - x I below zero in the block [s, t] (Sturm count); e2 = e^2.
+// Five FP64 instructions per row (16 cycles of the SM's FP64 pipe each); signs
+// and the pivot test on the high words.
 __device__ int sturm_count(const double* __restrict__ d, const double* __restrict__ e2, int s, int t, double x,
                            double pivmin) {
-  double q = d[s] - x;
-  if (fabs(q) < pivmin) q = -pivmin;
-  int c = q < 0.0;
+  const int phi = __double2hiint(pivmin);
+  auto guard = [&](double q) {
+    if ((__double2hiint(q) & 0x7fffffff) <= phi && fabs(q) < pivmin) q = -pivmin;
+    return q;
+  };
+  double q = guard(d[s] - x);
+  int c = (unsigned)__double2hiint(q) >> 31;
   for (int i = s + 1; i <= t; ++i) {
-    q = (d[i] - x) - e2[i - 1] * recip_nr(q);
-    if (fabs(q) < pivmin) q = -pivmin;
-    c += q < 0.0;
+    q = guard(fma(-e2[i - 1], recip_nr(q), d[i] - x));
+    c += (unsigned)__double2hiint(q) >> 31;
   }
   return c;
 }
@@ -450,11 +477,11 @@ __device__ void inverse_iteration(const double* __restrict__ d, const double* __
                                   const double* __restrict__ prev, long prev_stride, int nprev) {
   const int lane = threadIdx.x & 31;
   const int m = t - s + 1;
-  double* u0 = w;
-  double* u1 = w + m;
+  double* u0 = w;          // reciprocal pivots
+  double* u1 = w + m;      // first and second superdiagonal of U, divided by the pivot
   double* u2 = w + 2 * m;
-  double* l = w + 3 * m;   // multiplier; sign bit of the pivot flag kept in piv
-  double* piv = w + 4 * m;
+  double* l = w + 3 * m;   // multipliers
+  double* piv = w + 4 * m; // 1: rows i, i + 1 exchanged
   double* x = w + 5 * m;
   const double eps_piv = kEps * tnorm;
   if (lane == 0) {
@@ -464,8 +491,8 @@ __device__ void inverse_iteration(const double* __restrict__ d, const double* __
       const double sub = e[s + i], nd = d[s + i + 1] - lam, ns1 = (i + 2 < m) ? e[s + i + 1] : 0.0;
       if (fabs(r0) >= fabs(sub)) {
         if (r0 == 0.0) r0 = eps_piv;
-        const double mlt = sub / r0;
-        u0[i] = r0;
+        const double rc = recip_nr(r0), mlt = sub * rc;
+        u0[i] = rc;
         u1[i] = r1;
         u2[i] = 0.0;
         l[i] = mlt;
@@ -473,8 +500,8 @@ __device__ void inverse_iteration(const double* __restrict__ d, const double* __
         r0 = nd - mlt * r1;
         r1 = ns1;
       } else {
-        const double mlt = r0 / sub;
-        u0[i] = sub;
+        const double rc = recip_nr(sub), mlt = r0 * rc;
+        u0[i] = rc;
         u1[i] = nd;
         u2[i] = ns1;
         l[i] = mlt;
@@ -484,30 +511,42 @@ __device__ void inverse_iteration(const double* __restrict__ d, const double* __
       }
     }
     if (r0 == 0.0) r0 = eps_piv;
-    u0[m - 1] = r0;
+    u0[m - 1] = 1.0 / r0;
+    u1[m - 1] = u2[m - 1] = 0.0;
   }
   __syncwarp();
-  // u0 now holds the pivots' reciprocals (one division each, across the lanes)
   for (int i = lane; i < m; i += 32) {
-    u0[i] = 1.0 / u0[i];
+    u1[i] *= u0[i];
+    u2[i] *= u0[i];
     x[i] = start_value(seed, i);
   }
   __syncwarp();
+  // the serial chains of a solve are one FP64 FMA per row; a solve that grows
+  // its unit input to within a factor of 100 m of 1 / (eps ||T||) is followed by
+  // one more, at most four in all
+  bool last = false;
   for (int it = 0; it < 4; ++it) {
     if (lane == 0) {
+      double xi = x[0];
+#pragma unroll 4
       for (int i = 0; i + 1 < m; ++i) {
+        double xn = x[i + 1];
         if (piv[i] != 0.0) {
-          const double tmp = x[i];
-          x[i] = x[i + 1];
-          x[i + 1] = tmp;
+          const double tmp = xi;
+          xi = xn;
+          xn = tmp;
         }
-        x[i + 1] -= l[i] * x[i];
+        x[i] = xi;
+        xi = fma(-l[i], xi, xn);
       }
+      x[m - 1] = xi;
+      double x1 = 0.0, x2 = 0.0;
+#pragma unroll 4
       for (int i = m - 1; i >= 0; --i) {
-        double v = x[i];
-        if (i + 1 < m) v -= u1[i] * x[i + 1];
-        if (i + 2 < m) v -= u2[i] * x[i + 2];
-        x[i] = v * u0[i];
+        const double v = fma(-u1[i], x1, fma(-u2[i], x2, x[i] * u0[i]));
+        x[i] = v;
+        x2 = x1;
+        x1 = v;
       }
     }
     __syncwarp();
@@ -525,6 +564,8 @@ __device__ void inverse_iteration(const double* __restrict__ d, const double* __
     const double inv = nrm > 0.0 ? 1.0 / sqrt(nrm) : 0.0;
     for (int i = lane; i < m; i += 32) x[i] *= inv;
     __syncwarp();
+    if (last) break;
+    last = it > 0 && inv * 0.01 < m * kEps * tnorm;   // (the start vector is not normalised)
   }
   for (int i = lane; i < m; i += 32) zrow[s + i] = x[i];
   __syncwarp();
@@ -623,24 +664,30 @@ __global__ void __launch_bounds__(256) k_tri_fix(int n, const double* __restrict
                           const double* __restrict__ lam, double* __restrict__ Zt, int* __restrict__ rank,
                           double* __restrict__ evals) {
   extern __shared__ double smw[];
+  __shared__ double sl[TRIDIAG_WIDE_MAX_N];
+  __shared__ unsigned char close[TRIDIAG_WIDE_MAX_N];
   const double tnorm = scal[0];
+  for (int k = threadIdx.x; k < n; k += blockDim.x) {
+    sl[k] = lam[k];
+    close[k] = k > 0 && blk[k] == blk[k - 1] && blk[k] != blk[n + k] && lam[k] - lam[k - 1] < 1e-11 * tnorm;
+  }
+  __syncthreads();
   if (threadIdx.x < 32) {
     int run0 = 0;
     for (int k = 1; k < n; ++k) {
-      const bool same = blk[k] == blk[k - 1] && blk[k] != blk[n + k];
-      if (!(same && lam[k] - lam[k - 1] < 1e-11 * tnorm)) {
+      if (!close[k]) {
         run0 = k;
         continue;
       }
-      inverse_iteration(d, e, blk[k], blk[n + k], lam[k], tnorm, k + 7919, smw, Zt + (long)k * n,
+      inverse_iteration(d, e, blk[k], blk[n + k], sl[k], tnorm, k + 7919, smw, Zt + (long)k * n,
                         Zt + (long)run0 * n, n, k - run0);
     }
   }
   for (int k = threadIdx.x; k < n; k += blockDim.x) {
-    const double v = lam[k];
+    const double v = sl[k];
     int r = 0;
     for (int q = 0; q < n; ++q) {
-      const double u = lam[q];
+      const double u = sl[q];
       r += (u < v) || (u == v && q < k);
     }
     rank[k] = r;
@@ -660,8 +707,10 @@ __global__ void k_ns_mat(int n, const double* __restrict__ S, double* __restrict
 // per block; each reflector row is loaded once per block into shared memory
 // (double-buffered: row r - 1 loads while row r is applied), one barrier per
 // reflector.
-constexpr int TB_WARPS = 8;
-
+// TB_WARPS 2 (n <= 304: a block per SM) or 4: a warp's 3 n / 32 FP64 instructions
+// per reflector take 16 cycles of its SM's FP64 pipe each (eight warps per block
+// filled 26 of the 152 SMs at n = 208).
+template <int TB_WARPS>
 __global__ void __launch_bounds__(TB_WARPS * 32) k_tri_back(int n, const double* __restrict__ Vt,
                                                             const double* __restrict__ tau,
                                                             const double* __restrict__ Zt,
@@ -703,6 +752,22 @@ __global__ void __launch_bounds__(TB_WARPS * 32) k_tri_back(int n, const double*
 
 size_t tridiag_smem_bytes(int n) { return (size_t)(pidx(n, 0) + 2 * (long)n) * sizeof(double); }
 
+// The widest cluster form that runs here: 16 CTAs, 8, or none.
+static void check_sytrd(gbhf_ctx* c) {
+  if (c->sytrd_checked) return;
+  c->sytrd_checked = true;
+  c->sytrd8 = sytrd_runs<8>(c, SY_WIDE_N);
+  c->sytrd16 = sytrd_runs<16>(c, TRIDIAG_WIDE_MAX_N);
+}
+
+bool tridiag_takes(gbhf_ctx* c, int n) {
+  if (c->force_jacobi) return false;
+  if (n <= TRIDIAG_MAX_N) return tridiag_smem_bytes(n) <= c->smem_optin;
+  if (n > TRIDIAG_WIDE_MAX_N || c->force_sytrd_single) return false;
+  check_sytrd(c);
+  return n <= SY_WIDE_N ? c->sytrd8 || c->sytrd16 : c->sytrd16;
+}
+
 // d_evecs (n x n): eigenvectors of A in columns, ascending eigenvalues.
 gbhf_status eigh_tridiag(gbhf_ctx* c, int n, const double* d_A, double* d_evals, double* d_evecs) {
   TridiagWork& w = c->tri;
@@ -722,7 +787,7 @@ gbhf_status eigh_tridiag(gbhf_ctx* c, int n, const double* d_A, double* d_evals,
   GBHF_CUDA(c, w.M.alloc(nn));
   GBHF_CUDA(c, w.blk.alloc(2 * (size_t)n));
   GBHF_CUDA(c, w.rank.alloc(n));
-  const size_t smem = tridiag_smem_bytes(n);
+  const size_t smem = tridiag_smem_bytes(n);   // of the one-CTA form, n <= TRIDIAG_MAX_N
   // The attribute belongs to the kernel (per device, for the whole process):
   // always the largest size, so that no context lowers it under another's launch.
   GBHF_CUDA(c, cudaFuncSetAttribute(k_sytrd, cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -730,33 +795,31 @@ gbhf_status eigh_tridiag(gbhf_ctx* c, int n, const double* d_A, double* d_evals,
   if (n > 1) {
     GBHF_CUDA(c, cudaMemsetAsync(w.e.p, 0, n * sizeof(double), c->stream));
   }
-  // the cluster form when the device runs an 8-CTA cluster of it (checked once)
-  long sy_loc = 0;
-  for (int r = 0; r < SY_CS; ++r) sy_loc = std::max(sy_loc, sy_local_doubles(n, r));
-  const size_t sy_smem = (size_t)(sy_loc + 4L * n + 8) * sizeof(double);
-  if (c->sytrd_cluster == 0) {
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(SY_CS);
-    cfg.blockDim = dim3(SY_THREADS);
-    cfg.dynamicSmemBytes = (size_t)(sy_local_doubles(TRIDIAG_MAX_N, SY_CS - 1) + 4L * TRIDIAG_MAX_N + 8) * 8;
-    int ncl = 0;
-    const cudaError_t ce = cudaOccupancyMaxActiveClusters(&ncl, k_sytrd_cluster, &cfg);
-    c->sytrd_cluster = (ce == cudaSuccess && ncl >= 1) ? 1 : -1;
-    (void)cudaGetLastError();   // a refused query leaves no error behind
+  // above the one-CTA sizes a matrix with a non-finite entry is reported, as the
+  // Jacobi solver reports it
+  const bool wide = n > TRIDIAG_MAX_N;
+  if (wide) {
+    GBHF_CUDA(c, c->dev_status.alloc(1));
+    GBHF_CUDA(c, cudaMemsetAsync(c->dev_status.p, 0, sizeof(int), c->stream));
   }
-  if (c->sytrd_cluster > 0 && !c->force_sytrd_single && n >= 2 * SY_CS) {
-    k_sytrd_cluster<<<SY_CS, SY_THREADS, sy_smem, c->stream>>>(n, d_A, w.d.p, w.e.p, w.tau.p, w.Vt.p);
-    count_launch(c);
-    GBHF_LAUNCHED(c, "k_sytrd_cluster launch");
+  // the cluster forms where the device runs them; below two rows per CTA one CTA
+  check_sytrd(c);
+  if (c->sytrd8 && !c->force_sytrd_single && n >= 16 && n <= SY_WIDE_N) {
+    GBHF_TRY(launch_sytrd<8>(c, n, d_A, w));
+  } else if (c->sytrd16 && !c->force_sytrd_single && n >= 32) {
+    GBHF_TRY(launch_sytrd<16>(c, n, d_A, w));
   } else {
     k_sytrd<<<1, 1024, smem, c->stream>>>(n, d_A, w.d.p, w.e.p, w.tau.p, w.Vt.p);
     count_launch(c);
     GBHF_LAUNCHED(c, "k_sytrd launch");
   }
-  k_tri_prep<<<1, 256, 0, c->stream>>>(n, w.d.p, w.e.p, w.blk.p, w.e2.p, w.df.p, w.e2f.p, w.scal.p);
+  k_tri_prep<<<1, 256, 0, c->stream>>>(n, w.d.p, w.e.p, w.blk.p, w.e2.p, w.df.p, w.e2f.p, w.scal.p,
+                                      wide ? c->dev_status.p : nullptr);
   count_launch(c);
   GBHF_LAUNCHED(c, "k_tri_prep launch");
   const int wpb = 2;   // warps per block: vectors spread over many SMs
+  GBHF_CUDA(c, cudaFuncSetAttribute(k_tri_vec, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                    (int)(wpb * 6 * TRIDIAG_WIDE_MAX_N * sizeof(double))));
   const size_t vsm = (size_t)wpb * 6 * n * sizeof(double);
   k_tri_vec<<<(n + wpb - 1) / wpb, 32 * wpb, vsm, c->stream>>>(n, w.d.p, w.e.p, w.e2.p, w.df.p, w.e2f.p, w.blk.p,
                                                                w.scal.p, w.lam.p, w.Zt.p);
@@ -777,10 +840,20 @@ gbhf_status eigh_tridiag(gbhf_ctx* c, int n, const double* d_A, double* d_evals,
     GBHF_TRY(gemm(c, false, false, n, n, n, 1.0, w.M.p, n, zin, n, 0.0, zout, n));
     std::swap(zin, zout);
   }
-  k_tri_back<<<(n + TB_WARPS - 1) / TB_WARPS, TB_WARPS * 32, (size_t)(2 + TB_WARPS) * n * sizeof(double),
-               c->stream>>>(n, w.Vt.p, w.tau.p, zin, w.rank.p, d_evecs);
+  if (n <= 304)
+    k_tri_back<2><<<(n + 1) / 2, 64, 4 * (size_t)n * sizeof(double), c->stream>>>(n, w.Vt.p, w.tau.p, zin, w.rank.p,
+                                                                                  d_evecs);
+  else
+    k_tri_back<4><<<(n + 3) / 4, 128, 6 * (size_t)n * sizeof(double), c->stream>>>(n, w.Vt.p, w.tau.p, zin, w.rank.p,
+                                                                                   d_evecs);
   count_launch(c);
   GBHF_LAUNCHED(c, "k_tri_back launch");
+  if (wide) {
+    int st = 0;
+    GBHF_CUDA(c, cudaMemcpyAsync(&st, c->dev_status.p, sizeof(int), cudaMemcpyDeviceToHost, c->stream));
+    GBHF_CUDA(c, cudaStreamSynchronize(c->stream));
+    if (st & GBHF_DEV_ERR_NOTCONV) return fail(c, GBHF_ERR_NOT_CONVERGED, "eigen-solver: non-finite matrix");
+  }
   return GBHF_OK;
 }
 
