@@ -60,20 +60,25 @@ __device__ inline void os_table(double gamma, double s00, double pax, double pbx
     }
 }
 
-// Row i (global function) pairs with the functions j >= i of its molecule;
-// nuclear attraction over that molecule's atoms.  Output: the flat upper
-// triangle of one molecule (moff == nullptr), or both triangles of the
-// molecule's block of stacked square matrices.
-__global__ void k_onee(bool ref, int nbf, const int* __restrict__ fmol, const int* __restrict__ mfo,
+// A warp per function pair (i, j >= i) of a molecule; nuclear attraction over
+// that molecule's atoms.  The lanes take (primitive pair, atom) items, the lane of
+// a primitive pair's first atom its overlap and kinetic terms too, and the values
+// are added in item order - primitive pairs in the reference's nested-loop order,
+// its atoms inside - by every lane from shuffles.  A thread per function pair left
+// a molecule's few dozen threads to walk every item one after another: 1.24 ms for
+// water/STO-3G (28 pairs of 27 items; 0.14 ms here), 28.7 ms for 57 functions (1.1).  Output: the flat upper triangle of one
+// molecule (moff == nullptr), or both triangles of the molecule's block of stacked
+// square matrices.
+__global__ void __launch_bounds__(64) k_onee(bool ref, int nbf, const int* __restrict__ fmol, const int* __restrict__ mfo,
                        const int* __restrict__ mao, const long long* __restrict__ moff, const double* __restrict__ xyz,
                        const double* __restrict__ Z, const int* __restrict__ fn, const double* __restrict__ coef,
                        const double* __restrict__ expo, const double* __restrict__ grid,
                        const double* __restrict__ tab, double* __restrict__ S, double* __restrict__ H) {
-  const int i = blockIdx.y;
+  const int i = blockIdx.y, lane = threadIdx.x & 31;
   const int mol = fmol[i];
   const int f0m = mfo[mol], nm = mfo[mol + 1] - f0m, a0 = mao[mol], a1 = mao[mol + 1];
-  const int il = i - f0m, jl = blockIdx.x * blockDim.x + threadIdx.x;
-  if (jl >= nm || jl < il) return;
+  const int il = i - f0m, jl = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
+  if (jl >= nm || jl < il) return;   // whole warps
   const int j = f0m + jl;
   const DevFn f = load_fn(fn, i), g = load_fn(fn, j);
   const double *A = xyz + 3 * f.atom, *B = xyz + 3 * g.atom;
@@ -89,10 +94,12 @@ __global__ void k_onee(bool ref, int nbf, const int* __restrict__ fmol, const in
   }
   double s_sum = 0, t_sum = 0, v_sum = 0;
   const int L = f.l[0] + f.l[1] + f.l[2] + g.l[0] + g.l[1] + g.l[2];
-  double F[MD_LMAX + 1];
-  double R[MD_D * MD_D * MD_D];
-  for (int p1 = 0; p1 < f.np; ++p1)
-    for (int p2 = 0; p2 < g.np; ++p2) {
+  const int na = a1 - a0, items = f.np * g.np * na;
+  for (int base = 0; base < items; base += 32) {
+    const int r = base + lane;
+    double sv = 0, tv = 0, vv = 0;
+    if (r < items) {
+      const int pp = r / na, cn = a0 + r - pp * na, p1 = pp / g.np, p2 = pp - p1 * g.np;
       const double c1 = coef[f.off + p1], e1 = expo[f.off + p1];
       const double c2 = coef[g.off + p2], e2 = expo[g.off + p2];
       const double p = e1 + e2, mu = e1 * e2 / p;
@@ -103,32 +110,44 @@ __global__ void k_onee(bool ref, int nbf, const int* __restrict__ fmol, const in
         P[x] = (e1 * A[x] + e2 * B[x]) / p;
         const double ab = A[x] - B[x];
         const double ex = exp(-mu * ab * ab);
-        double s[3][5];
         const int l1 = f.l[x], l2 = g.l[x];
-        os_table(p, ex * cte, P[x] - A[x], P[x] - B[x], l1, l2 + 2, s);
-        sx[x] = s[l1][l2];
-        // kinetic 1-D term (tab, IntegralsEvaluation.hs:263-280)
-        tx[x] = -2.0 * e2 * e2 * s[l1][l2 + 2] + e2 * (2 * l2 + 1) * s[l1][l2] -
-                (l2 >= 2 ? 0.5 * l2 * (l2 - 1) * s[l1][l2 - 2] : 0.0);
+        if (cn == a0) {
+          double s[3][5];
+          os_table(p, ex * cte, P[x] - A[x], P[x] - B[x], l1, l2 + 2, s);
+          sx[x] = s[l1][l2];
+          // kinetic 1-D term (tab, IntegralsEvaluation.hs:263-280)
+          tx[x] = -2.0 * e2 * e2 * s[l1][l2 + 2] + e2 * (2 * l2 + 1) * s[l1][l2] -
+                  (l2 >= 2 ? 0.5 * l2 * (l2 - 1) * s[l1][l2 - 2] : 0.0);
+        }
         e_axis(E[x], l1, l2, p, P[x] - A[x], P[x] - B[x], ex);
       }
-      s_sum += (c1 * c2) * (sx[0] * sx[1] * sx[2]);
-      t_sum += c1 * c2 * (tx[0] * sx[1] * sx[2] + sx[0] * tx[1] * sx[2] + sx[0] * sx[1] * tx[2]);
-      // nuclear attraction (vijHermite/mcMurchie, IntegralsEvaluation.hs:395-414)
-      for (int cn = a0; cn < a1; ++cn) {
-        const double* Cc = xyz + 3 * cn;
-        const double PC[3] = {P[0] - Cc[0], P[1] - Cc[1], P[2] - Cc[2]};
-        boys_generic(ref, grid, tab, L, p * (PC[0] * PC[0] + PC[1] * PC[1] + PC[2] * PC[2]), F);
-        hermite_r<MD_LMAX>(L, p, PC[0], PC[1], PC[2], F, R);
-        double sum = 0;
-        for (int t = 0; t <= f.l[0] + g.l[0]; ++t)
-          for (int u = 0; u <= f.l[1] + g.l[1]; ++u)
-            for (int v = 0; v <= f.l[2] + g.l[2]; ++v)
-              sum += E[0].get(f.l[0], g.l[0], t) * E[1].get(f.l[1], g.l[1], u) * E[2].get(f.l[2], g.l[2], v) *
-                     R[(t * MD_D + u) * MD_D + v];
-        v_sum += (-Z[cn]) * (c1 * c2 * 2.0 * (GBHF_PI / p) * sum);
+      if (cn == a0) {
+        sv = (c1 * c2) * (sx[0] * sx[1] * sx[2]);
+        tv = c1 * c2 * (tx[0] * sx[1] * sx[2] + sx[0] * tx[1] * sx[2] + sx[0] * sx[1] * tx[2]);
       }
+      // nuclear attraction (vijHermite/mcMurchie, IntegralsEvaluation.hs:395-414)
+      double F[MD_LMAX + 1];
+      double R[MD_D * MD_D * MD_D];
+      const double* Cc = xyz + 3 * cn;
+      const double PC[3] = {P[0] - Cc[0], P[1] - Cc[1], P[2] - Cc[2]};
+      boys_generic(ref, grid, tab, L, p * (PC[0] * PC[0] + PC[1] * PC[1] + PC[2] * PC[2]), F);
+      hermite_r<MD_LMAX>(L, p, PC[0], PC[1], PC[2], F, R);
+      double sum = 0;
+      for (int t = 0; t <= f.l[0] + g.l[0]; ++t)
+        for (int u = 0; u <= f.l[1] + g.l[1]; ++u)
+          for (int v = 0; v <= f.l[2] + g.l[2]; ++v)
+            sum += E[0].get(f.l[0], g.l[0], t) * E[1].get(f.l[1], g.l[1], u) * E[2].get(f.l[2], g.l[2], v) *
+                   R[(t * MD_D + u) * MD_D + v];
+      vv = (-Z[cn]) * (c1 * c2 * 2.0 * (GBHF_PI / p) * sum);
     }
+    const int here = min(32, items - base);
+    for (int q = 0; q < here; ++q) {
+      s_sum += __shfl_sync(0xffffffffu, sv, q);
+      t_sum += __shfl_sync(0xffffffffu, tv, q);
+      v_sum += __shfl_sync(0xffffffffu, vv, q);
+    }
+  }
+  if (lane) return;
   const double sv = same ? 1.0 : s_sum, hv = t_sum + v_sum;
   if (S) S[out] = sv;
   if (H) H[out] = hv;
@@ -374,7 +393,7 @@ static gbhf_status onee_launch(gbhf_ctx* c, bool ref, bool stacked, double* d_S,
   }
   int max_fn = 0;
   for (int m = 0; m < b.nmol; ++m) max_fn = std::max(max_fn, b.mol_fn_off[m + 1] - b.mol_fn_off[m]);
-  dim3 grid((max_fn + 63) / 64, b.nbf);
+  dim3 grid((max_fn + 1) / 2, b.nbf);
   k_onee<<<grid, 64, 0, c->stream>>>(ref, b.nbf, t.fmol.p, t.mfo.p, t.mao.p, stacked ? t.moff.p : nullptr,
                                       c->d_xyz.p, c->d_Z.p, c->d_fn.p, c->d_coef.p, c->d_exp.p, c->boys_ref.p,
                                       c->boys64.p, d_S, d_H);
@@ -413,18 +432,35 @@ __device__ __forceinline__ void sort_key(long& i, long& j, long& k, long& l) {
   }
 }
 
+// Reference numerics, a warp per quartet (P <= Q): the lanes take its primitive
+// quartets in turn, and the first lane adds their values in the reference's
+// nested-loop order (a screened one is 0).  With a thread per quartet a molecule's
+// few hundred threads walked up to 6^4 primitive quartets each.  Water/STO-3G (406
+// quartets): 5.1 -> 0.18 ms; 35 functions: 118 -> 81 ms; 57 with d: 407 -> 204 ms;
+// bound by the FP64 pipe from some 30 functions on.
 template <int LM>
-__global__ void k_eri_canonical(bool ref, int nbf, const int* __restrict__ pair_i, const int* __restrict__ pair_j,
-                                long npair, const long* __restrict__ off, const double* __restrict__ xyz,
-                                const int* __restrict__ fn, const double* __restrict__ coef,
-                                const double* __restrict__ expo, const double* __restrict__ grid,
-                                const double* __restrict__ tab, double* __restrict__ eri) {
+__global__ void __launch_bounds__(128) k_eri_canonical_ref(int nbf, const int* __restrict__ pair_i,
+                                    const int* __restrict__ pair_j, long npair, const long* __restrict__ off,
+                                    const double* __restrict__ xyz, const int* __restrict__ fn,
+                                    const double* __restrict__ coef, const double* __restrict__ expo,
+                                    const double* __restrict__ grid, const double* __restrict__ tab, int max_terms,
+                                    double* __restrict__ eri) {
+  extern __shared__ double terms_sm[];
   const long P = blockIdx.y;
-  const long Q = (long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (Q >= npair || Q < P) return;
-  const long i = pair_i[P], j = pair_j[P], k = pair_i[Q], l = pair_j[Q];
-  eri[canon_pos(off, nbf, i, j, k, l)] =
-      eri_fn_generic<LM>(ref, xyz, fn, coef, expo, grid, tab, (int)i, (int)j, (int)k, (int)l);
+  const long Q = (long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
+  const int lane = threadIdx.x & 31;
+  if (Q >= npair || Q < P) return;   // whole warps leave together
+  double* term = terms_sm + (size_t)(threadIdx.x >> 5) * max_terms;
+  const int i = pair_i[P], j = pair_j[P], k = pair_i[Q], l = pair_j[Q];
+  const int nr = fn[6 * i + 4] * fn[6 * j + 4] * fn[6 * k + 4] * fn[6 * l + 4];
+  for (int r = lane; r < nr; r += 32)   // one term: r0 = r with a step past the end
+    term[r] = eri_fn_generic<LM>(true, xyz, fn, coef, expo, grid, tab, i, j, k, l, r, nr);
+  __syncwarp();
+  if (lane) return;
+  double v = 0;
+#pragma unroll 8
+  for (int r = 0; r < nr; ++r) v += term[r];
+  eri[canon_pos(off, nbf, i, j, k, l)] = v;
 }
 
 // The same array with a warp per (P <= Q): the lanes take the quartet's
@@ -458,13 +494,13 @@ static void canonical_offsets(long n, std::vector<long>& off) {
     }
 }
 
-struct CanonAux {
-  DBuf<int> pi, pj;
-  DBuf<long> off;
-};
-
-static gbhf_status canon_aux(gbhf_ctx* c, CanonAux& aux) {
+// Pair and offset tables of the canonical order; they depend on the number of
+// functions alone and stay with the context.
+static gbhf_status canon_aux(gbhf_ctx* c) {
+  CanonAux& aux = c->canon;
   const long n = c->basis.nbf, np = n * (n + 1) / 2;
+  if (aux.n == n) return GBHF_OK;
+  aux.n = -1;
   std::vector<int> hi(np), hj(np);
   long q = 0;
   for (long i = 0; i < n; ++i)
@@ -481,6 +517,7 @@ static gbhf_status canon_aux(gbhf_ctx* c, CanonAux& aux) {
   GBHF_CUDA(c, cudaMemcpyAsync(aux.pj.p, hj.data(), np * sizeof(int), cudaMemcpyHostToDevice, c->stream));
   GBHF_CUDA(c, cudaMemcpyAsync(aux.off.p, off.data(), n * n * sizeof(long), cudaMemcpyHostToDevice, c->stream));
   GBHF_CUDA(c, cudaStreamSynchronize(c->stream));
+  aux.n = n;
   return GBHF_OK;
 }
 
@@ -488,14 +525,13 @@ gbhf_status eri_canonical_dev(gbhf_ctx* c, bool ref, double* d_eri) {
   const Basis& b = c->basis;
   if (b.maxL > 2) return fail(c, GBHF_ERR_UNSUPPORTED, "canonical ERIs support s, p and d functions");
   if (ref && !c->have_grid) return fail(c, GBHF_ERR_BAD_INPUT, "reference mode needs gbhf_set_boys_grid");
-  CanonAux aux;
-  GBHF_TRY(canon_aux(c, aux));
+  GBHF_TRY(canon_aux(c));
+  const CanonAux& aux = c->canon;
   const long np = (long)b.nbf * (b.nbf + 1) / 2;
   if (np > 65535) return fail(c, GBHF_ERR_UNSUPPORTED, "canonical ERI array too large");
-  dim3 grid((unsigned)((np + 127) / 128), (unsigned)np);
   // per-thread Hermite cubes sized for the largest total angular momentum: s/p quartets L <= 4, d L <= 8
-  if (!ref) {   // exact numerics: a warp per quartet (the reference mode keeps its serial primitive order)
-    dim3 wgrid((unsigned)((np + 3) / 4), (unsigned)np);
+  const dim3 wgrid((unsigned)((np + 3) / 4), (unsigned)np);
+  if (!ref) {
     if (b.maxL <= 1)
       k_eri_canonical_warp<MD_LMAX><<<wgrid, 128, 0, c->stream>>>(ref, b.nbf, aux.pi.p, aux.pj.p, np, aux.off.p,
                                                                   c->d_xyz.p, c->d_fn.p, c->d_coef.p, c->d_exp.p,
@@ -504,17 +540,22 @@ gbhf_status eri_canonical_dev(gbhf_ctx* c, bool ref, double* d_eri) {
       k_eri_canonical_warp<8><<<wgrid, 128, 0, c->stream>>>(ref, b.nbf, aux.pi.p, aux.pj.p, np, aux.off.p,
                                                             c->d_xyz.p, c->d_fn.p, c->d_coef.p, c->d_exp.p,
                                                             c->boys_ref.p, c->boys64.p, d_eri);
-  } else if (b.maxL <= 1)
-    k_eri_canonical<MD_LMAX><<<grid, 128, 0, c->stream>>>(ref, b.nbf, aux.pi.p, aux.pj.p, np, aux.off.p, c->d_xyz.p,
-                                                          c->d_fn.p, c->d_coef.p, c->d_exp.p, c->boys_ref.p,
-                                                          c->boys64.p, d_eri);
-  else
-    k_eri_canonical<8><<<grid, 128, 0, c->stream>>>(ref, b.nbf, aux.pi.p, aux.pj.p, np, aux.off.p, c->d_xyz.p,
-                                                    c->d_fn.p, c->d_coef.p, c->d_exp.p, c->boys_ref.p, c->boys64.p,
-                                                    d_eri);
+  } else {
+    int mp = 1;   // at most 6 primitives a function: 6^4 terms, 41 KB for the four warps
+    for (int i = 0; i < b.nbf; ++i) mp = std::max(mp, b.cgf_nprim[i]);
+    const int terms = mp * mp * mp * mp;
+    const size_t smem = 4 * (size_t)terms * sizeof(double);
+    if (b.maxL <= 1)
+      k_eri_canonical_ref<MD_LMAX><<<wgrid, 128, smem, c->stream>>>(b.nbf, aux.pi.p, aux.pj.p, np, aux.off.p, c->d_xyz.p,
+                                                                    c->d_fn.p, c->d_coef.p, c->d_exp.p,
+                                                                    c->boys_ref.p, c->boys64.p, terms, d_eri);
+    else
+      k_eri_canonical_ref<8><<<wgrid, 128, smem, c->stream>>>(b.nbf, aux.pi.p, aux.pj.p, np, aux.off.p, c->d_xyz.p,
+                                                              c->d_fn.p, c->d_coef.p, c->d_exp.p, c->boys_ref.p,
+                                                              c->boys64.p, terms, d_eri);
+  }
   count_launch(c);
   GBHF_CUDA(c, cudaGetLastError());
-  GBHF_CUDA(c, cudaStreamSynchronize(c->stream));
   return GBHF_OK;
 }
 
@@ -545,14 +586,13 @@ __global__ void k_fock_canonical(int n, const long* __restrict__ off, const doub
 }
 
 gbhf_status fock_canonical_dev(gbhf_ctx* c, const double* d_H, const double* d_D, const double* d_eri, double* d_F) {
-  CanonAux aux;
-  GBHF_TRY(canon_aux(c, aux));
+  GBHF_TRY(canon_aux(c));
+  const CanonAux& aux = c->canon;
   const int n = c->basis.nbf;
   dim3 grid((n + 63) / 64, n);
   k_fock_canonical<<<grid, 64, 0, c->stream>>>(n, aux.off.p, d_H, d_D, d_eri, d_F);
   count_launch(c);
   GBHF_CUDA(c, cudaGetLastError());
-  GBHF_CUDA(c, cudaStreamSynchronize(c->stream));
   return GBHF_OK;
 }
 
@@ -565,11 +605,42 @@ namespace gbhf {
 // grid[m*1001+i] = boysF m (0.1 i).  boysF (Boys.hs:54-66): m = 0 from erf
 // (asymptotic beyond 50); m >= 1 by Kummer's integral with the 256-point
 // Gauss-Legendre rule that kummer selects for err = 0.1 (Boys.hs:106-118).
-__global__ void k_boys_ref_grid(const double* __restrict__ xq, const double* __restrict__ wq, int nq,
-                                double* __restrict__ grid) {
-  const int idx = blockIdx.x * blockDim.x + threadIdx.x;
-  if (idx >= 15 * 1001) return;
-  const int m = idx / 1001, i = idx % 1001;
+// pw[m - 1][side][k] = t^(m - 1/2) at the two nodes of pair k: the factor of the
+// integrand that no grid point changes.
+constexpr int BG_NODES = 128, BG_ORDERS = 14, BG_POINTS = 8;
+__global__ void __launch_bounds__(BG_NODES) k_boys_ref_powers(const double* __restrict__ xq, double* __restrict__ pw) {
+  const int k = threadIdx.x, side = blockIdx.x;
+  const double n = blockIdx.y + 1, a = n + 0.5;
+  const double t = 0.5 * ((1.0 - 0.0) * (side ? -xq[k] : xq[k]) + 1.0 + 0.0);
+  pw[(blockIdx.y * 2 + side) * BG_NODES + k] = pow(t, a - 1);
+}
+
+// The integrand is e^(-x t) (1 - t)^(b - a - 1) t^(a - 1) with b - a = 1: its first
+// factor is the same for every order, its second is 1, its third for every point.
+// So a block takes 8 points and computes their 2 x 128 exponentials once; a thread
+// per (order, point) then adds the 128 weighted pairs in node order.  126 blocks,
+// one wave, 0.10 ms.  (A thread per order and point computed all of them: 2.6 ms,
+// bound by the FP64 pipe in the power function.)
+__global__ void __launch_bounds__(BG_NODES) k_boys_ref_grid(const double* __restrict__ xq,
+                                                            const double* __restrict__ wq,
+                                                            const double* __restrict__ pw,
+                                                            double* __restrict__ grid) {
+  __shared__ double ex[2][BG_POINTS][BG_NODES + 1];
+  const int i0 = blockIdx.x * BG_POINTS;
+  const double e = exp(1.0);
+  {
+    const int k = threadIdx.x;
+    const double t1 = 0.5 * ((1.0 - 0.0) * xq[k] + 1.0 + 0.0);
+    const double t2 = 0.5 * ((1.0 - 0.0) * (-xq[k]) + 1.0 + 0.0);
+    for (int q = 0; q < BG_POINTS; ++q) {
+      const double z = -(0.1 * (i0 + q));
+      ex[0][q][k] = pow(e, z * t1);
+      ex[1][q][k] = pow(e, z * t2);
+    }
+  }
+  __syncthreads();
+  const int q = threadIdx.x % BG_POINTS, m = threadIdx.x / BG_POINTS, i = i0 + q;
+  if (i > 1000 || m > BG_ORDERS) return;
   const double x = 0.1 * i;
   double v;
   if (m == 0) {
@@ -577,20 +648,16 @@ __global__ void k_boys_ref_grid(const double* __restrict__ xq, const double* __r
     else if (x > 0.0) v = 0.5 * sqrt(GBHF_PI / x) * erf(sqrt(x));
     else v = 1.0;
   } else {
-    const double n = m, a = n + 0.5, b = n + 1.5, z = -x;
+    const double n = m, a = n + 0.5, b = n + 1.5;
     const double gamma_factor = tgamma(b) / (tgamma(a) * tgamma(b - a));
-    const double e = exp(1.0);
+    const double *p1 = pw + (size_t)(m - 1) * 2 * BG_NODES, *p2 = p1 + BG_NODES;
     double acc = 0;
-    for (int k = 0; k < nq; ++k) {
-      const double t1 = 0.5 * ((1.0 - 0.0) * xq[k] + 1.0 + 0.0);
-      const double t2 = 0.5 * ((1.0 - 0.0) * (-xq[k]) + 1.0 + 0.0);
-      const double f1 = (pow(e, z * t1) * pow(1 - t1, b - a - 1)) * pow(t1, a - 1);
-      const double f2 = (pow(e, z * t2) * pow(1 - t2, b - a - 1)) * pow(t2, a - 1);
-      acc += wq[k] * (f1 + f2);
-    }
+#pragma unroll 8
+    for (int k = 0; k < BG_NODES; ++k)
+      acc += wq[k] * (__dmul_rn(ex[0][q][k], p1[k]) + __dmul_rn(ex[1][q][k], p2[k]));
     v = gamma_factor * (0.5 * (1.0 - 0.0) * acc) / (2 * n + 1);
   }
-  grid[idx] = v;
+  grid[m * 1001 + i] = v;
 }
 
 // Positive Gauss-Legendre nodes/weights of the n-point rule, ascending
@@ -626,15 +693,24 @@ static void gauss_legendre_pos(int n, std::vector<double>& xs, std::vector<doubl
   }
 }
 
+// The rule's nodes and weights, computed once per process (long double, software
+// quad precision on some hosts: 16 ms there).
+struct GaussLegendre256 {
+  std::vector<double> x, w;
+  GaussLegendre256() { gauss_legendre_pos(2 * BG_NODES, x, w); }
+};
+
 gbhf_status boys_ref_grid_dev(gbhf_ctx* c, double* d_grid) {
-  std::vector<double> xs, wsv;
-  gauss_legendre_pos(256, xs, wsv);
-  DBuf<double> dx, dw;
-  GBHF_CUDA(c, dx.alloc(xs.size()));
-  GBHF_CUDA(c, dw.alloc(wsv.size()));
-  GBHF_CUDA(c, cudaMemcpyAsync(dx.p, xs.data(), xs.size() * sizeof(double), cudaMemcpyHostToDevice, c->stream));
-  GBHF_CUDA(c, cudaMemcpyAsync(dw.p, wsv.data(), wsv.size() * sizeof(double), cudaMemcpyHostToDevice, c->stream));
-  k_boys_ref_grid<<<(15 * 1001 + 127) / 128, 128, 0, c->stream>>>(dx.p, dw.p, (int)xs.size(), d_grid);
+  static const GaussLegendre256 gl;   // thread-safe one-time initialisation
+  DBuf<double> dx, dw, pw;
+  GBHF_CUDA(c, pw.alloc(2 * BG_NODES * BG_ORDERS));
+  GBHF_CUDA(c, dx.alloc(BG_NODES));
+  GBHF_CUDA(c, dw.alloc(BG_NODES));
+  GBHF_CUDA(c, cudaMemcpyAsync(dx.p, gl.x.data(), BG_NODES * sizeof(double), cudaMemcpyHostToDevice, c->stream));
+  GBHF_CUDA(c, cudaMemcpyAsync(dw.p, gl.w.data(), BG_NODES * sizeof(double), cudaMemcpyHostToDevice, c->stream));
+  k_boys_ref_powers<<<dim3(2, BG_ORDERS), BG_NODES, 0, c->stream>>>(dx.p, pw.p);
+  count_launch(c);
+  k_boys_ref_grid<<<(1001 + BG_POINTS - 1) / BG_POINTS, BG_NODES, 0, c->stream>>>(dx.p, dw.p, pw.p, d_grid);
   count_launch(c);
   GBHF_CUDA(c, cudaGetLastError());
   GBHF_CUDA(c, cudaStreamSynchronize(c->stream));

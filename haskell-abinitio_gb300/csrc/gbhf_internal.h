@@ -267,6 +267,13 @@ struct TaskLists {
   long f0_gen = -1;                    // basis generation f0 was uploaded for
 };
 
+// Tables of the canonical ERI order for n functions (eri_canon.cu).
+struct CanonAux {
+  DBuf<int> pi, pj;
+  DBuf<long> off;
+  long n = -1;
+};
+
 struct JacobiWork {
   DBuf<double> A, A2, V, rot, red, t1, t2, t3;
   DBuf<int> sweeps;
@@ -333,6 +340,7 @@ struct gbhf_ctx {
   // dense work buffers (n*n doubles)
   gbhf::DBuf<double> w[24];
   gbhf::JacobiWork jac;
+  gbhf::CanonAux canon;
   gbhf::TridiagWork tri;
   size_t smem_optin = 0;          // largest dynamic shared memory per block (opt-in)
   bool force_jacobi = false;      // GBHF_EIGEN=jacobi at gbhf_create: every eigen-solve by Jacobi
