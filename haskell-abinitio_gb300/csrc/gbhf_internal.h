@@ -367,7 +367,8 @@ struct gbhf_ctx {
   gbhf::DBuf<int> dff_exp;          // e
   gbhf::DBuf<int> dev_status;
   int purify_grid = 0;              // co-resident blocks of the fused purification kernel
-  int tc2_grid = 0;                 // co-resident blocks of the one-barrier TC2 kernel
+  int tc2_per_sm = 0;               // blocks per SM of the one-barrier TC2 kernel (0: not asked yet)
+  int small_dense = -1;             // the one-launch forms of small_dense.cu run here (-1: not asked yet)
   bool purify_defer = false;        // purify leaves its check to the next reduce_stats (SCF loop)
   bool purify_pending = false;      // a purification record waits in small[PURIFY_REC..+2]
   int purify_ne = 0;                // electrons of the pending purification
@@ -547,6 +548,15 @@ gbhf_status diagonal_hf_dev(gbhf_ctx* c, int n, const double* d_Fsq, const doubl
                             double* d_Dsq, double* d_eps, double* d_Cprime_warm);
 gbhf_status diis_error_dev(gbhf_ctx* c, int n, const double* d_F, const double* d_S, const double* d_D,
                            const double* d_X, double* d_e);
+// small_dense.cu: the same three steps for small n, one launch each.  d_rec: the
+// purification record; d_out: the last max |Z Y - I| and the iterations.
+constexpr int SMALL_DENSE_MAX_N = 56;   // matrices the shared memory and the kernels are laid out for
+constexpr int SMALL_DIIS_MAX_N = 40;    // (small_dense.cu has the figures of both sides)
+bool small_dense_takes(gbhf_ctx* c, int n);
+gbhf_status density_small(gbhf_ctx* c, int n, int ne, const double* d_F, const double* d_X, double* d_D, double* d_rec);
+gbhf_status inv_sqrt_small(gbhf_ctx* c, int n, const double* d_S, double* d_X, double* d_out);
+gbhf_status diis_error_small(gbhf_ctx* c, int n, const double* d_F, const double* d_S, const double* d_D,
+                             const double* d_X, double* d_e);
 gbhf_status gauss_elem_dev_call(gbhf_ctx* c, int m, const double* h_a, const double* h_b, double* h_x, bool* ok);
 // scf.cu
 gbhf_status scf_run(gbhf_ctx* c, const gbhf_scf_opts* o, gbhf_result* r);

@@ -187,74 +187,57 @@ __global__ void __launch_bounds__(128) k_dgemm_split(bool ta, bool tb, bool sym,
   dgemm_tile(ta, tb, sym, m, n, blockIdx.y, blockIdx.x, k0, k1, alpha, A, lda, B, ldb, C, ldc, nullptr, sm);
 }
 
-// Small-matrix variant on warp units: one warp per (16 x 16 tile of C, 16-long
-// k chunk), fragments of op(A) and op(B) loaded straight from global memory
-// (L2-resident for these sizes), DMMA, then alpha * partial added to C with
-// FP64 atomics (C pre-scaled by beta).  sym: only tiles on and above the
-// diagonal, each added at its mirror as well.  With 16 DMMA per unit the work
-// spreads evenly over every SM where 32 x 32 tiles leave SMs idle or doubled.
-constexpr int WG_T = 16, WG_K = 16, WG_THREADS = 256;
+// Small-matrix variant, one launch: a block per 8 x 8 tile of C, its four warps
+// taking 4-long k steps in turn, fragments of op(A) and op(B) straight from global
+// memory (L2-resident for these sizes), DMMA, and the four partial tiles summed in
+// shared memory.  sym: only tiles on and above the diagonal, each written at its
+// mirror as well.  Its predecessor (a warp per 16 x 16 tile and 16-long k chunk)
+// added its partials to a pre-scaled C with FP64 atomics, a second launch:
+// the DIIS error (four products) at n = 78 0.164 -> 0.114 ms, 104 0.167 -> 0.122, 208
+// 0.218 -> 0.199, 832 4.77 -> 4.50.
+constexpr int WG_T = 8, WG_THREADS = 128;
 
-__global__ void __launch_bounds__(WG_THREADS) k_dgemm_warp(bool ta, bool tb, bool sym, int m, int n, int k,
+__global__ void __launch_bounds__(WG_THREADS) k_dgemm_tile(bool ta, bool tb, bool sym, int m, int n, int k,
                                                            double alpha, const double* __restrict__ A, int lda,
-                                                           const double* __restrict__ B, int ldb,
+                                                           const double* __restrict__ B, int ldb, double beta,
                                                            double* __restrict__ C, int ldc) {
-  const int lane = threadIdx.x & 31;
-  const int gwarp = blockIdx.x * (WG_THREADS / 32) + (threadIdx.x >> 5), nwarps = gridDim.x * (WG_THREADS / 32);
-  const int mt = (m + WG_T - 1) / WG_T, ntl = (n + WG_T - 1) / WG_T, nkc = (k + WG_K - 1) / WG_K;
-  const long ntiles = sym ? (long)ntl * (ntl + 1) / 2 : (long)mt * ntl;
-  const long units = ntiles * nkc;
+  const int ct = blockIdx.x, rt = blockIdx.y;
+  if (sym && ct < rt) return;
+  __shared__ double part[WG_THREADS / 32][WG_T * WG_T];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int r = lane >> 2, q = lane & 3;
-  for (long u = gwarp; u < units; u += nwarps) {
-    long t = u / nkc;
-    const int kc = (int)(u - t * nkc);
-    int rt, ct;
-    if (sym) {
-      rt = 0;
-      while (t >= ntl - rt) {
-        t -= ntl - rt;
-        ++rt;
-      }
-      ct = rt + (int)t;
-    } else {
-      rt = (int)(t / ntl);
-      ct = (int)(t - (long)rt * ntl);
+  const int row = rt * WG_T + r, col = ct * WG_T + r;
+  const bool rok = row < m, cok = col < n;
+  const double* pa = A + (ta ? (long)row : (long)row * lda);
+  const double* pb = B + (tb ? (long)col * ldb : (long)col);
+  const long sa = ta ? lda : 1, sb = tb ? 1 : ldb;
+  double x[2] = {0, 0}, y[2] = {0, 0};
+  constexpr int KS = 4 * (WG_THREADS / 32);   // k step of the block
+  for (int k0 = 4 * warp; k0 < k; k0 += 4 * KS) {
+    double af[4], bf[4];
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      const int kk = k0 + u * KS + q;
+      af[u] = rok && kk < k ? pa[kk * sa] : 0.0;
+      bf[u] = cok && kk < k ? pb[kk * sb] : 0.0;
     }
-    const int k0 = kc * WG_K;
-    double af[WG_K / 4][2], bf[WG_K / 4][2];
-#pragma unroll
-    for (int k4 = 0; k4 < WG_K / 4; ++k4) {
-      const int kk = k0 + 4 * k4 + q;
-#pragma unroll
-      for (int i = 0; i < 2; ++i) {
-        const int row = rt * WG_T + 8 * i + r, col = ct * WG_T + 8 * i + r;
-        double va = 0.0, vb = 0.0;
-        if (row < m && kk < k) va = ta ? A[(long)kk * lda + row] : A[(long)row * lda + kk];
-        if (col < n && kk < k) vb = tb ? B[(long)col * ldb + kk] : B[(long)kk * ldb + col];
-        af[k4][i] = va;
-        bf[k4][i] = vb;
-      }
-    }
-    double acc[2][2][2] = {};
-#pragma unroll
-    for (int k4 = 0; k4 < WG_K / 4; ++k4)
-#pragma unroll
-      for (int i = 0; i < 2; ++i)
-#pragma unroll
-        for (int j = 0; j < 2; ++j) dmma(acc[i][j][0], acc[i][j][1], af[k4][i], bf[k4][j]);
-#pragma unroll
-    for (int i = 0; i < 2; ++i)
-#pragma unroll
-      for (int j = 0; j < 2; ++j)
-#pragma unroll
-        for (int h = 0; h < 2; ++h) {
-          const int row = rt * WG_T + 8 * i + r, col = ct * WG_T + 8 * j + 2 * q + h;
-          if (row < m && col < n) {
-            const double v = alpha * acc[i][j][h];
-            atomicAdd(C + (long)row * ldc + col, v);
-            if (sym && rt < ct) atomicAdd(C + (long)col * ldc + row, v);
-          }
-        }
+    dmma(x[0], x[1], af[0], bf[0]);
+    if (k0 + KS < k) dmma(y[0], y[1], af[1], bf[1]);
+    if (k0 + 2 * KS < k) dmma(x[0], x[1], af[2], bf[2]);
+    if (k0 + 3 * KS < k) dmma(y[0], y[1], af[3], bf[3]);
+  }
+  part[warp][r * WG_T + 2 * q] = x[0] + y[0];
+  part[warp][r * WG_T + 2 * q + 1] = x[1] + y[1];
+  __syncthreads();
+  if (threadIdx.x >= WG_T * WG_T) return;
+  const int e = threadIdx.x, i = rt * WG_T + e / WG_T, j = ct * WG_T + e % WG_T;
+  if (i >= m || j >= n) return;
+  const double v = alpha * ((part[0][e] + part[1][e]) + (part[2][e] + part[3][e]));
+  double* p = C + (long)i * ldc + j;
+  *p = beta == 0.0 ? v : fma(beta, *p, v);
+  if (sym && rt < ct) {
+    p = C + (long)j * ldc + i;
+    *p = beta == 0.0 ? v : fma(beta, *p, v);
   }
 }
 
@@ -278,15 +261,9 @@ gbhf_status gemm(gbhf_ctx* c, bool ta, bool tb, int m, int n, int k, double alph
     return GBHF_OK;
   }
   if (m <= 1024 && n <= 1024) {
-    // warp units: (16 x 16 tile, 16-long k chunk), about eight per SM or fewer
-    const long t16 = sym ? (long)((n + WG_T - 1) / WG_T) * ((n + WG_T - 1) / WG_T + 1) / 2
-                         : (long)((m + WG_T - 1) / WG_T) * ((n + WG_T - 1) / WG_T);
-    const long units = t16 * ((k + WG_K - 1) / WG_K);
-    const int grid = (int)std::max(1L, std::min<long>((units + WG_THREADS / 32 - 1) / (WG_THREADS / 32),
-                                                      4L * c->nsm));
-    k_scale_matrix<<<dim3((n + 127) / 128, m), 128, 0, c->stream>>>(m, n, beta, C, ldc);
-    k_dgemm_warp<<<grid, WG_THREADS, 0, c->stream>>>(ta, tb, sym, m, n, k, alpha, A, lda, B, ldb, C, ldc);
-    count_launch(c, 2);
+    const dim3 grid((n + WG_T - 1) / WG_T, (m + WG_T - 1) / WG_T);
+    k_dgemm_tile<<<grid, WG_THREADS, 0, c->stream>>>(ta, tb, sym, m, n, k, alpha, A, lda, B, ldb, beta, C, ldc);
+    count_launch(c);
     GBHF_CUDA(c, cudaGetLastError());
     return GBHF_OK;
   }
@@ -1132,173 +1109,143 @@ __global__ void __launch_bounds__(128) k_purify_fused(PurifyArgs a) {
   }
 }
 
-// Trace-correcting purification with one grid barrier per step.  Step s
-// computes P2_s = P_s P_s while P_s itself is only formed on the fly:
-// P_s = ca P_(s-1) + cb P2_(s-1) (tc2_next) when the GEMM tiles are loaded, and
-// written out (for step s + 1) by a strided pass that runs beside the GEMM.
-// P alternates between two buffers, P2 rotates over three (the one zeroed in
-// step s was last read in step s - 1), and the traces of P_s and P2_s sit in
-// three rotating slots, so that the single barrier at the end of a step is the
-// only ordering needed.  After the barrier every block takes the same step
-// decision from the same two traces.
+// Trace-correcting purification with one grid barrier per step.  A block owns
+// 8 x 8 tiles of P^2 on or above the diagonal, its four warps taking 4-long k steps
+// in turn (fragments straight from L2; P is exactly symmetric, so the column
+// fragment of B is a row fragment of P), and writes both candidates for the next P,
+// P^2 and 2 P - P^2, with its part of their traces.  After the barrier every block
+// adds the same partial traces in the same order, so all take the same decision and
+// the next P is already in memory: no atomics, no pass that forms it.  The three
+// buffers rotate: a step reads one and writes the other two, whose last readers are
+// behind the barrier.
+// The density step it closes (28 steps, four products), against 16 x 16 tiles split
+// over k with atomics and P formed while loading: n = 104 0.615 -> 0.246 ms, 208
+// 0.674 -> 0.632, 312 1.99 -> 1.45, 832 25.1 -> 19.6.  Bound by the FP64 pipe from
+// n = 208 on (52 DMMA a tile at some 140 cycles of the SM's pipe, up to three tiles
+// an SM: 11 of 19 us a step), by the barrier and L2 latency below (5 of 7 us at 104).
+// Loading more than 4 k steps ahead gains nothing and 16 cost 10%.
 struct Tc2Args {
   int n, ne, max_steps;
   double tol;
-  double *P0, *P1;        // P0 holds P_0 at launch; the result is copied back there
-  double *Q0, *Q1, *Q2;   // the three P2 buffers, zero at launch
-  double* tr;        // 6 slots: tr P_s at 2 (s % 3), tr P2_s at 2 (s % 3) + 1; zero at launch
-  double* out;       // [0] last tr(P - P^2), [1] steps
+  double *P0, *P1, *P2;   // P0 holds P_0 at launch; the result is copied back there
+  double* dg;             // partial traces: [step parity][candidate][2 nt]
+  double* out;            // [0] last tr(P - P^2), [1] steps
   unsigned* bar;
   int* status;
 };
 
-// The one formula for an element of P_s, used by the GEMM loads and by the
-// pass that writes P_s out, so that both give the same bits.
-__device__ __forceinline__ double tc2_next(double ca, double cb, double p, double p2) {
-  return __fma_rn(ca, p, __dmul_rn(cb, p2));
-}
-
-// GEMM units of a step: (16 x 16 tile on or above the diagonal, 16-long k
-// chunk), one warp each, fragments loaded straight from global memory (P_s is
-// exactly symmetric, so the column fragment of B is a row fragment of P_s) and
-// multiplied by DMMA; the tile (and its mirror) is added into P2_s with FP64
-// atomics.  256 threads per block.
-constexpr int TC2_THREADS = 256, TC2_T = 16, TC2_K = 16;
+constexpr int TC2_THREADS = 128, TC2_T = 8;
 
 __global__ void __launch_bounds__(TC2_THREADS) k_tc2_fused(Tc2Args a) {
-  __shared__ double s_red[TC2_THREADS / 32];
+  constexpr int W = TC2_THREADS / 32, KS = 4 * W, U = 4;   // k step of the block, steps in flight
+  __shared__ double part[W][TC2_T * TC2_T];
+  __shared__ double s_t[W];
   const int n = a.n, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const long nn = (long)n * n;
-  const int nt = (n + TC2_T - 1) / TC2_T, nkc = (n + TC2_K - 1) / TC2_K;
-  const int units = nt * (nt + 1) / 2 * nkc;
-  const int gwarp = blockIdx.x * (TC2_THREADS / 32) + warp, nwarps = gridDim.x * (TC2_THREADS / 32);
-  const long gt = blockIdx.x * (long)blockDim.x + tid, gs = (long)gridDim.x * blockDim.x;
+  const int nt = (n + TC2_T - 1) / TC2_T, ntiles = nt * (nt + 1) / 2;
+  const int r = lane >> 2, q = lane & 3;
   unsigned epoch = 0;
-  auto block_sum_add = [&](double v, double* dst) {
+  {   // tr P_0
+    double v = 0;
+    for (int i = tid; i < n; i += TC2_THREADS) v += a.P0[(long)i * n + i];
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-    if (lane == 0) s_red[warp] = v;
+    if (lane == 0) s_t[warp] = v;
     __syncthreads();
-    if (tid == 0) {
-      double t = 0.0;
-#pragma unroll
-      for (int w = 0; w < TC2_THREADS / 32; ++w) t += s_red[w];
-      if (t != 0.0) atomicAdd(dst, t);
-    }
-    __syncthreads();
-  };
-  auto pbuf = [&](int i) -> double* { return i == 0 ? a.P0 : a.P1; };
-  auto qbuf = [&](int i) -> double* { return i == 0 ? a.Q0 : (i == 1 ? a.Q1 : a.Q2); };
-  {
-    double v = 0;
-    for (long i = gt; i < n; i += gs) v += a.P0[i * n + i];
-    block_sum_add(v, a.tr);   // tr P_0 in slot 0
   }
-  if (!grid_barrier(a.bar, epoch, a.status)) return;
-  double ca = 1.0, cb = 0.0;   // P_s = ca P_(s-1) + cb P2_(s-1); step 0 reads P_0 as it is
-  int step = 0, final_buf = 0;
-  for (; step < a.max_steps; ++step) {
-    const double* Pin = pbuf(step == 0 ? 0 : (step - 1) & 1);   // P_(s-1) (P_0 at step 0)
-    const double* P2in = qbuf(step == 0 ? 2 : (step - 1) % 3);  // P2_(s-1) (zero at step 0)
-    double* Pout = pbuf(step & 1);
-    double* P2out = qbuf(step % 3);
-    double* trp = a.tr + 2 * (step % 3);
-    // the slots of step s + 1, last read after the barrier of step s - 2
-    if (gt == 0) {
-      a.tr[2 * ((step + 1) % 3)] = 0.0;
-      a.tr[2 * ((step + 1) % 3) + 1] = 0.0;
-    }
-    if (step > 0) {
-      // P_s written out with its trace (step 0: P_0 is already in P0), and the
-      // P2 buffer of step s + 1 cleared (it held P2_(s-2), read during step s - 1)
-      double* z = qbuf((step + 1) % 3);
-      double dsum = 0;
-      for (long e = gt; e < nn; e += gs) {
-        const double v = tc2_next(ca, cb, Pin[e], P2in[e]);
-        Pout[e] = v;
-        z[e] = 0.0;
-        if (e / n == e % n) dsum += v;
-      }
-      block_sum_add(dsum, trp);
-    }
-    // P2_s = P_s P_s
-    double dtr = 0.0;
-    for (int u = gwarp; u < units; u += nwarps) {
-      int t = u / nkc;
-      const int kc = u - t * nkc;
-      int rt = 0;
+  double t1 = (s_t[0] + s_t[1]) + (s_t[2] + s_t[3]);
+  double *cur = a.P0, *sq_buf = a.P1, *ex_buf = a.P2;
+  for (int step = 0; step < a.max_steps; ++step) {
+    double* dg = a.dg + (size_t)(step & 1) * 4 * nt;
+    for (int t0 = blockIdx.x; t0 < ntiles; t0 += gridDim.x) {
+      int t = t0, rt = 0;
       while (t >= nt - rt) {
         t -= nt - rt;
         ++rt;
       }
-      const int ct = rt + t;
-      const int k0 = kc * TC2_K;
-      const int r = lane >> 2, q = lane & 3;
-      double af[TC2_K / 4][2], bf[TC2_K / 4][2];
+      const int ct = rt + t, row = rt * TC2_T + r, col = ct * TC2_T + r;
+      const bool rok = row < n, cok = col < n;
+      const double *pa = cur + (long)row * n, *pb = cur + (long)col * n;
+      double x[2] = {0, 0}, y[2] = {0, 0};
+      for (int k0 = 4 * warp; k0 < n; k0 += U * KS) {
+        double af[U], bf[U];
 #pragma unroll
-      for (int k4 = 0; k4 < TC2_K / 4; ++k4) {
-        const int k = k0 + 4 * k4 + q;
+        for (int u = 0; u < U; ++u) {
+          const int k = k0 + u * KS + q;
+          af[u] = rok && k < n ? __ldcg(pa + k) : 0.0;
+          bf[u] = cok && k < n ? __ldcg(pb + k) : 0.0;
+        }
 #pragma unroll
-        for (int i = 0; i < 2; ++i) {
-          const int row = rt * TC2_T + 8 * i + r, col = ct * TC2_T + 8 * i + r;
-          double va = 0.0, vb = 0.0;
-          if (row < n && k < n) va = tc2_next(ca, cb, Pin[(long)row * n + k], P2in[(long)row * n + k]);
-          if (col < n && k < n) vb = tc2_next(ca, cb, Pin[(long)col * n + k], P2in[(long)col * n + k]);
-          af[k4][i] = va;
-          bf[k4][i] = vb;
+        for (int u = 0; u < U; u += 2) {
+          if (k0 + u * KS < n) dmma(x[0], x[1], af[u], bf[u]);
+          if (k0 + (u + 1) * KS < n) dmma(y[0], y[1], af[u + 1], bf[u + 1]);
         }
       }
-      double acc[2][2][2] = {};
-#pragma unroll
-      for (int k4 = 0; k4 < TC2_K / 4; ++k4)
-#pragma unroll
-        for (int i = 0; i < 2; ++i)
-#pragma unroll
-          for (int j = 0; j < 2; ++j) dmma(acc[i][j][0], acc[i][j][1], af[k4][i], bf[k4][j]);
-#pragma unroll
-      for (int i = 0; i < 2; ++i)
-#pragma unroll
-        for (int j = 0; j < 2; ++j)
-#pragma unroll
-          for (int h = 0; h < 2; ++h) {
-            const int row = rt * TC2_T + 8 * i + r, col = ct * TC2_T + 8 * j + 2 * q + h;
-            if (row < n && col < n) {
-              const double v = acc[i][j][h];
-              atomicAdd(P2out + (long)row * n + col, v);
-              if (rt < ct) atomicAdd(P2out + (long)col * n + row, v);
-              if (row == col) dtr += v;
-            }
+      part[warp][r * TC2_T + 2 * q] = x[0] + y[0];
+      part[warp][r * TC2_T + 2 * q + 1] = x[1] + y[1];
+      __syncthreads();
+      if (tid < TC2_T * TC2_T) {   // two whole warps
+        const int i = rt * TC2_T + tid / TC2_T, j = ct * TC2_T + tid % TC2_T;
+        double v = 0, e = 0;
+        if (i < n && j < n) {
+          v = (part[0][tid] + part[1][tid]) + (part[2][tid] + part[3][tid]);
+          e = __fma_rn(2.0, __ldcg(cur + (long)i * n + j), -v);
+          sq_buf[(long)i * n + j] = v;
+          ex_buf[(long)i * n + j] = e;
+          if (rt < ct) {
+            sq_buf[(long)j * n + i] = v;
+            ex_buf[(long)j * n + i] = e;
           }
+        }
+        if (rt == ct) {
+          v = i == j ? v : 0.0;
+          e = i == j ? e : 0.0;
+#pragma unroll
+          for (int o = 16; o > 0; o >>= 1) {
+            v += __shfl_xor_sync(0xffffffffu, v, o);
+            e += __shfl_xor_sync(0xffffffffu, e, o);
+          }
+          if (lane == 0) {
+            dg[2 * rt + warp] = v;
+            dg[2 * nt + 2 * rt + warp] = e;
+          }
+        }
+      }
+      __syncthreads();
     }
-    block_sum_add(dtr, trp + 1);
     if (!grid_barrier(a.bar, epoch, a.status)) return;
-    // the same decision in every block
-    const double t1 = *((volatile double*)trp), t2 = *((volatile double*)(trp + 1));
-    const double den = t1 - t2;
-    if (gt == 0) {
+    if (warp < 2) {
+      double v = 0;
+      for (int i = lane; i < 2 * nt; i += 32) v += __ldcg(dg + 2 * nt * warp + i);
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+      if (lane == 0) s_t[warp] = v;
+    }
+    __syncthreads();
+    const double t2 = s_t[0], te = s_t[1], den = t1 - t2;
+    if (blockIdx.x == 0 && tid == 0) {
       a.out[0] = den;
       a.out[1] = step + 1;
     }
-    final_buf = step == 0 ? 0 : (step & 1);
-    if (fabs(den) < a.tol * max(1, a.ne)) break;
+    if (fabs(den) < a.tol * max(1, a.ne)) break;   // the same decision in every block
     const bool sq = fabs(t2 - a.ne) < fabs(2 * t1 - t2 - a.ne);
-    ca = sq ? 0.0 : 2.0;
-    cb = sq ? 1.0 : -1.0;
+    double* next = sq ? sq_buf : ex_buf;
+    (sq ? sq_buf : ex_buf) = cur;
+    cur = next;
+    t1 = sq ? t2 : te;
   }
-  // the converged P_s back into P0
-  if (final_buf != 0)
-    for (long e = gt; e < nn; e += gs) a.P0[e] = a.P1[e];
+  // the converged P back into P0 (not read by anyone when it is not cur)
+  if (cur != a.P0) {
+    const long nn = (long)n * n, gs = (long)gridDim.x * TC2_THREADS;
+    for (long e = blockIdx.x * (long)TC2_THREADS + tid; e < nn; e += gs) a.P0[e] = __ldcg(cur + e);
+  }
 }
 
-// TC2 start: the spectrum of F mapped onto [0, 1], reversed (P0 = (hi I - F) / (hi - lo)).
+// TC2 start: the spectrum of F mapped onto [0, 1], reversed (P0 = (hi I - F) / (hi - lo)),
+// and the barrier counter and status word at zero.
 __global__ void k_tc2_init(int n, const double* __restrict__ F, const double* __restrict__ g, double* __restrict__ P,
-                           double* __restrict__ Q0, double* __restrict__ Q1, double* __restrict__ Q2,
-                           double* __restrict__ tr, unsigned* __restrict__ bar, int* __restrict__ status) {
-  // P0 = (hi I - F) / (hi - lo), and the zeros the fused kernel starts from
-  // (its three P^2 buffers, trace slots, barrier counter and status word)
+                           unsigned* __restrict__ bar, int* __restrict__ status) {
   const int i = blockIdx.y, j = blockIdx.x * blockDim.x + threadIdx.x;
   if (i == 0 && blockIdx.x == 0) {
-    if (threadIdx.x < 16) tr[threadIdx.x] = 0.0;
     if (threadIdx.x < 2) bar[threadIdx.x] = 0u;
     if (threadIdx.x == 0) *status = 0;
   }
@@ -1307,9 +1254,6 @@ __global__ void k_tc2_init(int n, const double* __restrict__ F, const double* __
   const double sc = hi > lo ? 1.0 / (hi - lo) : 0.0;
   const long e = (long)i * n + j;
   P[e] = sc * ((i == j ? hi : 0.0) - F[e]);
-  Q0[e] = 0.0;
-  Q1[e] = 0.0;
-  Q2[e] = 0.0;
 }
 
 // The spectral projector onto the ne lowest eigenvectors of the symmetric F.
@@ -1341,10 +1285,7 @@ gbhf_status purify(gbhf_ctx* c, int n, int ne, const double* d_F, double* d_P, d
   k_gershgorin<<<1, 1024, 0, c->stream>>>(n, d_F, g);
   count_launch(c);
   if (tc2) {
-    GBHF_CUDA(c, c->jac.t2.alloc(nn));
-    GBHF_CUDA(c, c->jac.t3.alloc(nn));
-    k_tc2_init<<<dim3((n + 127) / 128, n), 128, 0, c->stream>>>(n, d_F, g, d_P, P2, P3, c->jac.t2.p, tr,
-                                                                c->jac.bar.p, c->dev_status.p);
+    k_tc2_init<<<dim3((n + 127) / 128, n), 128, 0, c->stream>>>(n, d_F, g, d_P, c->jac.bar.p, c->dev_status.p);
     count_launch(c);
   } else {
     k_purify_init<<<dim3((n + 127) / 128, n), 128, 0, c->stream>>>(n, ne, d_F, g, d_P);
@@ -1363,29 +1304,32 @@ gbhf_status purify(gbhf_ctx* c, int n, int ne, const double* d_F, double* d_P, d
   const int ks = (n + kslice - 1) / kslice;
   double hout[2] = {1.0, 0.0};
   if (tc2) {
-    // one barrier per step: a second P buffer and three P2 buffers (zeroed by k_tc2_init)
+    const int nt8 = (n + TC2_T - 1) / TC2_T;
+    GBHF_CUDA(c, c->jac.t2.alloc(8 * (size_t)nt8));
     Tc2Args t;
     t.n = n;
     t.ne = ne;
     t.max_steps = 200;
     t.tol = 1e-13;   // E[D] is first order in the idempotency error
     t.P0 = d_P;
-    t.P1 = c->jac.t3.p;
-    t.Q0 = P2;
-    t.Q1 = P3;
-    t.Q2 = c->jac.t2.p;
-    t.tr = tr;
+    t.P1 = P2;
+    t.P2 = P3;
+    t.dg = c->jac.t2.p;
     t.out = out;
     t.bar = c->jac.bar.p;
     t.status = c->dev_status.p;
-    if (c->tc2_grid == 0) {
+    if (c->tc2_per_sm == 0) {
       int per_sm = 0;
       GBHF_CUDA(c, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_tc2_fused, TC2_THREADS, 0));
-      c->tc2_grid = std::max(1, c->nsm * std::min(std::max(per_sm, 1), 2));
+      c->tc2_per_sm = std::min(std::max(per_sm, 1), 4);
     }
-    const int nt16 = (n + TC2_T - 1) / TC2_T;
-    const long units = (long)nt16 * (nt16 + 1) / 2 * ((n + TC2_K - 1) / TC2_K);
-    const int grid = (int)std::max(1L, std::min<long>(c->tc2_grid, (units + 7) / 8));
+    // blocks per SM: the most, up to four, that leave no SM with more tiles than an
+    // even share (the tiles of a step are bound by the FP64 pipe of their SM)
+    const int tiles = nt8 * (nt8 + 1) / 2, share = (tiles + c->nsm - 1) / c->nsm;
+    int bps = 1;
+    for (int b = 2; b <= c->tc2_per_sm; ++b)
+      if (b * ((share + b - 1) / b) <= bps * ((share + bps - 1) / bps)) bps = b;
+    const int grid = std::min(c->nsm * bps, tiles);
     void* args[] = {&t};
     GBHF_CUDA(c, cudaLaunchCooperativeKernel((void*)k_tc2_fused, dim3(grid), dim3(TC2_THREADS), args, 0, c->stream));
     count_launch(c);
@@ -1461,15 +1405,23 @@ gbhf_status purify_finish(gbhf_ctx* c, const double* rec) {
 gbhf_status density_purified_dev(gbhf_ctx* c, int n, const double* d_Fsq, const double* d_X, int nocc,
                                  double* d_Dsq) {
   const size_t nn = (size_t)n * n;
+  if (nocc <= 0) {
+    GBHF_CUDA(c, cudaMemsetAsync(d_Dsq, 0, nn * sizeof(double), c->stream));
+    return GBHF_OK;
+  }
+  if (small_dense_takes(c, n)) {
+    GBHF_CUDA(c, c->small.alloc(64));
+    double* d_rec = c->small.p + PURIFY_REC;
+    GBHF_TRY(density_small(c, n, nocc, d_Fsq, d_X, d_Dsq, d_rec));
+    c->purify_ne = nocc;
+    c->purify_pending = true;
+    return c->purify_defer ? GBHF_OK : purify_flush(c);
+  }
   GBHF_WS(c, T1, 10, nn);
   GBHF_WS(c, Fp, 11, nn);
   GBHF_WS(c, P, 12, nn);
   GBHF_TRY(gemm(c, true, false, n, n, n, 1.0, d_X, n, d_Fsq, n, 0.0, T1, n));
   GBHF_TRY(gemm(c, false, false, n, n, n, 1.0, T1, n, d_X, n, 0.0, Fp, n, true));
-  if (nocc <= 0) {
-    GBHF_CUDA(c, cudaMemsetAsync(d_Dsq, 0, nn * sizeof(double), c->stream));
-    return GBHF_OK;
-  }
   GBHF_TRY(purify(c, n, nocc, Fp, P, nullptr));
   GBHF_TRY(gemm(c, false, false, n, n, n, 2.0, d_X, n, P, n, 0.0, T1, n));
   GBHF_TRY(gemm(c, false, true, n, n, n, 1.0, T1, n, d_X, n, 0.0, d_Dsq, n, true));
@@ -1521,6 +1473,15 @@ gbhf_status inv_sqrt_dev(gbhf_ctx* c, int n, const double* d_S, double* d_X, int
   GBHF_CUDA(c, c->small.alloc(64));
   double* g = c->small.p + 32;
   double* e = c->small.p + 44;
+  if (small_dense_takes(c, n)) {
+    double res[2];
+    GBHF_TRY(inv_sqrt_small(c, n, d_S, d_X, e));
+    GBHF_CUDA(c, cudaMemcpyAsync(res, e, sizeof res, cudaMemcpyDeviceToHost, c->stream));
+    GBHF_CUDA(c, cudaStreamSynchronize(c->stream));
+    if (iters) *iters = (int)res[1];
+    if (!(res[0] < 1e-10)) return fail(c, GBHF_ERR_NOT_CONVERGED, "Newton-Schulz S^-1/2 did not converge");
+    return GBHF_OK;
+  }
   k_gershgorin<<<1, 1024, 0, c->stream>>>(n, d_S, g);
   k_ns_init<<<dim3((n + 127) / 128, n), 128, 0, c->stream>>>(n, d_S, g, Y, Z);
   count_launch(c, 2);
@@ -1595,6 +1556,7 @@ gbhf_status diagonal_hf_dev(gbhf_ctx* c, int n, const double* d_Fsq, const doubl
 // S D F = (F D S)^T for symmetric F, D, S.
 gbhf_status diis_error_dev(gbhf_ctx* c, int n, const double* d_F, const double* d_S, const double* d_D,
                            const double* d_X, double* d_e) {
+  if (n <= SMALL_DIIS_MAX_N && small_dense_takes(c, n)) return diis_error_small(c, n, d_F, d_S, d_D, d_X, d_e);
   const size_t nn = (size_t)n * n;
   GBHF_WS(c, T1, 13, nn);
   GBHF_WS(c, T2, 14, nn);

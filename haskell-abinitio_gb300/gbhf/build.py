@@ -19,7 +19,7 @@ LIB = BUILD / "libgbhf.so"
 ARCH = ["-gencode", "arch=compute_103a,code=sm_103a"]
 SOURCES = ["jk.cu", "grad_ff.cu", "jk_ff.cu", "grad.cu", "jkd.cu", "gradd.cu", "api.cu", "setup.cu", "eri_canon.cu", "linalg.cu", "scf.cu", "measure.cu", "noalloc.cu", "batch.cu",
            "sad.cu", "bscf.cu", "uhf.cu",
-           "tune.cu", "tridiag.cu"]
+           "tune.cu", "tridiag.cu", "small_dense.cu"]
 HEADERS = ["gbhf_common.cuh", "gbhf_ff.cuh", "gbhf_internal.h", "gbhf_md.cuh", "eri_gen.cuh", "grad_gen.cuh", "jacobi.cuh",
            "dense.cuh", "mdwarp.cuh", "jk_kern.cuh",
            "grad_kern.cuh", "screen.cuh"]
