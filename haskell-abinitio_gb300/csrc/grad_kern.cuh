@@ -31,20 +31,20 @@ struct GamReg {
   __device__ __forceinline__ T get(int i) const { return v[i]; }
   __device__ __forceinline__ void set(int i, T x) { v[i] = x; }
 };
-template <typename T, int N>
-struct GamSmem {   // per-thread column of a [N][GR_THREADS] shared array
+template <typename T, int N, int TH>
+struct GamSmem {   // per-thread column of a [N][TH] shared array
   T* p;
   // volatile: a read stays where the code places it (the bra loop reads T_ab
   // block by block; hoisted out of the loop, all of T would be live at once)
   __device__ __forceinline__ T get(int i) const {
     if constexpr (std::is_same<T, ff>::value) {
-      const unsigned long long b = *(volatile const unsigned long long*)(p + i * GR_THREADS);
+      const unsigned long long b = *(volatile const unsigned long long*)(p + i * TH);
       return ff(__uint_as_float((unsigned)b), __uint_as_float((unsigned)(b >> 32)));
     } else {
-      return *(volatile const T*)(p + i * GR_THREADS);
+      return *(volatile const T*)(p + i * TH);
     }
   }
-  __device__ __forceinline__ void set(int i, T x) { p[i * GR_THREADS] = x; }
+  __device__ __forceinline__ void set(int i, T x) { p[i * TH] = x; }
 };
 
 template <int LA, int LB, int LC, int LD>
@@ -113,8 +113,9 @@ __device__ __forceinline__ double warp_sum_d(double v) {
 
 // One batch: the quartets of bra pair ib with the kets jk of the active lanes,
 // kets on the low lg bits of the lane; lanes beyond them split the primitive
-// quartets (as in k_jk) and the closing warp sum adds the slices.
-template <int LA, int LB, int LC, int LD, typename T, typename GamT, typename TkT>
+// quartets (as in k_jk) and the closing warp sum adds the slices.  STEP: every
+// primitive quartet is one tick of the block (k_grad_jk_step), in warp-uniform loops.
+template <int LA, int LB, int LC, int LD, typename T, typename GamT, typename TkT, bool STEP = false>
 __device__ __forceinline__ void grad_batch(const GradArgs<T>& a, GamT& gam, TkT& tk, const T* sbra, const T* sDab, int ib,
                                            int4 pab, int jk, int4 pcd, bool active, int lg, int lane, int Kb, int4 sg,
                                            int n, const T* __restrict__ Dm, float thrs, int dex) {
@@ -138,6 +139,8 @@ __device__ __forceinline__ void grad_batch(const GradArgs<T>& a, GamT& gam, TkT&
   const int sb = slice & (nsb - 1), sk = slice >> lb;
   T g[6] = {0, 0, 0, 0, 0, 0};
   S wgt = 0;
+  bool keep = false;
+  ff AC[3];
   if (active) {
     S gmax = S(0);
     // Gamma_abcd = jcoef D_ab D_cd - (D_ac D_bd + D_ad D_bc) / 4
@@ -167,12 +170,8 @@ __device__ __forceinline__ void grad_batch(const GradArgs<T>& a, GamT& gam, TkT&
           }
     // exact screening of this quartet by its own Gamma (the task lists bound it
     // by the pairs' density weights)
-    bool keep;
     if constexpr (sizeof(T) == 4 || FF) keep = a.scr.Qf[ib] * a.scr.Qf[jk] * gmax >= thrs;
     else keep = a.Q[ib] * a.Q[jk] * gmax >= a.thr;
-    const long long base = (long long)sg.w + (jk - sg.x);
-    const int nbl = sb < Kb && keep ? (Kb - sb + nsb - 1) / nsb : 0;
-    ff AC[3];
     if constexpr (FF) {
       const float4 a0v = a.cen[3 * A], a1v = a.cen[3 * A + 1], a2v = a.cen[3 * A + 2];
       const float4 c0v = a.cen[3 * C], c1v = a.cen[3 * C + 1], c2v = a.cen[3 * C + 2];
@@ -180,36 +179,54 @@ __device__ __forceinline__ void grad_batch(const GradArgs<T>& a, GamT& gam, TkT&
       AC[1] = diff3(a0v.y, a1v.y, a2v.y, c0v.y, c1v.y, c2v.y);
       AC[2] = diff3(a0v.z, a1v.z, a2v.z, c0v.z, c1v.z, c2v.z);
     }
+    wgt = (A == B ? S(1) : S(2)) * (C == Dd ? S(1) : S(2));
+  }
+  const long long base = (long long)sg.w + (jk - sg.x);
+  const int nbl = sb < Kb && keep ? (Kb - sb + nsb - 1) / nsb : 0;
+  T q = 0, Qx = 0, Qy = 0, Qz = 0, Kcd = 0;
+  auto ket_prim = [&](int kc) {
+    const long long idx = base + (long long)kc * len;
+    q = a.ket[BRA_P * npp + idx];
+    const T invq = a.ket[BRA_INVP * npp + idx];
+    T QCx = 0, QCy = 0, QCz = 0, QDx = 0, QDy = 0, QDz = 0;
+    if (LC >= 1 || FF) {
+      QCx = a.ket[BRA_PAX * npp + idx];
+      QCy = a.ket[BRA_PAY * npp + idx];
+      QCz = a.ket[BRA_PAZ * npp + idx];
+    }
+    if (LD >= 1) {
+      QDx = a.ket[BRA_PBX * npp + idx];
+      QDy = a.ket[BRA_PBY * npp + idx];
+      QDz = a.ket[BRA_PBZ * npp + idx];
+    }
+    if constexpr (FF) {   // the bra's P is P - A: Q - A here
+      Qx = nrm(QCx - AC[0]);
+      Qy = nrm(QCy - AC[1]);
+      Qz = nrm(QCz - AC[2]);
+    } else {
+      Qx = a.ket[BRA_PX * npp + idx];
+      Qy = a.ket[BRA_PY * npp + idx];
+      Qz = a.ket[BRA_PZ * npp + idx];
+    }
+    Kcd = a.ket[BRA_K * npp + idx];
+    GradFn<LA, LB, LC, LD>::ket(invq, QCx, QCy, QCz, QDx, QDy, QDz, gam, tk);
+  };
+  if constexpr (STEP) {
+    const int nbu = __any_sync(0xffffffffu, keep) ? (Kb + nsb - 1) / nsb : 0;   // the longest lane's
+    for (int k0 = 0; nbu > 0 && k0 < K; k0 += nsk) {
+      const bool mine = keep && k0 + sk < K;
+      if (mine) ket_prim(k0 + sk);
+      for (int kb = 0; kb < nbu; ++kb) {
+        __syncthreads_or(1);   // a tick
+        if (mine && kb < nbl)
+          GradFn<LA, LB, LC, LD>::run(sbra + (sb + kb * nsb) * BRA_SB, 1, BRA_SB, q, Qx, Qy, Qz, Kcd, a.boys, tk, g);
+      }
+    }
+  } else {
     for (int kc = sk; keep && kc < K; kc += nsk) {
-      const long long idx = base + (long long)kc * len;
-      const T q = a.ket[BRA_P * npp + idx];
-      const T invq = a.ket[BRA_INVP * npp + idx];
-      T Qx, Qy, Qz;
-      T QCx = 0, QCy = 0, QCz = 0, QDx = 0, QDy = 0, QDz = 0;
-      if (LC >= 1 || FF) {
-        QCx = a.ket[BRA_PAX * npp + idx];
-        QCy = a.ket[BRA_PAY * npp + idx];
-        QCz = a.ket[BRA_PAZ * npp + idx];
-      }
-      if (LD >= 1) {
-        QDx = a.ket[BRA_PBX * npp + idx];
-        QDy = a.ket[BRA_PBY * npp + idx];
-        QDz = a.ket[BRA_PBZ * npp + idx];
-      }
-      if constexpr (FF) {   // the bra's P is P - A: Q - A here
-        Qx = nrm(QCx - AC[0]);
-        Qy = nrm(QCy - AC[1]);
-        Qz = nrm(QCz - AC[2]);
-      } else {
-        Qx = a.ket[BRA_PX * npp + idx];
-        Qy = a.ket[BRA_PY * npp + idx];
-        Qz = a.ket[BRA_PZ * npp + idx];
-      }
-      const T Kcd = a.ket[BRA_K * npp + idx];
-      GradFn<LA, LB, LC, LD>::ket(invq, QCx, QCy, QCz, QDx, QDy, QDz, gam, tk);
+      ket_prim(kc);
       GradFn<LA, LB, LC, LD>::run(sbra + sb * BRA_SB, nbl, nsb * BRA_SB, q, Qx, Qy, Qz, Kcd, a.boys, tk, g);
     }
-    wgt = (A == B ? S(1) : S(2)) * (C == Dd ? S(1) : S(2));
   }
 #pragma unroll
   for (int x = 0; x < 6; ++x) {
@@ -229,8 +246,8 @@ __global__ void __launch_bounds__(GR_THREADS) k_grad_jk(GradArgs<T> a) {
   __shared__ int sq[QUEUE ? GR_WARPS : 1][64];
   extern __shared__ double gsm_dyn[];
   constexpr int NT = NAB * nherm_c(LC + LD);
-  using GamT = typename std::conditional<SG, GamSmem<T, NOUT>, GamReg<T, NOUT>>::type;
-  using TkT = typename std::conditional<SG, GamSmem<T, NT>, GamReg<T, NT>>::type;
+  using GamT = typename std::conditional<SG, GamSmem<T, NOUT, GR_THREADS>, GamReg<T, NOUT>>::type;
+  using TkT = typename std::conditional<SG, GamSmem<T, NT, GR_THREADS>, GamReg<T, NT>>::type;
   GamT gam;
   TkT tk;
   if constexpr (SG) {
@@ -301,6 +318,108 @@ __global__ void __launch_bounds__(GR_THREADS) k_grad_jk(GradArgs<T> a) {
   }
 }
 
+// The queue form with the block's warps in step.  The two-float code of a (pp|ps)
+// primitive quartet is some 7,000 instructions in one run; warps that go through it
+// at places of their own fetch it eight times over, and waiting for instructions
+// took 80% of their time (0.43 instructions per cycle and SM, 2.9 in (ss|ps)).  Here a
+// primitive quartet is one tick: the warps of the block, each with its own batch,
+// meet at a barrier before every one and go through the code together.  (H2O)8 FP64
+// gradient, (pp|ps) 2.19 -> 1.12 ms, (ps|pp) 0.90 -> 0.42, (pp|ss) 1.64 -> 1.07, (pp|pp)
+// 1.26 -> 1.01, the gradient 10.0 -> 7.7; a barrier per batch instead of per tick left
+// (pp|ps) at 1.47, its batches being uneven.  Still bound by instruction fetch and by
+// waiting at the ticks.  256 threads where registers and shared memory allow, so that
+// one block fills the SM.
+template <int LA, int LB, int LC, int LD, typename T, bool SG, int TH>
+__global__ void __launch_bounds__(TH) k_grad_jk_step(GradArgs<T> a) {
+  constexpr int NA = ncart_c(LA), NB = ncart_c(LB), NC = ncart_c(LC), ND = ncart_c(LD);
+  constexpr int NAB = NA * NB, NOUT = NAB * NC * ND, W = TH / 32;
+  __shared__ __align__(16) T sbra[W][KMAX_PRIM_PAIRS * BRA_SB];
+  __shared__ T sDab[W][NAB];
+  __shared__ int sq[W][64];
+  extern __shared__ double gsm_dyn[];
+  constexpr int NT = NAB * nherm_c(LC + LD);
+  using GamT = typename std::conditional<SG, GamSmem<T, NOUT, TH>, GamReg<T, NOUT>>::type;
+  using TkT = typename std::conditional<SG, GamSmem<T, NT, TH>, GamReg<T, NT>>::type;
+  GamT gam;
+  TkT tk;
+  if constexpr (SG) {
+    gam.p = reinterpret_cast<T*>(gsm_dyn) + threadIdx.x;
+    tk.p = reinterpret_cast<T*>(gsm_dyn) + NOUT * TH + threadIdx.x;
+  }
+  constexpr bool FF = std::is_same<T, ff>::value;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  int dex = 0;          // as in k_grad_jk
+  float thrs = (float)a.thr;
+  if constexpr (FF) {
+    dex = 2 * *a.dexp;
+    thrs = (float)scalbn(a.thr, -dex);
+  }
+  const int start = a.range[0];
+  const int ntask = a.range[1] - start;
+  int4 task = make_int4(0, 0, 0, 0);
+  int queued = 0, scanned = 0;
+  bool more = true;   // tasks left
+  while (true) {
+    // the warp's next batch: survivors of its task, or of the next ones
+    while (true) {
+      if (scanned < task.z) {
+        const int ib = task.x;
+        const BraScreen bs(a.scr, ib, a.scr.pinfo[ib], a.pmol[ib]);
+        while (queued < 32 && scanned < task.z) {
+          const int o = scanned + lane;
+          const int jk = task.y + o;
+          const bool pass = o < task.z && bs.gamma_pass(a.scr, jk, a.jabs);
+          queue_push(sq[warp], queued, jk, pass, lane);
+          scanned += 32;
+        }
+      }
+      if (queued > 0 || !more) break;
+      int t = 0;
+      if (lane == 0) t = atomicAdd(a.counter, 1);
+      t = __shfl_sync(0xffffffffu, t, 0);
+      more = t < ntask;
+      if (!more) {
+        task.z = 0;
+        break;
+      }
+      task = a.tasks[start + t];
+      scanned = 0;
+      const int ib = task.x, mol = a.pmol[ib], n = a.mn[mol];
+      const T* __restrict__ Dm = a.D + a.moff[mol];
+      const int kb0 = task.w & 0xffff, Kb = (task.w >> 16) - kb0, pb0 = a.poff[ib] + kb0;
+      const unsigned rkb = (65536u + Kb - 1) / Kb;
+      for (int idx = lane; idx < BRA_NFIELD * Kb; idx += 32) {
+        const int f = (int)(((unsigned)idx * rkb) >> 16), k = idx - f * Kb;
+        sbra[warp][k * BRA_SB + f] = a.bra[(long long)f * a.npp + pb0 + k];
+      }
+      const int4 pab = a.scr.pinfo[ib];
+      for (int i = lane; i < NAB; i += 32) sDab[warp][i] = Dm[(long long)(pab.z + i / NB) * n + pab.w + i % NB];
+      __syncwarp();
+    }
+    if (queued == 0) break;   // out of work
+    {
+      const int ib = task.x, mol = a.pmol[ib];
+      const int nk = min(queued, 32);
+      const int lg = 32 - __clz(nk - 1);
+      const bool active = (lane & ((1 << lg) - 1)) < nk;
+      const int jk = active ? sq[warp][lane & ((1 << lg) - 1)] : task.y;
+      grad_batch<LA, LB, LC, LD, T, GamT, TkT, true>(a, gam, tk, sbra[warp], sDab[warp], ib, a.scr.pinfo[ib], jk,
+                                                     a.scr.pinfo[jk], active, lg, lane,
+                                                     (task.w >> 16) - (task.w & 0xffff), a.seg[a.kseg[task.y]],
+                                                     a.mn[mol], a.D + a.moff[mol], thrs, dex);
+      queue_pop(sq[warp], queued, nk, lane);
+    }
+  }
+  while (__syncthreads_or(0)) {   // keeps ticking until the block's other warps are done as well
+  }
+}
+
+// Code that fits runs better alone: (ps|ps) 0.81 ms, 0.83 in step; (ss|pp) 0.18 and 0.21.
+template <int LA, int LB, int LC, int LD, typename T>
+constexpr bool grad_in_step() {
+  return std::is_same<T, ff>::value && LA < 2 && LB < 2 && LC < 2 && LD < 2 && LA == 1 && (LB == 1 || LD == 1);
+}
+
 template <int LA, int LB, int LC, int LD, typename T>
 static gbhf_status launch_grad_class(gbhf_ctx* c, cudaStream_t strm, int combo, int prec, const T* D, double* grad,
                                      int ntask) {
@@ -308,17 +427,21 @@ static gbhf_status launch_grad_class(gbhf_ctx* c, cudaStream_t strm, int combo, 
   constexpr int NOUT = ncart_c(LA) * ncart_c(LB) * ncart_c(LC) * ncart_c(LD);
   constexpr int NT = ncart_c(LA) * ncart_c(LB) * nherm_c(LC + LD);
   constexpr bool SG = sizeof(T) == 8 ? NOUT > 9 : NOUT > 27;   // Gamma and T in shared memory
-  const size_t smem = SG ? (size_t)(NOUT + NT) * GR_THREADS * sizeof(T) : 0;
-  auto kern = k_grad_jk<LA, LB, LC, LD, T, SG, (LA < 2 && LB < 2 && LC < 2 && LD < 2)>;
+  constexpr bool STEP = grad_in_step<LA, LB, LC, LD, T>();
+  constexpr int TH = STEP && (NOUT + NT) * 256 * sizeof(T) <= 160 * 1024 ? 256 : GR_THREADS;
+  const size_t smem = SG ? (size_t)(NOUT + NT) * TH * sizeof(T) : 0;
+  void (*kern)(GradArgs<T>);
+  if constexpr (STEP) kern = k_grad_jk_step<LA, LB, LC, LD, T, SG, TH>;
+  else kern = k_grad_jk<LA, LB, LC, LD, T, SG, (LA < 2 && LB < 2 && LC < 2 && LD < 2)>;
   static bool attr_set = false;
   if (SG && !attr_set) {
     GBHF_CUDA(c, cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     attr_set = true;
   }
   int per_sm = 0;
-  GBHF_CUDA(c, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, GR_THREADS, smem));
+  GBHF_CUDA(c, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, TH, smem));
   per_sm = std::max(per_sm, 1);
-  const int grid = std::min(c->nsm * per_sm, (ntask + GR_WARPS - 1) / GR_WARPS);
+  const int grid = std::min(c->nsm * per_sm, (ntask + TH / 32 - 1) / (TH / 32));
   PairData& P = c->pairs;
   TaskLists& gt = c->gtasks;
   GradArgs<T> a;
@@ -346,7 +469,7 @@ static gbhf_status launch_grad_class(gbhf_ctx* c, cudaStream_t strm, int combo, 
   a.scr = quartet_screen(c, gt.thr_exact);
   a.jabs = (float)std::fabs(c->grad_jcoef);
   a.jcoef = T(c->grad_jcoef);
-  kern<<<grid, GR_THREADS, smem, strm>>>(a);
+  kern<<<grid, TH, smem, strm>>>(a);
   count_launch(c);
   GBHF_CUDA(c, cudaGetLastError());
   return GBHF_OK;

@@ -120,6 +120,7 @@ struct TaskGenArgs {
   int* count;                    // NTIER per item
   const int* off;                // exclusive scans, NTIER x (nitems + 1)
   int4* tasks[NTIER];            // FP64, FP32, two-float
+  int fine_div[2][NTIER], fine_kets[2][NTIER];   // finer tasks by (d classes, tier): divisor of lane_prims, most kets
 };
 
 __device__ __forceinline__ int count_ge(const double* Q, int lo, int hi, double thr) {
@@ -177,22 +178,25 @@ __global__ void k_tasks(TaskGenArgs g) {
       const int kd = ffq > 0 ? count_ge(g.Q, lo, lo + k64, fmax(ffq / qi, g.ffw / (qi * w))) : k64;
       // split the bra primitives so that one lane handles at most about
       // lane_prims primitive quartets per task (bounds the launch tail)
-      const int lp = g.lane_prims[k], tk = g.task_kets[k];
-      const int nch0 = min(kb, (kb * s.z + lp - 1) / lp);
-      const int cs = (kb + nch0 - 1) / nch0;
-      const int nch = (kb + cs - 1) / cs;
       const int first[NTIER] = {lo, lo + k64, lo + kd}, len[NTIER] = {kd, keep - k64, k64 - kd};
-      if (FILL) {
-        for (int ch = 0; ch < nch; ++ch) {
-          const int w = (ch * cs) | (min(kb, (ch + 1) * cs) << 16);
 #pragma unroll
-          for (int t = 0; t < NTIER; ++t)
+      for (int t = 0; t < NTIER; ++t) {
+        if (len[t] <= 0) continue;
+        const int d = X > 2 || Y > 2;
+        const int lp = max(1, g.lane_prims[k] / g.fine_div[d][t]);
+        const int tk = min(g.task_kets[k], g.fine_kets[d][t]);
+        const int nch0 = min(kb, (kb * s.z + lp - 1) / lp);
+        const int cs = (kb + nch0 - 1) / nch0;
+        const int nch = (kb + cs - 1) / cs;
+        if (FILL) {
+          for (int ch = 0; ch < nch; ++ch) {
+            const int w = (ch * cs) | (min(kb, (ch + 1) * cs) << 16);
             for (int o = 0; o < len[t]; o += tk)
               g.tasks[t][wt[t]++] = make_int4(i, first[t] + o, min(tk, len[t] - o), w);
+          }
+        } else {
+          nt[t] += nch * ((len[t] + tk - 1) / tk);
         }
-      } else {
-#pragma unroll
-        for (int t = 0; t < NTIER; ++t) nt[t] += nch * ((len[t] + tk - 1) / tk);
       }
     }
   }
@@ -522,6 +526,24 @@ static gbhf_status build_task_lists(gbhf_ctx* c, TaskLists& TL, int ncombo, cons
     // FP32 launches gain 13-14% (fewer ket-field loads per primitive
     // quartet); (pp|pp) FP64 lost 18% that way (its launch is tail-bound)
     g.ket_ge[k] = k < ncombo && cbra[k] == cket[k] && cbra[k] <= 1 ? 1 : 0;
+  }
+  // Finer tasks where a list is too short to keep the SMs busy to its end.
+  // - d classes (a warp per quartet), below 4096 shell pairs: twelfths.  6-31G*
+  //   gradient of 1, 2, 3 (mixed), 5 waters 11.4, 15.3, 10.4, 23.7 -> 6.9, 9.3, 6.9,
+  //   18.6 ms, Fock build 1.46, 1.96, 1.40, 3.46 -> 0.90, 1.42, 1.09, 3.32.  With
+  //   5050 pairs (10 waters) the gradient lost 2%.
+  // - FP64 gradient tasks of s/p classes, quarters: the two-float list leaves few of
+  //   them, and one ran for a third of the launch.  (H2O)8 7.88 -> 7.47 ms.
+  // - two-float gradient tasks, at most 64 kets ((H2O)8 7.47 -> 7.10 ms, (H2O)12 mixed
+  //   7.35 -> 6.66), below 4096 pairs halves ((H2O)4 2.75 -> 2.56).
+  // The s/p Fock builds gain nothing of the kind ((H2O)16 FP64 6.7 -> 7.4 ms with
+  // halved two-float tasks).
+  const bool few = P.npairs < 4096;
+  for (int t = 0; t < NTIER; ++t) {
+    g.fine_div[0][t] = !all_pairs ? 1 : (t == TIER_64 ? 4 : (t == TIER_FF && few ? 2 : 1));
+    g.fine_kets[0][t] = all_pairs && t == TIER_FF ? 64 : 1 << 20;
+    g.fine_div[1][t] = few ? 12 : 1;
+    g.fine_kets[1][t] = 1 << 20;
   }
   g.all_pairs = all_pairs ? 1 : 0;
   g.square_w = square_w ? 1 : 0;
