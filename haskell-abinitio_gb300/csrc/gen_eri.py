@@ -159,8 +159,8 @@ def gen_class(la, lb, lc, ld):
     out = []
     w = out.append
     w(f"// ---- class ({cls[0]}{cls[1]}|{cls[2]}{cls[3]}): {nab}x{ncd} integrals, L = {L}")
-    w("template <typename T, typename Acc>")
-    w(f"__device__ __forceinline__ void eri_ketprim_{cls}(const T* __restrict__ sb, int nbra, int bstep,")
+    w("template <typename T, typename Acc, typename NB>")
+    w(f"__device__ __forceinline__ void eri_ketprim_{cls}(const T* __restrict__ sb, const NB nbra, int bstep,")
     w("    const T q, const T invq, const T Qx, const T Qy, const T Qz,")
     w("    const T QCx, const T QCy, const T QCz, const T QDx, const T QDy, const T QDz,")
     w("    const T Kcd, const T* __restrict__ boys, Acc& acc) {")
@@ -201,7 +201,8 @@ def gen_class(la, lb, lc, ld):
     # (ss|ss) and (ps|ss): two bra primitives in flight (two independent load
     # and Boys chains; the larger classes keep their registers for one)
     w("  #pragma unroll 2" if L <= 1 else "  #pragma unroll 1")
-    w("  for (int kb = 0; kb < nbra; ++kb) {")
+    w("  for (int kb = 0; kb < nb_end(nbra); ++kb) {")
+    w("    if (nb_skip(nbra, kb)) continue;")
     w("    BraPrim<T> bp;")
     w("    load_bra_prim(sb + kb * bstep, bp);")
     w("    const T p = bp.p, invp = bp.invp, Px = bp.Px, Py = bp.Py, Pz = bp.Pz;")
@@ -329,8 +330,8 @@ def gen_class_deferred(la, lb, lc, ld):
     out = []
     w = out.append
     w(f"// ---- class ({cls[0]}{cls[1]}|{cls[2]}{cls[3]}): {nab}x{ncd} integrals, L = {L}, ket transformation deferred")
-    w("template <typename T, typename Acc>")
-    w(f"__device__ __forceinline__ void eri_ketprim_{cls}(const T* __restrict__ sb, int nbra, int bstep,")
+    w("template <typename T, typename Acc, typename NB>")
+    w(f"__device__ __forceinline__ void eri_ketprim_{cls}(const T* __restrict__ sb, const NB nbra, int bstep,")
     w("    const T q, const T invq, const T Qx, const T Qy, const T Qz,")
     w("    const T QCx, const T QCy, const T QCz, const T QDx, const T QDy, const T QDz,")
     w("    const T Kcd, const T* __restrict__ boys, Acc& acc) {")
@@ -379,7 +380,8 @@ def gen_class_deferred(la, lb, lc, ld):
         for h in ket_union:
             w(f"  T V{iab}_{h[0]}{h[1]}{h[2]} = T(0);")
     w("  #pragma unroll 1")
-    w("  for (int kb = 0; kb < nbra; ++kb) {")
+    w("  for (int kb = 0; kb < nb_end(nbra); ++kb) {")
+    w("    if (nb_skip(nbra, kb)) continue;")
     w("    BraPrim<T> bp;")
     w("    load_bra_prim(sb + kb * bstep, bp);")
     w("    const T p = bp.p, invp = bp.invp, Px = bp.Px, Py = bp.Py, Pz = bp.Pz;")
@@ -468,7 +470,11 @@ def render():
     # warp-per-quartet kernels of jkd.cu)
     classes += [(2, 0, 0, 0), (2, 0, 1, 0), (2, 0, 1, 1), (2, 0, 2, 0), (2, 1, 0, 0), (2, 1, 1, 0), (2, 2, 0, 0)]
     parts = ["// GENERATED by gen_eri.py -- do not edit by hand.",
-             "#pragma once", ""]
+             "#pragma once", "",
+             "// The bra loop's trip count: a lane's own, or (k_jk_step) a warp-uniform one with a",
+             "// block barrier before each primitive quartet (nb_end, nb_skip of StepCount).",
+             "__device__ __forceinline__ int nb_end(int n) { return n; }",
+             "__device__ __forceinline__ bool nb_skip(int, int) { return false; }", ""]
     for c in classes:
         code, *_ = gen_class(*c)
         parts.append(code)

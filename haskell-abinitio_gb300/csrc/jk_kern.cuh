@@ -22,16 +22,26 @@ struct RegAcc {
   __device__ __forceinline__ T get(int i) const { return v[i]; }
 };
 
-template <typename T, int N>
+template <typename T, int N, int TH>
 struct SmemAcc {
-  T* p;   // this thread's column, stride blockDim (128)
-  __device__ __forceinline__ T& operator[](int i) { return p[i * 128]; }
+  T* p;   // this thread's column, stride blockDim (TH)
+  __device__ __forceinline__ T& operator[](int i) { return p[i * TH]; }
   __device__ __forceinline__ void zero() {
 #pragma unroll 4
-    for (int i = 0; i < N; ++i) p[i * 128] = T(0);
+    for (int i = 0; i < N; ++i) p[i * TH] = T(0);
   }
-  __device__ __forceinline__ T get(int i) const { return p[i * 128]; }
+  __device__ __forceinline__ T get(int i) const { return p[i * TH]; }
 };
+
+// Bra primitives of a lane and of the warp's longest lane (k_jk_step).
+struct StepCount {
+  int own, all;
+};
+__device__ __forceinline__ int nb_end(StepCount n) { return n.all; }
+__device__ __forceinline__ bool nb_skip(StepCount n, int kb) {
+  __syncthreads_or(1);   // a tick
+  return kb >= n.own;
+}
 
 }  // namespace gbhf
 
@@ -70,11 +80,11 @@ struct ClassFn;
 #define GBHF_CLASS_FN(la, lb, lc, ld, name)                                                              \
   template <>                                                                                            \
   struct ClassFn<la, lb, lc, ld> {                                                                       \
-    template <typename T, typename Acc>                                                                  \
-    static __device__ __forceinline__ void run(const T* sb, int nbra, int bstep, T q, T invq, T Qx, T Qy, T Qz,  \
+    template <typename T, typename Acc, typename NB>                                                     \
+    static __device__ __forceinline__ void run(const T* sb, NB nbra, int bstep, T q, T invq, T Qx, T Qy, T Qz,  \
                                                T QCx, T QCy, T QCz, T QDx, T QDy, T QDz, T Kcd,           \
                                                const T* boys, Acc& acc) {                                 \
-      eri_ketprim_##name<T, Acc>(sb, nbra, bstep, q, invq, Qx, Qy, Qz, QCx, QCy, QCz, QDx, QDy, QDz, Kcd, boys, \
+      eri_ketprim_##name<T, Acc, NB>(sb, nbra, bstep, q, invq, Qx, Qy, Qz, QCx, QCy, QCz, QDx, QDy, QDz, Kcd, boys, \
                                  acc);                                                                   \
     }                                                                                                    \
   };
@@ -112,8 +122,9 @@ constexpr int JK_THREADS = 128;
 constexpr int JK_WARPS = JK_THREADS / 32;
 
 // One batch: the quartets of bra pair ib with the kets jk of the lanes that
-// `keep` one, kets on the low lg bits of the lane.
-template <int LA, int LB, int LC, int LD, typename T, typename AccT>
+// `keep` one, kets on the low lg bits of the lane.  STEP: every primitive quartet is
+// one tick of the block (k_jk_step), in warp-uniform loops.
+template <int LA, int LB, int LC, int LD, typename T, typename AccT, bool STEP = false>
 __device__ __forceinline__ void jk_batch(const JKArgs<T>& a, AccT& acc, const T* sbra, const T* sDab, int ib, int4 pab,
                                          int jk, int4 pcd, bool keep, int lg, int lane, int kb0, int Kb, int4 sg, int n,
                                          const T* __restrict__ Dm, double* __restrict__ Gm, int dex,
@@ -151,7 +162,7 @@ __device__ __forceinline__ void jk_batch(const JKArgs<T>& a, AccT& acc, const T*
   const int A = pab.x, B = pab.y, a0 = pab.z, b0 = pab.w;
   const int C = pcd.x, Dd = pcd.y, c0 = pcd.z, d0 = pcd.w;
   acc.zero();
-  if (keep) {
+  if (!STEP && keep) {
     const long long base = (long long)sg.w + (jk - sg.x);
     const int nbl = sb < Kb ? (Kb - sb + nsb - 1) / nsb : 0;   // this lane's bra primitives
     ff AC[3];
@@ -193,6 +204,48 @@ __device__ __forceinline__ void jk_batch(const JKArgs<T>& a, AccT& acc, const T*
     }
     cnt_q += lead_k && kb0 == 0;
     cnt_p += (unsigned long long)nbl * (sk < K ? (K - sk + nsk - 1) / nsk : 0);
+  }
+  if constexpr (STEP) {   // the same, warp-uniform: lanes without a primitive quartet come along for the ticks
+    static_assert(FF, "two-float kernels");
+    const long long base = (long long)sg.w + (jk - sg.x);
+    const int nbl = keep && sb < Kb ? (Kb - sb + nsb - 1) / nsb : 0;   // this lane's bra primitives
+    ff AC[3];
+    if (keep) {
+      const float4 a0v = a.cen[3 * A], a1v = a.cen[3 * A + 1], a2v = a.cen[3 * A + 2];
+      const float4 c0v = a.cen[3 * C], c1v = a.cen[3 * C + 1], c2v = a.cen[3 * C + 2];
+      AC[0] = diff3(a0v.x, a1v.x, a2v.x, c0v.x, c1v.x, c2v.x);
+      AC[1] = diff3(a0v.y, a1v.y, a2v.y, c0v.y, c1v.y, c2v.y);
+      AC[2] = diff3(a0v.z, a1v.z, a2v.z, c0v.z, c1v.z, c2v.z);
+    }
+    const int all = __any_sync(0xffffffffu, keep) ? (Kb + nsb - 1) / nsb : 0;
+    for (int k0 = 0; all > 0 && k0 < K; k0 += nsk) {
+      const bool mine = keep && k0 + sk < K;
+      T q = 0, invq = 0, Qx = 0, Qy = 0, Qz = 0, Kcd = 0;
+      T QCx = 0, QCy = 0, QCz = 0, QDx = 0, QDy = 0, QDz = 0;
+      if (mine) {
+        const long long idx = base + (long long)(k0 + sk) * len;
+        q = a.ket[BRA_P * npp + idx];
+        invq = a.ket[BRA_INVP * npp + idx];
+        QCx = a.ket[BRA_PAX * npp + idx];
+        QCy = a.ket[BRA_PAY * npp + idx];
+        QCz = a.ket[BRA_PAZ * npp + idx];
+        if (LD >= 1) {
+          QDx = a.ket[BRA_PBX * npp + idx];
+          QDy = a.ket[BRA_PBY * npp + idx];
+          QDz = a.ket[BRA_PBZ * npp + idx];
+        }
+        Qx = nrm(QCx - AC[0]);
+        Qy = nrm(QCy - AC[1]);
+        Qz = nrm(QCz - AC[2]);
+        Kcd = a.ket[BRA_K * npp + idx];
+      }
+      ClassFn<LA, LB, LC, LD>::template run<T, AccT>(sbra + sb * BRA_SB, StepCount{mine ? nbl : 0, all}, nsb * BRA_SB, q,
+                                                     invq, Qx, Qy, Qz, QCx, QCy, QCz, QDx, QDy, QDz, Kcd, a.boys, acc);
+    }
+    if (keep) {
+      cnt_q += lead_k && kb0 == 0;
+      cnt_p += (unsigned long long)nbl * (sk < K ? (K - sk + nsk - 1) / nsk : 0);
+    }
   }
   // warp-uniform: sum the slices (every lane ends with the total of its ket)
   for (int o = 1 << lg; o < 32; o <<= 1) {
@@ -309,7 +362,7 @@ __global__ void __launch_bounds__(JK_THREADS) k_jk(JKArgs<T> a) {
   const int start = a.range[0];
   const int ntask = a.range[1] - start;
   unsigned long long cnt_q = 0, cnt_p = 0;
-  using AccT = typename std::conditional<SACC, SmemAcc<T, NOUT>, RegAcc<T, NOUT>>::type;
+  using AccT = typename std::conditional<SACC, SmemAcc<T, NOUT, JK_THREADS>, RegAcc<T, NOUT>>::type;
   AccT acc;
   if constexpr (SACC) acc.p = reinterpret_cast<T*>(sacc_dyn) + threadIdx.x;
   const long long npp = a.npp;
@@ -378,28 +431,121 @@ __global__ void __launch_bounds__(JK_THREADS) k_jk(JKArgs<T> a) {
   }
 }
 
+// The queue form with the block's warps in step, as k_grad_jk_step and for the same
+// reason (the two-float code of these two classes was waiting for instructions most of
+// the time): (H2O)16 FP64, (ps|pp) 1.76 -> 1.30 ms, (pp|pp) 1.10 -> 0.90, the build 6.7
+// -> 5.9; (H2O)64 mixed build 55.7 -> 51.8.  Eight warps a block: with four the builds
+// took 6.4 and 53.9 ms.  The other classes' code fits the caches.
+template <int LA, int LB, int LC, int LD, typename T, bool SACC, int TH>
+__global__ void __launch_bounds__(TH) k_jk_step(JKArgs<T> a) {
+  constexpr int NA = ncart_c(LA), NB = ncart_c(LB), NC = ncart_c(LC), ND = ncart_c(LD);
+  constexpr int NAB = NA * NB, NOUT = NAB * NC * ND, W = TH / 32;
+  __shared__ __align__(16) T sbra[W][KMAX_PRIM_PAIRS * BRA_SB];
+  __shared__ T sDab[W][NAB > 1 ? NAB : 1];
+  __shared__ int sq[W][64];
+  constexpr bool FF = std::is_same<T, ff>::value;
+  extern __shared__ double sacc_dyn[];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int dex = FF ? *a.dexp : 0;
+  const int start = a.range[0];
+  const int ntask = a.range[1] - start;
+  unsigned long long cnt_q = 0, cnt_p = 0;
+  using AccT = typename std::conditional<SACC, SmemAcc<T, NOUT, TH>, RegAcc<T, NOUT>>::type;
+  AccT acc;
+  if constexpr (SACC) acc.p = reinterpret_cast<T*>(sacc_dyn) + threadIdx.x;
+  int4 task = make_int4(0, 0, 0, 0);
+  int queued = 0, scanned = 0;
+  bool more = true;   // tasks left
+  while (true) {
+    // the warp's next batch: survivors of its task, or of the next ones
+    while (true) {
+      if (scanned < task.z) {
+        const int ib = task.x;
+        const BraScreen bs(a.scr, ib, a.scr.pinfo[ib], a.pmol[ib]);
+        while (queued < 32 && scanned < task.z) {
+          const int o = scanned + lane;
+          const int jk = task.y + o;
+          const bool pass = o < task.z && bs.jk_pass(a.scr, jk);
+          queue_push(sq[warp], queued, jk, pass, lane);
+          scanned += 32;
+        }
+      }
+      if (queued > 0 || !more) break;
+      int t = 0;
+      if (lane == 0) t = atomicAdd(a.counter, 1);
+      t = __shfl_sync(0xffffffffu, t, 0);
+      more = t < ntask;
+      if (!more) {
+        task.z = 0;
+        break;
+      }
+      task = a.tasks[start + t];
+      scanned = 0;
+      const int ib = task.x, mol = a.pmol[ib], n = a.mn[mol];
+      const T* __restrict__ Dm = a.D + a.moff[mol];
+      const int kb0 = task.w & 0xffff, Kb = (task.w >> 16) - kb0, pb0 = a.poff[ib] + kb0;
+      const unsigned rkb = (65536u + Kb - 1) / Kb;
+      for (int idx = lane; idx < BRA_NJK * Kb; idx += 32) {
+        const int f = (int)(((unsigned)idx * rkb) >> 16), k = idx - f * Kb;
+        sbra[warp][k * BRA_SB + f] = a.bra[(long long)f * a.npp + pb0 + k];
+      }
+      const int4 pab = a.scr.pinfo[ib];
+      for (int i = lane; i < NAB; i += 32) sDab[warp][i] = Dm[(long long)(pab.z + i / NB) * n + pab.w + i % NB];
+      __syncwarp();
+    }
+    if (queued == 0) break;   // out of work
+    const int ib = task.x, mol = a.pmol[ib], kb0 = task.w & 0xffff;
+    const int nk = min(queued, 32);
+    const int lg = 32 - __clz(nk - 1);
+    const bool keep = (lane & ((1 << lg) - 1)) < nk;
+    const int jk = keep ? sq[warp][lane & ((1 << lg) - 1)] : task.y;
+    jk_batch<LA, LB, LC, LD, T, AccT, true>(a, acc, sbra[warp], sDab[warp], ib, a.scr.pinfo[ib], jk, a.scr.pinfo[jk],
+                                            keep, lg, lane, kb0, (task.w >> 16) - kb0, a.seg[a.kseg[task.y]], a.mn[mol],
+                                            a.D + a.moff[mol], a.G + a.moff[mol], dex, cnt_q, cnt_p);
+    queue_pop(sq[warp], queued, nk, lane);
+  }
+  while (__syncthreads_or(0)) {   // keeps ticking until the block's other warps are done as well
+  }
+  cnt_q = (unsigned long long)warp_sum((double)cnt_q);
+  cnt_p = (unsigned long long)warp_sum((double)cnt_p);
+  if (lane == 0 && a.stats) {
+    atomicAdd(&a.stats[0], cnt_q);
+    atomicAdd(&a.stats[1], cnt_q * (unsigned long long)(NOUT));
+    atomicAdd(&a.stats[2], cnt_p);
+  }
+}
+
+template <int LA, int LB, int LC, int LD, typename T>
+constexpr bool jk_in_step() {
+  return std::is_same<T, ff>::value && LA == 1 && LC == 1 && LD == 1 && LB < 2;
+}
+
 template <int LA, int LB, int LC, int LD, typename T, bool SACC>
 static gbhf_status launch_class(gbhf_ctx* c, cudaStream_t strm, int combo, int prec, const T* D, double* G, int ntask,
                                 int with_j) {
   if (ntask <= 0) return GBHF_OK;
   constexpr int NOUT = ncart_c(LA) * ncart_c(LB) * ncart_c(LC) * ncart_c(LD);
-  const size_t smem = SACC ? (size_t)NOUT * JK_THREADS * sizeof(T) : 0;
+  constexpr bool STEP = jk_in_step<LA, LB, LC, LD, T>();
+  constexpr int TH = STEP ? 256 : JK_THREADS;
+  const size_t smem = SACC ? (size_t)NOUT * TH * sizeof(T) : 0;
   // The queue packs the survivors of a task's kets into full batches (s/p classes;
   // a d task is one batch of at most 32 kets): (ps|ss) FP32 of (H2O)64 17.5 ->
   // 11.9 ms, (ss|ss) 10.7 -> 7.1, the whole mixed build 84.6 -> 61 ms.  The (dd|ss)
   // instance of the queue form read out of bounds on the device although the same
   // source is clean on a host emulation under address and thread sanitizers: the d
   // classes keep the plain form.
-  auto kern = k_jk<LA, LB, LC, LD, T, SACC, (LA < 2 && LB < 2 && LC < 2 && LD < 2)>;
+  void (*kern)(JKArgs<T>);
+  if constexpr (STEP) kern = k_jk_step<LA, LB, LC, LD, T, SACC, TH>;
+  else kern = k_jk<LA, LB, LC, LD, T, SACC, (LA < 2 && LB < 2 && LC < 2 && LD < 2)>;
   static bool attr_set = false;
   if (SACC && !attr_set) {
     GBHF_CUDA(c, cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     attr_set = true;
   }
   int per_sm = 0;
-  GBHF_CUDA(c, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, JK_THREADS, smem));
+  GBHF_CUDA(c, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, TH, smem));
   per_sm = std::max(per_sm, 1);
-  int grid = std::min(c->nsm * per_sm, (ntask + JK_WARPS - 1) / JK_WARPS);
+  int grid = std::min(c->nsm * per_sm, (ntask + TH / 32 - 1) / (TH / 32));
   PairData& P = c->pairs;
   JKArgs<T> a;
   a.tasks = c->tasks.tasks[prec].p;
@@ -423,7 +569,7 @@ static gbhf_status launch_class(gbhf_ctx* c, cudaStream_t strm, int combo, int p
   a.scr = quartet_screen(c, c->tasks.thr_exact);
   a.cen = c->tasks.cen.p;
   a.dexp = c->dff_exp.p;
-  kern<<<grid, JK_THREADS, smem, strm>>>(a);
+  kern<<<grid, TH, smem, strm>>>(a);
   count_launch(c);
   GBHF_CUDA(c, cudaGetLastError());
   return GBHF_OK;
