@@ -182,27 +182,6 @@ __global__ void k_b_ns_finish(BDesc d, const double* __restrict__ g, const doubl
   X[o + idx] = Z[o + idx] / sqrt(g[4 * m + 1]);
 }
 
-// Canonical purification start (Palser & Manolopoulos 1998):
-// P = lambda/n (mu I - F) + ne/n I, mu = tr F / n.
-__global__ void k_b_purify_init(BDesc d, const int* __restrict__ ne, const double* __restrict__ F,
-                                const double* __restrict__ g, double* __restrict__ P) {
-  BD_ELEMENT;
-  const double lo = g[4 * m], hi = g[4 * m + 1], mu = g[4 * m + 2] / n;
-  const int e = ne[m];
-  double lam = 1e300;
-  if (hi - mu > 0) lam = fmin(lam, e / (hi - mu));
-  if (mu - lo > 0) lam = fmin(lam, (n - e) / (mu - lo));
-  if (!(lam < 1e300)) lam = 0;
-  P[o + idx] = (lam / n) * ((i == j ? mu : 0.0) - F[o + idx]) + (i == j ? (double)e / n : 0.0);
-}
-
-__global__ void k_b_purify_update(BDesc d, const double* __restrict__ coef, double* __restrict__ P,
-                                  const double* __restrict__ P2, const double* __restrict__ P3) {
-  BD_ELEMENT;
-  const double* c = coef + 4 * m;
-  P[o + idx] = c[0] * P[o + idx] + c[1] * P2[o + idx] + c[2] * P3[o + idx];
-}
-
 // Per-molecule reductions: one block per molecule.
 // Gershgorin bounds and trace of A_m: g[4m] = lo, g[4m+1] = hi, g[4m+2] = trace.
 __global__ void k_b_gershgorin(BDesc d, const double* __restrict__ A, double* __restrict__ g) {
@@ -261,50 +240,6 @@ __global__ void k_b_maxdev_identity(BDesc d, const double* __restrict__ T, doubl
   if (threadIdx.x == 0) out[m] = v;
 }
 
-// traces of P, P^2, P^3 -> next purification polynomial, coef[4m] = (a, b, c, tr(P - P^2));
-// a molecule whose idempotency error is below tol * nocc leaves the purification
-// (its flag in d.active, a copy of the batch's flags, is cleared)
-__global__ void k_b_purify_coef(BDesc d, const double* __restrict__ P, const double* __restrict__ P2,
-                                const double* __restrict__ P3, double* __restrict__ coef,
-                                const int* __restrict__ nocc, double tol, int* __restrict__ pact) {
-  const int m = blockIdx.x;
-  if (!d.active[m]) return;
-  const int n = d.n[m];
-  const long long o = d.off[m];
-  double t1 = 0, t2 = 0, t3 = 0;
-  for (int i = threadIdx.x; i < n; i += blockDim.x) {
-    t1 += P[o + (long)i * n + i];
-    t2 += P2[o + (long)i * n + i];
-    t3 += P3[o + (long)i * n + i];
-  }
-  t1 = block_reduce(t1, false);
-  __syncthreads();
-  t2 = block_reduce(t2, false);
-  __syncthreads();
-  t3 = block_reduce(t3, false);
-  if (threadIdx.x == 0) {
-    const double den = t1 - t2, num = t2 - t3;
-    double a = 1, b = 0, c = 0;
-    if (fabs(den) > 1e-300) {
-      const double cc = num / den;
-      if (cc >= 0.5) {
-        a = 0;
-        b = (1 + cc) / cc;
-        c = -1 / cc;
-      } else {
-        a = (1 - 2 * cc) / (1 - cc);
-        b = (1 + cc) / (1 - cc);
-        c = -1 / (1 - cc);
-      }
-    }
-    coef[4 * m] = a;
-    coef[4 * m + 1] = b;
-    coef[4 * m + 2] = c;
-    coef[4 * m + 3] = den;
-    if (fabs(den) < tol * (double)max(1, nocc[m])) pact[m] = 0;   // P meets the tolerance: no further update
-  }
-}
-
 // TC2 purification (one GEMM per step): start P = (hi I - F) / (hi - lo), then
 // P <- P^2 or 2P - P^2, whichever moves tr P toward nocc.
 __global__ void k_b_tc2_init(BDesc d, const double* __restrict__ F, const double* __restrict__ g,
@@ -315,32 +250,146 @@ __global__ void k_b_tc2_init(BDesc d, const double* __restrict__ F, const double
   P[o + idx] = sc * ((i == j ? hi : 0.0) - F[o + idx]);
 }
 
-// traces of P and P^2 -> coef[4m] = (a, b, 0, tr(P - P^2)) of P' = a P + b P^2;
-// converged molecules leave as in k_b_purify_coef
-__global__ void k_b_tc2_coef(BDesc d, const double* __restrict__ P, const double* __restrict__ P2,
-                             double* __restrict__ coef, const int* __restrict__ nocc, double tol,
-                             int* __restrict__ pact) {
-  const int m = blockIdx.x;
-  if (!d.active[m]) return;
-  const int n = d.n[m];
-  const long long o = d.off[m];
-  double t1 = 0, t2 = 0;
-  for (int i = threadIdx.x; i < n; i += blockDim.x) {
-    t1 += P[o + (long)i * n + i];
-    t2 += P2[o + (long)i * n + i];
+// One purification step of every molecule as one launch, on the plan of k_tc2_fused:
+// a block owns an 8 x 8 tile of P^2 on or above the diagonal (four warps over the
+// k steps) and writes both candidates for the next P, P^2 and 2 P - P^2, with its part
+// of their traces; the next step's blocks add their molecule's partial traces, all in
+// the same order, and so take the same decision without a launch between.  A
+// molecule's state alternates between two slots (a step reads one, its first tile's
+// block writes the other), its three buffers rotate.  Blocks take the largest molecules
+// first.  Bound by the FP64 pipe.  48 conformers of 1 to 12 waters: 50 us a step, where a 16 x 16 tile
+// product, a trace launch and an update launch took 75 + 6 + 6 us and their gaps (the
+// batch with gradients 207 -> 194 ms).
+struct BTc2State {
+  double t1;              // tr P of the molecule's current P
+  double den;             // last tr(P - P^2)
+  int cur, sq, ex;        // buffers: P, and those that hold P^2 and 2 P - P^2
+  int open;               // 1: a step's traces await the decision; 0: first step
+  int done, pad;
+};
+struct BTc2Args {
+  BDesc d;
+  const int* ord;         // molecules, largest first
+  const int* t8;          // first tile of each in that order (M + 1)
+  const int* dg0;         // offset of each molecule's partial traces in dg, 8 nt values
+  const int* nocc;
+  double* buf[3];
+  double* dg;             // [step parity][candidate][2 nt]
+  BTc2State* st;          // [step parity][molecule]
+  double tol;
+};
+
+__global__ void k_b_tc2_start(BTc2Args a) {   // tr P_0
+  const int m = blockIdx.x, n = a.d.n[m];
+  const double* P = a.buf[0] + a.d.off[m];
+  double t = 0;
+  for (int i = threadIdx.x; i < n; i += blockDim.x) t += a.d.active[m] ? P[(long)i * n + i] : 0.0;
+  t = block_reduce(t, false);
+  if (threadIdx.x == 0) a.st[a.d.M + m] = BTc2State{t, 1.0, 0, 1, 2, 0, a.d.active[m] ? 0 : 1, 0};
+}
+
+__global__ void __launch_bounds__(128) k_b_tc2_step(BTc2Args a, int par) {
+  constexpr int T8 = 8, W = 4, KS = 4 * W, U = 4;
+  __shared__ double part[W][T8 * T8];
+  __shared__ double s_t[2];
+  const int slot = bd_mol(a.t8, a.d.M, blockIdx.x), m = a.ord[slot];
+  BTc2State s = a.st[(par ^ 1) * a.d.M + m];
+  const bool first = (int)blockIdx.x == a.t8[slot] && threadIdx.x == 0;   // writes the state
+  const int n = a.d.n[m], tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int nt = (n + T8 - 1) / T8;
+  if (!s.done && s.open) {
+    const double* dg = a.dg + a.dg0[m] + (par ^ 1) * 4 * nt;
+    if (warp < 2) {
+      double v = 0;
+      for (int i = lane; i < 2 * nt; i += 32) v += dg[2 * nt * warp + i];
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+      if (lane == 0) s_t[warp] = v;
+    }
+    __syncthreads();
+    const double t2 = s_t[0], te = s_t[1], ne = (double)a.nocc[m];
+    s.den = s.t1 - t2;
+    if (fabs(s.den) < a.tol * (double)max(1, a.nocc[m])) {
+      s.done = 1;
+    } else if (fabs(t2 - ne) < fabs(2 * s.t1 - t2 - ne)) {
+      const int c = s.cur;
+      s.cur = s.sq;
+      s.sq = c;
+      s.t1 = t2;
+    } else {
+      const int c = s.cur;
+      s.cur = s.ex;
+      s.ex = c;
+      s.t1 = te;
+    }
   }
-  t1 = block_reduce(t1, false);
+  s.open = 1;
+  if (first) a.st[par * a.d.M + m] = s;
+  if (s.done) return;
+  int t = blockIdx.x - a.t8[slot], rt = 0;
+  while (t >= nt - rt) {
+    t -= nt - rt;
+    ++rt;
+  }
+  const int ct = rt + t, r = lane >> 2, q = lane & 3, row = rt * T8 + r, col = ct * T8 + r;
+  const bool rok = row < n, cok = col < n;
+  const long long o = a.d.off[m];
+  const double* cur = a.buf[s.cur] + o;
+  double *sqb = a.buf[s.sq] + o, *exb = a.buf[s.ex] + o;
+  const double *pa = cur + (long)row * n, *pb = cur + (long)col * n;
+  double x[2] = {0, 0}, y[2] = {0, 0};
+  for (int k0 = 4 * warp; k0 < n; k0 += U * KS) {
+    double af[U], bf[U];
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      const int k = k0 + u * KS + q;
+      af[u] = rok && k < n ? pa[k] : 0.0;
+      bf[u] = cok && k < n ? pb[k] : 0.0;
+    }
+#pragma unroll
+    for (int u = 0; u < U; u += 2) {
+      if (k0 + u * KS < n) dmma(x[0], x[1], af[u], bf[u]);
+      if (k0 + (u + 1) * KS < n) dmma(y[0], y[1], af[u + 1], bf[u + 1]);
+    }
+  }
+  part[warp][r * T8 + 2 * q] = x[0] + y[0];
+  part[warp][r * T8 + 2 * q + 1] = x[1] + y[1];
   __syncthreads();
-  t2 = block_reduce(t2, false);
-  if (threadIdx.x == 0) {
-    const double den = t1 - t2, ne = (double)nocc[m];
-    const bool sq = fabs(t2 - ne) < fabs(2 * t1 - t2 - ne);
-    coef[4 * m] = sq ? 0.0 : 2.0;
-    coef[4 * m + 1] = sq ? 1.0 : -1.0;
-    coef[4 * m + 2] = 0.0;
-    coef[4 * m + 3] = den;
-    if (fabs(den) < tol * (double)max(1, nocc[m])) pact[m] = 0;
+  if (tid >= T8 * T8) return;   // two whole warps stay
+  const int i = rt * T8 + tid / T8, j = ct * T8 + tid % T8;
+  double v = 0, e = 0;
+  if (i < n && j < n) {
+    v = (part[0][tid] + part[1][tid]) + (part[2][tid] + part[3][tid]);
+    e = __fma_rn(2.0, cur[(long)i * n + j], -v);
+    sqb[(long)i * n + j] = v;
+    exb[(long)i * n + j] = e;
+    if (rt < ct) {
+      sqb[(long)j * n + i] = v;
+      exb[(long)j * n + i] = e;
+    }
   }
+  if (rt == ct) {
+    v = i == j ? v : 0.0;
+    e = i == j ? e : 0.0;
+#pragma unroll
+    for (int o2 = 16; o2 > 0; o2 >>= 1) {
+      v += __shfl_xor_sync(0xffffffffu, v, o2);
+      e += __shfl_xor_sync(0xffffffffu, e, o2);
+    }
+    if (lane == 0) {
+      double* dg = a.dg + a.dg0[m] + par * 4 * nt;
+      dg[2 * rt + warp] = v;
+      dg[2 * nt + 2 * rt + warp] = e;
+    }
+  }
+}
+
+// The converged P of every molecule into the first buffer.
+__global__ void k_b_tc2_final(BDesc d, const BTc2State* __restrict__ st, double* __restrict__ P,
+                              const double* __restrict__ P1, const double* __restrict__ P2) {
+  BD_ELEMENT;
+  const int cur = st[d.M + m].cur;
+  if (cur) P[o + idx] = (cur == 1 ? P1 : P2)[o + idx];
 }
 
 struct HistPtrs {
@@ -438,7 +487,10 @@ struct BatchRun {
   size_t nst = 0;
   std::vector<int> n, tstart, nocc, active;
   std::vector<long long> off;
-  DBuf<int> d_n, d_tstart, d_active, d_nocc, d_pact;
+  DBuf<int> d_n, d_tstart, d_active, d_nocc, d_tc2;   // d_tc2: order, first tiles, trace offsets
+  DBuf<double> d_dg;
+  DBuf<BTc2State> d_st;
+  int ntiles8 = 0;
   DBuf<long long> d_off;
   BDesc desc{};
 
@@ -470,6 +522,25 @@ struct BatchRun {
     GBHF_CUDA(c, cudaMemcpyAsync(d_tstart.p, tstart.data(), (M + 1) * sizeof(int), cudaMemcpyHostToDevice,
                                  c->stream));
     GBHF_CUDA(c, cudaMemcpyAsync(d_nocc.p, nocc.data(), M * sizeof(int), cudaMemcpyHostToDevice, c->stream));
+    {   // purification tiles, largest molecules first
+      std::vector<int> v(3 * (size_t)M + 1);
+      int *ord = v.data(), *t8 = ord + M, *dg0 = t8 + M + 1, ndg = 0;
+      for (int m = 0; m < M; ++m) ord[m] = m;
+      std::stable_sort(ord, ord + M, [&](int x, int y) { return n[x] > n[y]; });
+      t8[0] = 0;
+      for (int k = 0; k < M; ++k) {
+        const int nt = (n[ord[k]] + 7) / 8;
+        t8[k + 1] = t8[k] + nt * (nt + 1) / 2;
+        dg0[ord[k]] = ndg;
+        ndg += 8 * nt;
+      }
+      ntiles8 = t8[M];
+      GBHF_CUDA(c, d_tc2.alloc(v.size()));
+      GBHF_CUDA(c, d_dg.alloc(ndg));
+      GBHF_CUDA(c, d_st.alloc(2 * (size_t)M));
+      GBHF_CUDA(c, cudaMemcpyAsync(d_tc2.p, v.data(), v.size() * sizeof(int), cudaMemcpyHostToDevice, c->stream));
+      GBHF_CUDA(c, cudaStreamSynchronize(c->stream));
+    }
     GBHF_TRY(set_active(active));
     desc.M = M;
     desc.n = d_n.p;
@@ -538,56 +609,52 @@ gbhf_status b_inv_sqrt(BatchRun& br, const double* S, double* X, double* Y, doub
 // D_m = X_m (2 P_m) X_m^T with P_m the projector onto the nocc_m lowest
 // eigenvectors of X_m^T F_m X_m (trace-correcting purification, as density_purified_dev).
 gbhf_status b_density(BatchRun& br, const double* F, const double* X, double* D, double* T1, double* Fp, double* P,
-                      double* P2, double* P3, double* g, double* coef) {
+                      double* P2, double* P3, double* g) {
   gbhf_ctx* c = br.c;
   GBHF_TRY(br.gemm(true, false, 1.0, X, F, 0.0, T1));
   GBHF_TRY(br.gemm(false, false, 1.0, T1, X, 0.0, Fp, true));
-  // trace-correcting purification: a third fewer GEMMs than the canonical one
-  // on water clusters (see purify in linalg.cu)
-  constexpr bool tc2 = true;
   k_b_gershgorin<<<br.M, 256, 0, c->stream>>>(br.desc, Fp, g);
-  if (tc2) k_b_tc2_init<<<br.egrid(), 256, 0, c->stream>>>(br.desc, Fp, g, P);
-  else k_b_purify_init<<<br.egrid(), 256, 0, c->stream>>>(br.desc, br.d_nocc.p, Fp, g, P);
-  count_launch(c, 2);
-  std::vector<double> hc(4 * (size_t)br.M);
-  // molecules still purifying: a copy of the active flags that k_b_purify_coef clears
-  GBHF_CUDA(c, br.d_pact.alloc(br.M));
-  GBHF_CUDA(c, cudaMemcpyAsync(br.d_pact.p, br.d_active.p, br.M * sizeof(int), cudaMemcpyDeviceToDevice, c->stream));
-  BDesc pd = br.desc;
-  pd.active = br.d_pact.p;
-  const double tol = 1e-13;
+  k_b_tc2_init<<<br.egrid(), 256, 0, c->stream>>>(br.desc, Fp, g, P);
+  BTc2Args a;
+  a.d = br.desc;
+  a.ord = br.d_tc2.p;
+  a.t8 = a.ord + br.M;
+  a.dg0 = a.t8 + br.M + 1;
+  a.nocc = br.d_nocc.p;
+  a.buf[0] = P;
+  a.buf[1] = P2;
+  a.buf[2] = P3;
+  a.dg = br.d_dg.p;
+  a.st = br.d_st.p;
+  a.tol = 1e-13;
+  k_b_tc2_start<<<br.M, 128, 0, c->stream>>>(a);
+  count_launch(c, 3);
+  GBHF_CUDA(c, cudaGetLastError());
+  std::vector<BTc2State> hs(br.M);
   // four purification steps per CUDA-graph replay, convergence read between replays
   auto four_steps = [&]() -> gbhf_status {
-    for (int k = 0; k < 4; ++k) {
-      GBHF_TRY(br.gemm(false, false, 1.0, P, P, 0.0, P2, true, &pd));
-      if (tc2) {
-        k_b_tc2_coef<<<br.M, 256, 0, c->stream>>>(pd, P, P2, coef, br.d_nocc.p, tol, br.d_pact.p);
-        k_b_purify_update<<<br.egrid(), 256, 0, c->stream>>>(pd, coef, P, P2, P2);   // third coefficient 0
-        count_launch(c, 2);
-        continue;
-      }
-      GBHF_TRY(br.gemm(false, false, 1.0, P, P2, 0.0, P3, true, &pd));
-      k_b_purify_coef<<<br.M, 256, 0, c->stream>>>(pd, P, P2, P3, coef, br.d_nocc.p, tol, br.d_pact.p);
-      k_b_purify_update<<<br.egrid(), 256, 0, c->stream>>>(pd, coef, P, P2, P3);
-      count_launch(c, 2);
-    }
+    for (int k = 0; k < 4; ++k) k_b_tc2_step<<<br.ntiles8, 128, 0, c->stream>>>(a, k & 1);
+    count_launch(c, 4);
     return GBHF_OK;
   };
-  const std::vector<const void*> key = {(const void*)(size_t)br.M, (const void*)(size_t)br.ntiles,
-                                        (const void*)(size_t)br.nmax, br.desc.n, br.desc.off, br.desc.tstart,
-                                        br.d_pact.p, br.d_nocc.p, P, P2, P3, coef};
+  const std::vector<const void*> key = {(const void*)(size_t)br.M, (const void*)(size_t)br.ntiles8, br.desc.n,
+                                        br.desc.off, br.desc.active, br.d_tc2.p, br.d_nocc.p, br.d_dg.p, br.d_st.p,
+                                        P, P2, P3};
   bool done = false;
   for (int rep = 0; rep < 50 && !done; ++rep) {
     GBHF_TRY(graph_run(c, c->g_bpurify, key, four_steps));
-    GBHF_CUDA(c, cudaMemcpyAsync(hc.data(), coef, hc.size() * sizeof(double), cudaMemcpyDeviceToHost, c->stream));
+    GBHF_CUDA(c, cudaMemcpyAsync(hs.data(), br.d_st.p + br.M, br.M * sizeof(BTc2State), cudaMemcpyDeviceToHost,
+                                 c->stream));
     GBHF_CUDA(c, cudaStreamSynchronize(c->stream));
     done = true;
     for (int m = 0; m < br.M; ++m)
-      if (br.active[m] && !(std::fabs(hc[4 * m + 3]) < tol * std::max(1, br.nocc[m]))) done = false;
+      if (br.active[m] && !hs[m].done) done = false;
   }
   for (int m = 0; m < br.M; ++m)
-    if (br.active[m] && !(std::fabs(hc[4 * m + 3]) < 1e-6 * std::max(1, br.nocc[m])))
+    if (br.active[m] && !(std::fabs(hs[m].den) < 1e-6 * std::max(1, br.nocc[m])))
       return fail(c, GBHF_ERR_NOT_CONVERGED, "density purification did not converge for molecule " + std::to_string(m));
+  k_b_tc2_final<<<br.egrid(), 256, 0, c->stream>>>(br.desc, br.d_st.p, P, P2, P3);
+  count_launch(c);
   GBHF_TRY(br.gemm(false, false, 2.0, X, P, 0.0, T1));
   GBHF_TRY(br.gemm(false, true, 1.0, T1, X, 0.0, D, true));
   return GBHF_OK;
@@ -656,7 +723,6 @@ gbhf_status bscf_run(gbhf_ctx* c, const gbhf_scf_opts* o, double* energies, int*
   DBuf<double> small;
   GBHF_CUDA(c, small.alloc(32 * (size_t)M + 64));
   double* d_g = small.p;                  // 4 per molecule
-  double* d_coef = small.p + 4 * M;       // 4 per molecule
   double* d_err = small.p + 8 * M;        // 1 per molecule
   double* d_emax = small.p + 9 * M;       // 1 per molecule
   double* d_stats = small.p + 10 * M;     // 2 per molecule
@@ -680,7 +746,7 @@ gbhf_status bscf_run(gbhf_ctx* c, const gbhf_scf_opts* o, double* energies, int*
   if (o->guess == GBHF_GUESS_SAD) {
     GBHF_TRY(sad_density(c, D));
   } else if (o->guess == GBHF_GUESS_CORE) {
-    GBHF_TRY(b_density(br, H, X, D, T1, Fp, P, P2, P3, d_g, d_coef));
+    GBHF_TRY(b_density(br, H, X, D, T1, Fp, P, P2, P3, d_g));
   } else {
     return fail(c, GBHF_ERR_UNSUPPORTED, "batched SCF starts from the SAD or core guess");
   }
@@ -871,7 +937,7 @@ gbhf_status bscf_run(gbhf_ctx* c, const gbhf_scf_opts* o, double* energies, int*
     c->prof.ph_diis += ms_since(t_phase);
     t_phase = clk::now();
     // ---- new densities
-    status = b_density(br, Fd, X, Dn, T1, Fp, P, P2, P3, d_g, d_coef);
+    status = b_density(br, Fd, X, Dn, T1, Fp, P, P2, P3, d_g);
     if (status != GBHF_OK) break;
     GBHF_CUDA(c, cudaStreamSynchronize(c->stream));
     c->prof.ph_diag += ms_since(t_phase);
@@ -937,7 +1003,7 @@ gbhf_status bscf_run(gbhf_ctx* c, const gbhf_scf_opts* o, double* energies, int*
     // D and W from the orbitals of the last F(D): D' = projector of F, W = D' F D' / 2
     std::vector<int> all(M, 1);
     GBHF_TRY(br.set_active(all));
-    GBHF_TRY(b_density(br, Ffin, X, Dg, T1, Fp, P, P2, P3, d_g, d_coef));
+    GBHF_TRY(b_density(br, Ffin, X, Dg, T1, Fp, P, P2, P3, d_g));
     GBHF_TRY(br.gemm(false, false, 1.0, Dg, Ffin, 0.0, T1));
     GBHF_TRY(br.gemm(false, false, 0.5, T1, Dg, 0.0, Wm, true));
     DBuf<double> dgrad;
