@@ -379,6 +379,8 @@ def run_gbhf(args, world, rank, local):
                                        "in a full mixed Fock build (profiles/traffic.json); the ERI kernels "
                                        "are compute-bound, traffic far below their roofline"},
         "classes": cls_tab,
+        "classes_note": "the fp64 entries hold the FP64 and the two-float launches of a class (FP64 work on the "
+                        "FP32 pipe); their frac is against the FP64 FMA peak and can exceed 1",
         "fma_peaks": peaks_clk,
         "clocks": clk.summary(),
         "e2e": {"value": e2e_v, "unit": "s/molecule", "h2d_bytes_per_step": int(h2d), "d2h_bytes_per_step": int(d2h),
