@@ -32,3 +32,33 @@ def test_gradient_against_fp64_lists(ctx, waters, basis):
     d, w = (np.insert(np.insert(x, at, 0, axis=0), at, 0, axis=1) for x in (d, w))
     ref = ctx.gradient(O.square_to_tri(d), O.square_to_tri(w), schwarz=0.0)
     np.testing.assert_allclose(got, ref, rtol=0, atol=1e-10)
+
+
+@pytest.mark.parametrize("waters,basis", [(1, "6-31g*"), (5, "sto-3g"), (6, "sto-3g"), (11, "sto-3g")])
+def test_one_electron_terms_against_differences(ctx, waters, basis):
+    """3, 15, 18 and 33 nuclei (on 4, 16 and 32 lanes, and in two rounds).  The
+    one-electron terms are odd in (D, W), the rest is even; tr D H - tr W S by fourth-order
+    central differences: rounding 1e3 * 2^-53 / 1e-3, truncation 1e-12 / 30 times a fifth
+    derivative of up to 1e5: 1e-7 absolute."""
+    xyz = M.water_cluster(waters, np.random.default_rng(waters))
+    labels = M.water_labels(waters)
+    fb = B.flatten(B.make_atoms(labels, xyz, basis))
+    rng = np.random.default_rng(7)
+    d, w = (O.square_to_tri(m + m.T) for m in rng.standard_normal((2, fb.n_cgf, fb.n_cgf)) * 0.1)
+    off = np.full(fb.n_cgf * (fb.n_cgf + 1) // 2, 2.0)
+    off[np.cumsum(np.concatenate([[0], np.arange(fb.n_cgf, 1, -1)]))] = 1.0    # diagonal of the flat triangle
+    ctx.set_basis(fb)
+    got = 0.5 * (ctx.gradient(d, w) - ctx.gradient(-d, -w))
+
+    def value(coords):
+        ctx.set_basis(B.flatten(B.make_atoms(labels, coords, basis)))
+        return off @ (d * ctx.hcore(_lib.MODE_EXACT) - w * ctx.overlap(_lib.MODE_EXACT))
+
+    step = 1e-3
+    for atom, x in ((0, 0), (1, 2), (3 * waters - 1, 1)):
+        f = []
+        for k in (-2, -1, 1, 2):
+            c = np.array(xyz, float)
+            c[atom, x] += k * step
+            f.append(value(c))
+        assert abs((f[0] - 8 * f[1] + 8 * f[2] - f[3]) / (12 * step) - got[atom, x]) < 1e-7
