@@ -391,7 +391,7 @@ struct gbhf_ctx {
   // concurrently so that the tail of one persistent launch overlaps the next
   // side streams for the J/K class launches (eight measured 1% faster than four on the
   // (H2O)16 mixed SCF); the gradient's class launches use the first NSIDE_GRAD (four: eight
-  // were 3% slower there)
+  // were 3% slower there), its one-electron terms the others
   static constexpr int NSIDE = 8;
   static constexpr int NSIDE_GRAD = 4;
   cudaStream_t side[NSIDE] = {};
