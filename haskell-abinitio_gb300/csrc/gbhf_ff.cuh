@@ -160,6 +160,26 @@ __device__ __forceinline__ void boys_eval_ff(ff tin, const ff* __restrict__ tab,
   }
 }
 
+// Range of a primitive pair in two floats, as exponents of two.  The class code
+// forms pref (-2 alpha)^n F_n times expansion coefficients, pref = K_ab K_cd /
+// sqrt(p + q), alpha = p q / (p + q) <= min(p, q), n <= L_ab + L_cd + 1 (one order
+// more in the gradient, whose coefficients also take a factor 2a <= 2p).  A
+// coefficient is a polynomial of degree <= L + 1 in P - A, P - B (r: the largest of
+// their components) and 1 / (2p); the powers of P - Q fall off with F_n.  Split over
+// the two pairs, `grow` bounds the factors on K but those of r (where r is large, K
+// is small) and `size` all of them times |K|.
+__host__ __device__ inline void ff_pair_range(double p, double K, double r, int L, float& size, float& grow) {
+  const float lp = log2f((float)p), lh = fmaxf(0.0f, -lp - 1.0f);
+  grow = ((float)L + 1.5f) * fmaxf(0.0f, lp + 1.0f) + fmaxf(0.0f, -0.25f * lp) + ((float)L + 1.0f) * lh;
+  size = grow + ((float)L + 1.0f) * fmaxf(0.0f, log2f((float)r) - lh) + log2f((float)(K < 0 ? -K : K));
+}
+// Largest values for which every quartet of such pairs may run in two floats.  FP32
+// ends at 2^128: 2^20 are left to the sums over components, density blocks and
+// primitives.  An operation loses at most 2^-149 to underflow; the factors that
+// follow make that 2^-45 of the molecule's largest quartet qmax^2 by this estimate,
+// 2^-58 without the second 2a that it counts for a steep shell.
+// (6-31G* stays within 43 and 50 up to neon.)
+constexpr float FF_MAX_SIZE = 54.0f, FF_MAX_GROW = 52.0f;   // the latter plus log2(qmax)
 
 // The type of an exactly representable constant in generated code, and of the
 // screening magnitudes: FP32 beside two-float values.

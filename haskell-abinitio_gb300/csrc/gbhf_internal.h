@@ -200,6 +200,13 @@ struct Basis {
   long long stacked = 0;             // sum of n_m^2
 };
 
+// Two-float quartets of a molecule: those with Q_ab Q_cd below q (0: none); off: a
+// primitive pair was outside the FP32 range (ff_pair_range), all stay in FP64.
+struct FFLimit {
+  double q;
+  int off, pad;
+};
+
 // Shell-pair data on the device, in the order used by the J/K kernels:
 // class 0 pairs, then class 1, then class 2; inside a class grouped by
 // primitive-pair count (segments), inside a segment by Schwarz bound descending.
@@ -226,7 +233,7 @@ struct PairData {
   DBuf<double> bra64, ket64;   // BRA_NFIELD arrays of length nprimpairs each
   DBuf<float> bra32, ket32;
   DBuf<ff> braff, ketff;       // two-float values; Px, Py, Pz unused (P - A stands for P)
-  DBuf<double> ffq;            // per molecule: two-float below this Q_ab Q_cd (0: never)
+  DBuf<FFLimit> ffq;           // per molecule: which quartets run in two floats
   bool use_ff = false;         // some molecule's limit is above 0
   size_t nprim_pairs = 0;
 };

@@ -113,8 +113,8 @@ struct TaskGenArgs {
   const double* Q;
   const int* pK;                 // primitive pairs per shell pair
   double thr_all, thr64;         // cutoff / weight, mixed cutoff / weight
-  const double* ffq;             // per molecule: two-float below this Q_ab Q_cd (0: never) ...
-  double ffw;                    // ... or below this weighted bound (mixed precision), see ff_limit
+  const FFLimit* ffq;            // per molecule: two-float below its Q_ab Q_cd ...
+  double ffw;                    // ... or below this weighted bound (mixed precision), see ff_weighted_limit
   const double* pw;              // per-pair density weight (local mode) or nullptr
   const double* sw;              // per-segment max of pw (local mode)
   int* count;                    // NTIER per item
@@ -151,7 +151,7 @@ __global__ void k_tasks(TaskGenArgs g) {
   const int kb = g.pK[i];
   if (qi > 0) {
     const int m = g.pmol[i];
-    const double ffq = g.ffq[m];
+    const double ffq = g.ffq[m].off ? 0.0 : g.ffq[m].q;
     const int s_lo = g.mseg[2 * (Y * g.nmol + m)], s_hi = g.mseg[2 * (Y * g.nmol + m) + 1];
     for (int sidx = s_lo; sidx < s_hi; ++sidx) {
       const int4 s = g.seg[sidx];

@@ -357,16 +357,20 @@ __global__ void k_pair_fields(int np, const int* __restrict__ pA, const int* __r
   }
 }
 
+constexpr double FF_QUARTET_RATIO = 32;   // ff_limits
+
 // Final layouts of the sorted pairs: bra (pair-contiguous) and ket
 // (segment-transposed: primitive k of pair t at data_off + k*len + (t - start)),
-// FP64 and FP32.
+// FP64, FP32 and two-float; a pair outside the two-float range turns that tier off
+// for its molecule.
 __global__ void k_pair_layouts(int np, const int* __restrict__ pA, const int* __restrict__ pB,
                                const int* __restrict__ poff, const int* __restrict__ kseg,
                                const int4* __restrict__ seg, const int4* __restrict__ sh,
                                const double* __restrict__ xyz, const double* __restrict__ coef,
                                const double* __restrict__ expo, long long npp, double* __restrict__ bra64,
                                double* __restrict__ ket64, float* __restrict__ bra32, float* __restrict__ ket32,
-                               ff* __restrict__ braff, ff* __restrict__ ketff) {
+                               ff* __restrict__ braff, ff* __restrict__ ketff, const int* __restrict__ pmol,
+                               FFLimit* __restrict__ ffq) {
   const int t = blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= np) return;
   const int A = pA[t], B = pB[t];
@@ -392,6 +396,12 @@ __global__ void k_pair_layouts(int np, const int* __restrict__ pA, const int* __
       f[BRA_PAX + x] = -fb * ab;
       f[BRA_PBX + x] = fa * ab;
     }
+    double r = 0;
+    for (int x = 0; x < 6; ++x) r = fmax(r, fabs(f[BRA_PAX + x]));
+    FFLimit& lim = ffq[pmol[t]];
+    float size, grow;
+    ff_pair_range(f[BRA_P], f[BRA_K], r, sh[A].w + sh[B].w, size, grow);
+    if (!(size <= FF_MAX_SIZE && grow <= FF_MAX_GROW + 0.5f * log2f((float)(FF_QUARTET_RATIO * lim.q)))) lim.off = 1;
     for (int fl = 0; fl < BRA_NFIELD; ++fl) {
       braff[(long long)fl * npp + bi] = ff(f[fl]);
       ketff[(long long)fl * npp + ki] = ff(f[fl]);
@@ -407,19 +417,20 @@ __global__ void k_pair_layouts(int np, const int* __restrict__ pA, const int* __
 // a handful of tasks and the extra launches cost more than the arithmetic saves
 // (SCF + gradient of a water, 250 pairs: 11.0 -> 11.5 ms with the two-float
 // lists; the dimer's Fock build, 1000 pairs: 377 -> 188 us), and when an exponent, a coefficient or a
-// coordinate is outside the range that FP32 exponents leave for the products.
-static std::vector<double> ff_limits(const Basis& b, const PairData& P) {
+// coordinate is far outside what FP32 exponents hold.  k_pair_layouts then checks what
+// each primitive pair brings into the products (ff_pair_range).
+static std::vector<FFLimit> ff_limits(const Basis& b, const PairData& P) {
+  std::vector<FFLimit> lim(b.nmol, FFLimit{0.0, 0, 0});
   bool range = true;
   for (double e : b.prim_exp) range &= e >= 1e-8 && e <= 1e8;
   for (double k : b.prim_coef) range &= std::fabs(k) <= 1e8;
   for (double x : b.xyz) range &= std::fabs(x) <= 1e5;
-  std::vector<double> lim(b.nmol, 0.0);
   if (!range || P.nprim_pairs < SMALL_PRIM_PAIRS) return lim;
   for (int t = 0; t < P.npairs; ++t) {
-    double& q = lim[b.shells[P.hA[t]].mol];
+    double& q = lim[b.shells[P.hA[t]].mol].q;
     q = std::max(q, P.hQ[t]);
   }
-  for (double& q : lim) q = q * q / 32;
+  for (FFLimit& l : lim) l.q = l.q * l.q / FF_QUARTET_RATIO;
   return lim;
 }
 
@@ -435,11 +446,11 @@ gbhf_status ensure_pairs(gbhf_ctx* c) {
   GBHF_TRY(ensure_boys_tables(c));
   GBHF_TRY(ensure_shell_arrays(c));   // component scales for the d-class Schwarz bounds
   const int ns = (int)b.shells.size();
-  // shell table for the device: atom, primitives, first primitive of the shell's first CGF
+  // shell table for the device: atom, primitives, first primitive of the shell's first CGF, L
   std::vector<int4> shv(ns);
   for (int s2 = 0; s2 < ns; ++s2) {
     const Shell& sh = b.shells[s2];
-    shv[s2] = make_int4(sh.atom, sh.np, b.cgf_off[sh.f0], 0);
+    shv[s2] = make_int4(sh.atom, sh.np, b.cgf_off[sh.f0], sh.L);
   }
   DBuf<int4> dsh;
   GBHF_CUDA(c, dsh.alloc(std::max(ns, 1)));
@@ -627,8 +638,8 @@ gbhf_status ensure_pairs(gbhf_ctx* c) {
   GBHF_CUDA(c, P.ket64.alloc(nf));
   GBHF_CUDA(c, P.bra32.alloc(nf));
   GBHF_CUDA(c, P.ket32.alloc(nf));
-  const std::vector<double> ffq = ff_limits(b, P);
-  const bool use_ff = P.use_ff = *std::max_element(ffq.begin(), ffq.end()) > 0;
+  const std::vector<FFLimit> ffq = ff_limits(b, P);
+  const bool use_ff = P.use_ff = std::any_of(ffq.begin(), ffq.end(), [](const FFLimit& l) { return l.q > 0; });
   if (use_ff) {
     GBHF_TRY(ensure_boys_ff(c));
     GBHF_CUDA(c, P.braff.alloc(nf));
@@ -656,7 +667,7 @@ gbhf_status ensure_pairs(gbhf_ctx* c) {
   GBHF_CUDA(c, P.Qf.alloc(std::max(np, 1)));
   GBHF_CUDA(c, up(P.Qf.p, qf.data(), np * sizeof(float)));
   GBHF_CUDA(c, P.ffq.alloc(ffq.size()));
-  GBHF_CUDA(c, up(P.ffq.p, ffq.data(), ffq.size() * sizeof(double)));
+  GBHF_CUDA(c, up(P.ffq.p, ffq.data(), ffq.size() * sizeof(FFLimit)));
   GBHF_CUDA(c, up(P.seg_info.p, seginfo.data(), seginfo.size() * sizeof(int4)));
   GBHF_CUDA(c, up(P.mol.p, pmol.data(), np * sizeof(int)));
   GBHF_CUDA(c, up(P.mseg.p, P.hmseg.data(), P.hmseg.size() * sizeof(int)));
@@ -664,7 +675,7 @@ gbhf_status ensure_pairs(gbhf_ctx* c) {
     k_pair_layouts<<<(np + 127) / 128, 128, 0, c->stream>>>(np, P.A.p, P.B.p, P.poff.p, P.kseg.p, P.seg_info.p, dsh.p,
                                                             c->d_xyz.p, c->d_coef.p, c->d_exp.p, (long long)npp,
                                                             P.bra64.p, P.ket64.p, P.bra32.p, P.ket32.p, use_ff ? P.braff.p : nullptr,
-                                                            use_ff ? P.ketff.p : nullptr);
+                                                            use_ff ? P.ketff.p : nullptr, P.mol.p, P.ffq.p);
     count_launch(c);
     GBHF_CUDA(c, cudaGetLastError());
   }
