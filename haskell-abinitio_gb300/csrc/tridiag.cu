@@ -37,22 +37,44 @@ constexpr double kEps = DBL_EPSILON;
 
 __host__ __device__ __forceinline__ long pidx(int i, int j) { return (long)i * (i + 1) / 2 + j; }   // j <= i
 
+// The solver squares matrix elements (reflector norms) and vectors of size
+// 1 / (eps ||T||) (inverse iteration), which leaves the FP64 range for elements
+// below about 2^-460 or above 2^510.  A matrix whose largest element lies outside
+// 2^-400 .. 2^400 is therefore reduced after scaling by 2^-x, x the exponent of
+// that element (exact; scal[3] = x, and k_tri_fix scales the eigenvalues back).
+__device__ __forceinline__ int scale_exponent(double amax) {
+  if (!(amax > 0.0 && amax <= DBL_MAX)) return 0;
+  const int x = ilogb(amax);
+  return x < -400 || x > 400 ? x : 0;
+}
+
 // One CTA of 1024 threads.  Shared memory: packed lower triangle of A
 // (n(n+1)/2), v (n), p / w (n).  Outputs: d (n), e (n - 1), tau (n), Vt (row k:
-// reflector k, zero up to column k, 1 at column k + 1; rows 0 .. n - 3).
+// reflector k, zero up to column k, 1 at column k + 1; rows 0 .. n - 3), scal[3].
 __global__ void __launch_bounds__(1024) k_sytrd(int n, const double* __restrict__ A, double* __restrict__ d,
                                                 double* __restrict__ e, double* __restrict__ tau,
-                                                double* __restrict__ Vt) {
+                                                double* __restrict__ Vt, double* __restrict__ scal) {
   extern __shared__ double sm[];
   double* P = sm;
   double* sv = P + pidx(n, 0);   // n(n+1)/2 doubles before it
   double* sp = sv + n;
   __shared__ double s_bc[4];
   const int tid = threadIdx.x, nt = blockDim.x;
+  double amax = 0.0;
   for (long q = tid; q < (long)n * n; q += nt) {
     const int i = (int)(q / n), j = (int)(q % n);
-    if (j <= i) P[pidx(i, j)] = A[q];
+    if (j <= i) {
+      P[pidx(i, j)] = A[q];
+      amax = fmax(amax, fabs(A[q]));
+    }
   }
+  amax = block_reduce(amax, true);
+  if (tid == 0) s_bc[0] = amax;
+  __syncthreads();
+  const int sx = scale_exponent(s_bc[0]);
+  if (tid == 0) scal[3] = sx;
+  if (sx)
+    for (int q = tid; q < (int)pidx(n, 0); q += nt) P[q] = scalbn(P[q], -sx);
   __syncthreads();
   for (int k = 0; k + 2 < n; ++k) {
     const int m = n - 1 - k;   // trailing size, >= 2
@@ -184,11 +206,11 @@ inline size_t sy_smem_bytes(int n, int cs) {
 template <int CS>
 __global__ void __launch_bounds__(SY_THREADS)
     k_sytrd_cluster(int n, const double* __restrict__ A, double* __restrict__ d, double* __restrict__ e,
-                    double* __restrict__ tau, double* __restrict__ Vt) {
+                    double* __restrict__ tau, double* __restrict__ Vt, double* __restrict__ scal) {
   namespace cg = cooperative_groups;
   cg::cluster_group cluster = cg::this_cluster();
   extern __shared__ double sm[];
-  __shared__ double s_bc[3];
+  __shared__ double s_bc[3], s_amax;
   const int r = (int)cluster.block_rank(), tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int nq = n > r ? (n - r + CS - 1) / CS : 0;   // rows owned: r + CS q
   const int ld = sy_ld(n);
@@ -199,13 +221,28 @@ __global__ void __launch_bounds__(SY_THREADS)
   double* vp = v + n;       // the last step's v and w
   double* wp = vp + n;
   double* P = wp + n;       // owned rows
+  double amax = 0.0;
   for (int q = warp; q < nq; q += SY_WARPS)
     for (int j = lane; j < n; j += 32) {   // the lower triangle is what counts
       const int i = r + CS * q;
-      P[q * ld + j] = j <= i ? A[(long)i * n + j] : A[(long)j * n + i];
+      const double a = j <= i ? A[(long)i * n + j] : A[(long)j * n + i];
+      P[q * ld + j] = a;
+      amax = fmax(amax, fabs(a));
     }
   for (int i = tid; i < n; i += SY_THREADS) vp[i] = wp[i] = 0.0;
+  amax = block_reduce(amax, true);
+  if (tid == 0) s_amax = amax;
   cluster.sync();
+  amax = lane < CS ? *cluster.map_shared_rank(&s_amax, lane) : 0.0;
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) amax = fmax(amax, __shfl_xor_sync(0xffffffffu, amax, o));
+  const int sx = scale_exponent(amax);   // the same in every thread of the cluster
+  if (r == 0 && tid == 0) scal[3] = sx;
+  if (sx) {
+    for (int q = warp; q < nq; q += SY_WARPS)
+      for (int j = lane; j < n; j += 32) P[q * ld + j] = scalbn(P[q * ld + j], -sx);
+    __syncthreads();
+  }
   for (int k = 0; k + 2 < n; ++k) {
     const int q0 = k >= r ? (k - r) / CS + 1 : 0;   // first own row > k
     // A: column k of own rows > k, to every CTA
@@ -333,7 +370,7 @@ gbhf_status launch_sytrd(gbhf_ctx* c, int n, const double* d_A, TridiagWork& w) 
   cudaLaunchConfig_t cfg;
   cudaLaunchAttribute attr;
   GBHF_TRY(sytrd_config<CS>(c, n, cfg, attr));
-  GBHF_CUDA(c, cudaLaunchKernelEx(&cfg, k_sytrd_cluster<CS>, n, d_A, w.d.p, w.e.p, w.tau.p, w.Vt.p));
+  GBHF_CUDA(c, cudaLaunchKernelEx(&cfg, k_sytrd_cluster<CS>, n, d_A, w.d.p, w.e.p, w.tau.p, w.Vt.p, w.scal.p));
   count_launch(c);
   return GBHF_OK;
 }
@@ -667,6 +704,7 @@ __global__ void __launch_bounds__(256) k_tri_fix(int n, const double* __restrict
   __shared__ double sl[TRIDIAG_WIDE_MAX_N];
   __shared__ unsigned char close[TRIDIAG_WIDE_MAX_N];
   const double tnorm = scal[0];
+  const int sx = (int)scal[3];   // exponent of the scaling (scale_exponent)
   for (int k = threadIdx.x; k < n; k += blockDim.x) {
     sl[k] = lam[k];
     close[k] = k > 0 && blk[k] == blk[k - 1] && blk[k] != blk[n + k] && lam[k] - lam[k - 1] < 1e-11 * tnorm;
@@ -691,7 +729,7 @@ __global__ void __launch_bounds__(256) k_tri_fix(int n, const double* __restrict
       r += (u < v) || (u == v && q < k);
     }
     rank[k] = r;
-    evals[r] = v;
+    evals[r] = sx ? scalbn(v, sx) : v;
   }
 }
 
@@ -809,7 +847,7 @@ gbhf_status eigh_tridiag(gbhf_ctx* c, int n, const double* d_A, double* d_evals,
   } else if (c->sytrd16 && !c->force_sytrd_single && n >= 32) {
     GBHF_TRY(launch_sytrd<16>(c, n, d_A, w));
   } else {
-    k_sytrd<<<1, 1024, smem, c->stream>>>(n, d_A, w.d.p, w.e.p, w.tau.p, w.Vt.p);
+    k_sytrd<<<1, 1024, smem, c->stream>>>(n, d_A, w.d.p, w.e.p, w.tau.p, w.Vt.p, w.scal.p);
     count_launch(c);
     GBHF_LAUNCHED(c, "k_sytrd launch");
   }

@@ -49,3 +49,18 @@ def test_non_finite_matrix_is_reported(ctx):
     a[7, 7] = np.nan
     with pytest.raises(_lib.NotConverged):
         ctx.eigen_solve(a)
+
+
+@pytest.mark.parametrize("n", [2, 20, 200, 240, 300])
+@pytest.mark.parametrize("power", [-520, -470, -401, 401, 500])
+def test_elements_far_from_one(ctx, n, power):
+    """A power of two on every element scales the eigenvalues by it and leaves the
+    vectors as they are, also where squares of the elements leave the FP64 range."""
+    a = np.random.default_rng(n).standard_normal((n, n))
+    a = a + a.T
+    w, v = ctx.eigen_solve(a * 2.0 ** power)
+    w = w * 2.0 ** -power
+    sc = max(1.0, np.abs(w).max())
+    np.testing.assert_allclose(w, np.linalg.eigvalsh(a), rtol=0, atol=1e-12 * sc)
+    assert np.max(np.abs(a @ v - v * w)) < 1e-11 * sc
+    assert np.max(np.abs(v.T @ v - np.eye(n))) < 1e-12
