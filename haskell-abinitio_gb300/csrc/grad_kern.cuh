@@ -105,6 +105,12 @@ struct GradArgs {
   const int* dexp;
 };
 
+// The screening threshold of two-float kernels, whose Gamma is 2^-dex times the
+// density's, rounded down by more than the FP32 magnitudes beside it are.
+__device__ __forceinline__ float grad_threshold(double thr, int dex) {
+  return __double2float_rd(scalbn(thr * (1.0 - 3e-7), -dex));
+}
+
 __device__ __forceinline__ double warp_sum_d(double v) {
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
@@ -260,7 +266,7 @@ __global__ void __launch_bounds__(GR_THREADS) k_grad_jk(GradArgs<T> a) {
   float thrs = (float)a.thr;
   if constexpr (FF) {
     dex = 2 * *a.dexp;
-    thrs = (float)scalbn(a.thr, -dex);
+    thrs = grad_threshold(a.thr, dex);
   }
   const int start = a.range[0];
   const int ntask = a.range[1] - start;
@@ -352,7 +358,7 @@ __global__ void __launch_bounds__(TH) k_grad_jk_step(GradArgs<T> a) {
   float thrs = (float)a.thr;
   if constexpr (FF) {
     dex = 2 * *a.dexp;
-    thrs = (float)scalbn(a.thr, -dex);
+    thrs = grad_threshold(a.thr, dex);
   }
   const int start = a.range[0];
   const int ntask = a.range[1] - start;

@@ -10,7 +10,8 @@
 // block (four gathers from two rows that stay in L1, the rest coalesced),
 // queues the survivors in shared memory and evaluates them in full batches.
 // Magnitudes are rounded up to FP32 and the threshold down, so a quartet that
-// the FP64 test would keep is kept.
+// the FP64 test would keep is kept; a density above the FP32 range has infinite
+// maxima, and where those meet a zero block (NaN) the quartet is kept as well.
 #pragma once
 #include "gbhf_internal.h"
 
@@ -52,14 +53,14 @@ struct BraScreen {
     if (!s.Ds) return true;
     const int4 p = s.pinfo[jk];
     const float d = fmaxf(fmaxf(fmaxf(ra[p.x], ra[p.y]), fmaxf(rb[p.x], rb[p.y])), fmaxf(dab, s.pbf[jk]));
-    return q * s.Qf[jk] * d >= s.thr;
+    return !(q * s.Qf[jk] * d < s.thr);
   }
   // Q_ab Q_cd times a bound of |Gamma| = |jcoef D_ab D_cd - (D_ac D_bd + D_ad D_bc) / 4|
   __device__ __forceinline__ bool gamma_pass(const QuartetScreen& s, int jk, float jcoef) const {
     if (!s.Ds) return true;
     const int4 p = s.pinfo[jk];
     const float g = fabsf(jcoef) * dab * s.pbf[jk] + 0.25f * (ra[p.x] * rb[p.y] + ra[p.y] * rb[p.x]);
-    return q * s.Qf[jk] * g * 1.000001f >= s.thr;
+    return !(q * s.Qf[jk] * g * 1.000001f < s.thr);
   }
 };
 

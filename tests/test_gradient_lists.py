@@ -62,3 +62,26 @@ def test_one_electron_terms_against_differences(ctx, waters, basis):
             c[atom, x] += k * step
             f.append(value(c))
         assert abs((f[0] - 8 * f[1] + 8 * f[2] - f[3]) / (12 * step) - got[atom, x]) < 1e-7
+
+
+@pytest.mark.parametrize("open_shell", [False, True])
+def test_gradient_of_densities_outside_the_fp32_range(ctx, open_shell):
+    """The two-electron gradient is quadratic in the density, also where block maxima
+    leave the FP32 range beside blocks that are zero (1e-12 of its largest component:
+    the order of the FP64 atomics differs)."""
+    xyz = M.water_cluster(3, np.random.default_rng(3))
+    fb = B.flatten(B.make_atoms(M.water_labels(3), xyz, "6-31g"))
+    ctx.set_basis(fb)
+    d = np.random.default_rng(2).standard_normal((fb.n_cgf, fb.n_cgf))
+    d = (d + d.T) * (fb.cgf_atom[:, None] == fb.cgf_atom[None])   # no blocks between atoms
+    zero = np.zeros(fb.n_cgf * (fb.n_cgf + 1) // 2)
+
+    def two_electron(scale):
+        def grad(sign):
+            t = O.square_to_tri(d * (sign * scale))
+            return ctx.gradient_uhf(t, -0.5 * t, zero, schwarz=0.0) if open_shell else ctx.gradient(t, zero, schwarz=0.0)
+        return 0.5 * (grad(1.0) + grad(-1.0)) / scale ** 2
+
+    nuc = ctx.gradient(zero, zero)
+    one, far = two_electron(1.0) - nuc, two_electron(2.0 ** 200)
+    np.testing.assert_allclose(far, one, rtol=0, atol=1e-12 * np.abs(one).max())
