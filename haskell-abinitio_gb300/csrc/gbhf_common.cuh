@@ -262,6 +262,25 @@ __device__ __forceinline__ void boys_eval(T t, const T* __restrict__ tab, T* F) 
   else boys_eval_num<T, L>(t, tab, F);
 }
 
+// One tick of a block whose warps go through long code in step (k_jk_step,
+// k_grad_jk_step): every warp of the block meets the others here; true when any of
+// them passed `work`.  The calls stand at several places, which PTX allows (a barrier
+// is its number, not its place in the code), and inside loops whose body the lanes of a
+// warp leave apart: __syncwarp and the barrier's form without .aligned ask for no more
+// than that every thread arrives.  Every one does: a warp ticks a finite number of times
+// for each batch of a finite task list, then ticks without work until none has any.
+__device__ __forceinline__ bool block_tick(bool work) {
+  __syncwarp();
+  int any;
+  asm volatile(
+      "{\n\t.reg .pred p, q;\n\tsetp.ne.s32 p, %1, 0;\n\tbarrier.cta.red.or.pred q, 1, p;\n\t"
+      "selp.s32 %0, 1, 0, q;\n\t}"
+      : "=r"(any)
+      : "r"((int)work)
+      : "memory");
+  return any != 0;
+}
+
 // Error codes written by kernels into the context's device status word.
 #define GBHF_DEV_ERR_TIMEOUT 1
 #define GBHF_DEV_ERR_NOTCONV 2

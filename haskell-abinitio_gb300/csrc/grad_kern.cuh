@@ -223,7 +223,7 @@ __device__ __forceinline__ void grad_batch(const GradArgs<T>& a, GamT& gam, TkT&
       const bool mine = keep && k0 + sk < K;
       if (mine) ket_prim(k0 + sk);
       for (int kb = 0; kb < nbu; ++kb) {
-        __syncthreads_or(1);   // a tick
+        block_tick(true);
         if (mine && kb < nbl)
           GradFn<LA, LB, LC, LD>::run(sbra + (sb + kb * nsb) * BRA_SB, 1, BRA_SB, q, Qx, Qy, Qz, Kcd, a.boys, tk, g);
       }
@@ -416,7 +416,7 @@ __global__ void __launch_bounds__(TH) k_grad_jk_step(GradArgs<T> a) {
       queue_pop(sq[warp], queued, nk, lane);
     }
   }
-  while (__syncthreads_or(0)) {   // keeps ticking until the block's other warps are done as well
+  while (block_tick(false)) {   // keeps ticking until the block's other warps are done as well
   }
 }
 

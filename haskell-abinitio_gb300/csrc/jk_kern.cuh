@@ -39,7 +39,7 @@ struct StepCount {
 };
 __device__ __forceinline__ int nb_end(StepCount n) { return n.all; }
 __device__ __forceinline__ bool nb_skip(StepCount n, int kb) {
-  __syncthreads_or(1);   // a tick
+  block_tick(true);
   return kb >= n.own;
 }
 
@@ -504,7 +504,7 @@ __global__ void __launch_bounds__(TH) k_jk_step(JKArgs<T> a) {
                                             a.D + a.moff[mol], a.G + a.moff[mol], dex, cnt_q, cnt_p);
     queue_pop(sq[warp], queued, nk, lane);
   }
-  while (__syncthreads_or(0)) {   // keeps ticking until the block's other warps are done as well
+  while (block_tick(false)) {   // keeps ticking until the block's other warps are done as well
   }
   cnt_q = (unsigned long long)warp_sum((double)cnt_q);
   cnt_p = (unsigned long long)warp_sum((double)cnt_p);
