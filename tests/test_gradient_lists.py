@@ -72,8 +72,11 @@ def test_gradient_of_densities_outside_the_fp32_range(ctx, open_shell):
     xyz = M.water_cluster(3, np.random.default_rng(3))
     fb = B.flatten(B.make_atoms(M.water_labels(3), xyz, "6-31g"))
     ctx.set_basis(fb)
-    d = np.random.default_rng(2).standard_normal((fb.n_cgf, fb.n_cgf))
-    d = (d + d.T) * (fb.cgf_atom[:, None] == fb.cgf_atom[None])   # no blocks between atoms
+    rng = np.random.default_rng(2)
+    d = rng.standard_normal((fb.n_cgf, fb.n_cgf))
+    at = fb.cgf_atom
+    some = rng.random((fb.n_atoms, fb.n_atoms)) < 0.5   # about a third of the atom blocks is zero
+    d = (d + d.T) * (some | some.T | np.eye(fb.n_atoms, dtype=bool))[at[:, None], at[None]]
     zero = np.zeros(fb.n_cgf * (fb.n_cgf + 1) // 2)
 
     def two_electron(scale):
