@@ -264,8 +264,9 @@ gbhf_status gbhf_fock(gbhf_ctx* c, int mode, int precision, double schwarz_cutof
   GBHF_TRY(flat_to_square(c, n, fD, Dsq));
   GBHF_TRY(flat_to_square(c, n, fH, Hsq));
   GBHF_CUDA(c, cudaMemsetAsync(Gpp, 0, nn * sizeof(double), c->stream));
-  GBHF_TRY(jk_build(c, Dsq, Gpp, precision, schwarz_cutoff, mixed_cutoff, 1.0));
-  GBHF_TRY(add_sym(c, n, Hsq, Gpp, Fsq));
+  const double* Gff = nullptr;
+  GBHF_TRY(jk_build(c, Dsq, Gpp, precision, schwarz_cutoff, mixed_cutoff, 1.0, false, true, &Gff));
+  GBHF_TRY(add_sym(c, n, Hsq, Gpp, Fsq, Gff));
   GBHF_TRY(square_to_flat(c, n, Fsq, fF));
   return download(c, f_flat, fF, ntri * sizeof(double));
 }

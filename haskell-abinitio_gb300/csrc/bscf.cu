@@ -150,10 +150,12 @@ __global__ void __launch_bounds__(128) k_bgemm(BDesc d, int ta, int tb, int sym,
   (void)i;                                                          \
   (void)j
 
-// out = base + G + G^T (base may be nullptr or alias out)
-__global__ void k_b_addsym(BDesc d, const double* base, const double* __restrict__ G, double* out) {
+// out = base + G + G^T (base may be nullptr or alias out), G = G1 + G2 where there is a G2
+__global__ void k_b_addsym(BDesc d, const double* base, const double* __restrict__ G1, const double* __restrict__ G2,
+                           double* out) {
   BD_ELEMENT;
-  const double v = G[o + (long)i * n + j] + G[o + (long)j * n + i];
+  const long long ij = o + (long)i * n + j, ji = o + (long)j * n + i;
+  const double v = G2 ? (G1[ij] + G2[ij]) + (G1[ji] + G2[ji]) : G1[ij] + G1[ji];
   out[o + idx] = (base ? base[o + idx] : 0.0) + v;
 }
 
@@ -786,17 +788,18 @@ gbhf_status bscf_run(gbhf_ctx* c, const gbhf_scf_opts* o, double* energies, int*
                       since_full >= (o->full_rebuild_every > 0 ? o->full_rebuild_every : (1 << 30)) || step == 0 ||
                       fp64_final_phase;
     GBHF_CUDA(c, cudaMemsetAsync(Gpp, 0, nst * sizeof(double), c->stream));
+    const double* Gff = nullptr;
     if (full) {
       c->tasks.thr_all = -1;   // the active set may have changed since the cached lists
-      status = jk_build(c, D, Gpp, precision, o->schwarz_cutoff, o->mixed_cutoff, 1.0);
+      status = jk_build(c, D, Gpp, precision, o->schwarz_cutoff, o->mixed_cutoff, 1.0, false, true, &Gff);
       if (status != GBHF_OK) break;
-      k_b_addsym<<<br.egrid(), 256, 0, c->stream>>>(br.desc, nullptr, Gpp, Gacc);
+      k_b_addsym<<<br.egrid(), 256, 0, c->stream>>>(br.desc, nullptr, Gpp, Gff, Gacc);
       since_full = 1;
     } else {
       GBHF_TRY(axpby(c, nst, 1.0, D, -1.0, Dref, Dn));   // dD (Dn as scratch)
-      status = jk_build(c, Dn, Gpp, precision, o->schwarz_cutoff, o->mixed_cutoff, 1.0, true);
+      status = jk_build(c, Dn, Gpp, precision, o->schwarz_cutoff, o->mixed_cutoff, 1.0, true, true, &Gff);
       if (status != GBHF_OK) break;
-      k_b_addsym<<<br.egrid(), 256, 0, c->stream>>>(br.desc, Gacc, Gpp, Gacc);
+      k_b_addsym<<<br.egrid(), 256, 0, c->stream>>>(br.desc, Gacc, Gpp, Gff, Gacc);
       ++since_full;
     }
     count_launch(c);

@@ -372,6 +372,7 @@ struct gbhf_ctx {
   gbhf::DBuf<float> dfloat;
   gbhf::DBuf<gbhf::ff> dff;         // density of the two-float kernels, scaled by 2^-e
   gbhf::DBuf<int> dff_exp;          // e
+  gbhf::DBuf<double> gff;           // the two-float launches' accumulator of a J/K build
   gbhf::DBuf<int> dev_status;
   int purify_grid = 0;              // co-resident blocks of the fused purification kernel
   int tc2_per_sm = 0;               // blocks per SM of the one-barrier TC2 kernel (0: not asked yet)
@@ -510,11 +511,14 @@ gbhf_status boys_ref_grid_dev(gbhf_ctx* c, double* d_grid);
 gbhf_status ensure_shell_arrays(gbhf_ctx* c);
 gbhf_status build_grad_tasks(gbhf_ctx* c, const double* d_D, double cutoff, double mixed_cutoff, int precision);
 // with_j = false: exchange only, G = -K(D)/2 (the open-shell spin-density term).
+// d_Gff: receives the accumulator of the two-float launches (null: none ran), which the
+// caller adds to G_acc (add_sym); without it jk_build adds it.
 // Add the J/K kernels' counters of the builds since the last call to the
 // profile (one copy and one host synchronisation).
 gbhf_status flush_jk_stats(gbhf_ctx* c);
 gbhf_status jk_build(gbhf_ctx* c, const double* d_Dsq, double* d_G, int precision, double schwarz,
-                     double mixed_cutoff, double weight, bool local_weights = false, bool with_j = true);
+                     double mixed_cutoff, double weight, bool local_weights = false, bool with_j = true,
+                     const double** d_Gff = nullptr);
 // Q of every pair in [cls_start[cl], cls_start[cl+1]) (pairs grouped by class,
 // bra-layout primitive data at d_poff), FP64 class code.
 gbhf_status schwarz_classes_dev(gbhf_ctx* c, const int* cls_start, const int* d_K, const int* d_poff,
@@ -596,7 +600,8 @@ gbhf_status lincomb(gbhf_ctx* c, int n2, int k, const double* const* mats, const
 gbhf_status reduce_stats(gbhf_ctx* c, int n, const double* d_e, const double* d_H, const double* d_F,
                          const double* d_Dnew, const double* d_Dold, double* host_out4);
 gbhf_status axpby(gbhf_ctx* c, size_t n, double a, const double* x, double b, const double* y, double* out);
-gbhf_status add_sym(gbhf_ctx* c, int n, const double* d_H, const double* d_Gpp, double* d_out);
+gbhf_status add_sym(gbhf_ctx* c, int n, const double* d_H, const double* d_Gpp, double* d_out,
+                    const double* d_Gff = nullptr);
 gbhf_status max_abs(gbhf_ctx* c, size_t n, const double* d_x, double* host_out);
 // Purification record slots in c->small and its checks (the deferred one runs
 // in reduce_stats; purify_flush reads a pending one on its own).  c->small holds

@@ -360,7 +360,7 @@ __global__ void k_shell_dmax(int ns, const int* __restrict__ f0, const int* __re
 // FP32 (d32) and two-float (dff), the latter scaled by 2^-e with e the exponent
 // of max |D| (clamped to +-400; 0 when the maximum is 0 or not finite), so that
 // any density an FP64 build takes stays inside the FP32 exponent range; and it
-// zeroes the work-queue heads.
+// zeroes the work-queue heads and the two-float accumulator (gff, where asked for).
 struct PrepArgs {
   int np, ns;
   const int *pA, *pB, *pmol, *f0, *nc, *mn;
@@ -373,6 +373,7 @@ struct PrepArgs {
   float* d32;
   ff* dff;
   int* dexp;
+  double* gff;
   int* counters;
   int ncounters;
 };
@@ -407,6 +408,7 @@ __global__ void __launch_bounds__(128) k_density_prep(PrepArgs a) {
     const double v = a.D[i] * sc;
     const float h = (float)v;
     a.dff[i] = ff(h, (float)(v - (double)h));
+    if (a.gff) a.gff[i] = 0.0;
   }
 }
 
@@ -441,10 +443,10 @@ static gbhf_status to_float(gbhf_ctx* c, size_t n, const double* d_x, float* d_y
 
 // Everything the kernels of the next build need of its density d_dD: maxima for
 // the screening (c->tasks.Ds, pbf), FP32 and two-float copies, zeroed work-queue
-// heads of st (ncounters) and, with `segments`, the segment maxima of the weighted
-// task lists.
+// heads of st (ncounters), a zeroed c->gff (`fock`) and, with `segments`, the segment
+// maxima of the weighted task lists.
 static gbhf_status density_prep(gbhf_ctx* c, TaskLists& st, const double* d_dD, int precision, int ncounters,
-                                bool segments) {
+                                bool segments, bool fock) {
   PairData& P = c->pairs;
   TaskLists& sh = c->tasks;   // per-shell and per-molecule arrays
   const int ns = (int)c->basis.shells.size();
@@ -460,12 +462,13 @@ static gbhf_status density_prep(gbhf_ctx* c, TaskLists& st, const double* d_dD, 
   if (P.use_ff) {
     GBHF_CUDA(c, c->dff.alloc(nst));
     GBHF_CUDA(c, c->dff_exp.alloc(1));
+    if (fock) GBHF_CUDA(c, c->gff.alloc(nst));
   }
   k_shell_dmax<<<ns, 128, 0, c->stream>>>(ns, sh.f0.p, sh.nc.p, sh.smol.p, sh.mn.p, sh.moff.p, sh.ms0.p, sh.soff.p, d_dD,
                                           st.row.p, sh.Ds.p);
   const PrepArgs a{P.npairs,   ns,          P.A.p, P.B.p,  P.mol.p, sh.f0.p, sh.nc.p, sh.mn.p, sh.moff.p, d_dD, st.row.p,
                    st.pw.p,    st.pb.p,     sh.pbf.p, nst, precision != GBHF_PREC_FP64 ? c->dfloat.p : nullptr,
-                   P.use_ff ? c->dff.p : nullptr, c->dff_exp.p, st.counters.p, ncounters};
+                   P.use_ff ? c->dff.p : nullptr, c->dff_exp.p, P.use_ff && fock ? c->gff.p : nullptr, st.counters.p, ncounters};
   const int blocks = (int)std::min<size_t>((std::max<size_t>(P.npairs, nst) + 127) / 128, (size_t)c->nsm * 8);
   k_density_prep<<<std::max(blocks, 1), 128, 0, c->stream>>>(a);
   if (segments && P.nseg_total > 0) {
@@ -733,7 +736,7 @@ gbhf_status build_grad_tasks(gbhf_ctx* c, const double* d_D, double cutoff, doub
   GBHF_TRY(ensure_pairs(c));
   GBHF_TRY(ensure_shell_arrays(c));
   TaskLists& gt = c->gtasks;
-  GBHF_TRY(density_prep(c, gt, d_D, precision, NTIER * NCOMBO_MAX, true));
+  GBHF_TRY(density_prep(c, gt, d_D, precision, NTIER * NCOMBO_MAX, true, false));
   // FP32 up to the cutoff, but never above a bound of 1/8: two floats take the
   // rest of what a larger cutoff gives to FP32
   const double t64 = precision == GBHF_PREC_FP64 ? 0.0 : std::min(mixed_cutoff, 0.125);
@@ -743,7 +746,7 @@ gbhf_status build_grad_tasks(gbhf_ctx* c, const double* d_D, double cutoff, doub
 }
 
 gbhf_status jk_build(gbhf_ctx* c, const double* d_Dsq, double* d_G, int precision, double schwarz,
-                     double mixed_cutoff, double weight, bool local_weights, bool with_j) {
+                     double mixed_cutoff, double weight, bool local_weights, bool with_j, const double** d_Gff) {
   const int wj = with_j ? 1 : 0;
   c->tasks.thr_exact = schwarz;   // per-quartet test in the kernels, on the density passed here
   GBHF_TRY(ensure_pairs(c));
@@ -751,7 +754,7 @@ gbhf_status jk_build(gbhf_ctx* c, const double* d_Dsq, double* d_G, int precisio
   TaskLists& st = c->tasks;
   GBHF_TRY(ensure_shell_arrays(c));
   if (local_weights || P.nprim_pairs >= SMALL_PRIM_PAIRS) {
-    GBHF_TRY(density_prep(c, st, d_Dsq, precision, NTIER * NCOMBO, local_weights));
+    GBHF_TRY(density_prep(c, st, d_Dsq, precision, NTIER * NCOMBO, local_weights, true));
   } else {
     st.screened = false;
     GBHF_CUDA(c, st.counters.alloc(NTIER * NCOMBO));
@@ -801,6 +804,12 @@ gbhf_status jk_build(gbhf_ctx* c, const double* d_Dsq, double* d_G, int precisio
   // ((H2O)64 mixed, 3.1 million tasks: 56.2 ms in order, 61.8 on eight streams;
   // (H2O)16, 170 thousand: 42.7 against 39.4 ms per SCF)
   const int nside = total >= (1l << 20) ? 1 : gbhf_ctx::NSIDE;
+  // The two-float launches add into an accumulator of their own.  Theirs are many small
+  // terms, and into the common one, near its final size once the FP64 launches are
+  // through, each was rounded at that size: the FP64 Fock matrix of (H2O)8/6-31G was
+  // 1.0e-14 rms from its exact value ((H2O)16 1.8e-14), against 7.8e-15 (1.2e-14) by
+  // FP64 arithmetic alone and 2.8e-15 (3.8e-15) now.
+  bool two_float = false;
   int ne = 0, nl = 0;
   int ev_combo[NTIER * NCOMBO], ev_prec[NTIER * NCOMBO];
   if (ev) GBHF_CUDA(c, cudaEventRecord(c->evc[ne], c->stream));
@@ -814,10 +823,12 @@ gbhf_status jk_build(gbhf_ctx* c, const double* d_Dsq, double* d_G, int precisio
       if (nt[k][tier] <= 0) continue;
       cudaStream_t strm = ev ? c->stream : c->side[nl % nside];
       ++nl;
-      if (k >= NCOMBO_SP && !gen_dclass(k)) GBHF_TRY(launch_jk_dclass(c, strm, k, tier, d_Dsq, d_G, nt[k][tier], wj));
-      else if (tier == TIER_64) GBHF_TRY(launch_combo<double>(c, strm, k, tier, d_Dsq, d_G, nt[k][tier], wj));
-      else if (tier == TIER_32) GBHF_TRY(launch_combo<float>(c, strm, k, tier, c->dfloat.p, d_G, nt[k][tier], wj));
-      else GBHF_TRY(launch_jk_ff(c, strm, k, d_G, nt[k][tier], wj));
+      double* G = tier == TIER_FF ? c->gff.p : d_G;
+      two_float |= tier == TIER_FF;
+      if (k >= NCOMBO_SP && !gen_dclass(k)) GBHF_TRY(launch_jk_dclass(c, strm, k, tier, d_Dsq, G, nt[k][tier], wj));
+      else if (tier == TIER_64) GBHF_TRY(launch_combo<double>(c, strm, k, tier, d_Dsq, G, nt[k][tier], wj));
+      else if (tier == TIER_32) GBHF_TRY(launch_combo<float>(c, strm, k, tier, c->dfloat.p, G, nt[k][tier], wj));
+      else GBHF_TRY(launch_jk_ff(c, strm, k, G, nt[k][tier], wj));
       if (ev) {
         ev_combo[ne] = k;
         ev_prec[ne] = tier == TIER_32 ? 1 : 0;   // two-float work counts as FP64 in the profile
@@ -832,6 +843,8 @@ gbhf_status jk_build(gbhf_ctx* c, const double* d_Dsq, double* d_G, int precisio
       GBHF_CUDA(c, cudaStreamWaitEvent(c->stream, c->join_ev[i], 0));
     }
   }
+  if (d_Gff) *d_Gff = two_float ? c->gff.p : nullptr;
+  else if (two_float) GBHF_TRY(axpby(c, (size_t)c->basis.stacked, 1.0, d_G, 1.0, c->gff.p, d_G));
   // statistics: read with the per-class event times when those are taken,
   // else when the profile is read (no host synchronisation per build)
   if (!ev) return GBHF_OK;

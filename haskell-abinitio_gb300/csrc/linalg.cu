@@ -324,16 +324,23 @@ gbhf_status axpby(gbhf_ctx* c, size_t n, double a, const double* x, double b, co
   return GBHF_OK;
 }
 
-// out = H + G + G^T (all square)
-__global__ void k_add_sym(int n, const double* __restrict__ H, const double* __restrict__ G, double* __restrict__ out) {
+// out = H + G + G^T (all square), G = G1 + G2 where there is a G2
+__global__ void k_add_sym(int n, const double* __restrict__ H, const double* __restrict__ G1,
+                          const double* __restrict__ G2, double* __restrict__ out) {
   const int i = blockIdx.y, j = blockIdx.x * blockDim.x + threadIdx.x;
   if (j >= n) return;
   const long ij = (long)i * n + j, ji = (long)j * n + i;
-  out[ij] = (H ? H[ij] : 0.0) + G[ij] + G[ji];
+  double g = G1[ij], gt = G1[ji];
+  if (G2) {
+    g += G2[ij];
+    gt += G2[ji];
+  }
+  out[ij] = (H ? H[ij] : 0.0) + g + gt;
 }
 
-gbhf_status add_sym(gbhf_ctx* c, int n, const double* d_H, const double* d_Gpp, double* d_out) {
-  k_add_sym<<<dim3((n + 127) / 128, n), 128, 0, c->stream>>>(n, d_H, d_Gpp, d_out);
+gbhf_status add_sym(gbhf_ctx* c, int n, const double* d_H, const double* d_Gpp, double* d_out,
+                    const double* d_Gff) {
+  k_add_sym<<<dim3((n + 127) / 128, n), 128, 0, c->stream>>>(n, d_H, d_Gpp, d_Gff, d_out);
   count_launch(c);
   GBHF_CUDA(c, cudaGetLastError());
   return GBHF_OK;

@@ -253,16 +253,17 @@ gbhf_status scf_run(gbhf_ctx* c, const gbhf_scf_opts* o, gbhf_result* r) {
       const bool full = !o->incremental || since_full >= (o->full_rebuild_every > 0 ? o->full_rebuild_every : (1 << 30)) ||
                         step == 0 || fp64_final_phase;
       GBHF_CUDA(c, cudaMemsetAsync(Gpp, 0, nn * sizeof(double), c->stream));
+      const double* Gff = nullptr;
       if (full) {
-        GBHF_TRY(jk_build(c, D, Gpp, precision, o->schwarz_cutoff, o->mixed_cutoff, 1.0));
-        GBHF_TRY(add_sym(c, n, nullptr, Gpp, Gacc));
+        GBHF_TRY(jk_build(c, D, Gpp, precision, o->schwarz_cutoff, o->mixed_cutoff, 1.0, false, true, &Gff));
+        GBHF_TRY(add_sym(c, n, nullptr, Gpp, Gacc, Gff));
         since_full = 1;
       } else {
         GBHF_TRY(axpby(c, nn, 1.0, D, -1.0, Dref, Dnew));   // dD (Dnew as scratch)
         // per-pair weights from the local size of dD (tighter than its global
         // max; a zero dD leaves the task lists empty)
-        GBHF_TRY(jk_build(c, Dnew, Gpp, precision, o->schwarz_cutoff, o->mixed_cutoff, 1.0, true));
-        GBHF_TRY(add_sym(c, n, Gacc, Gpp, Gacc));
+        GBHF_TRY(jk_build(c, Dnew, Gpp, precision, o->schwarz_cutoff, o->mixed_cutoff, 1.0, true, true, &Gff));
+        GBHF_TRY(add_sym(c, n, Gacc, Gpp, Gacc, Gff));
         ++since_full;
       }
       GBHF_CUDA(c, cudaMemcpyAsync(Dref, D, nn * sizeof(double), cudaMemcpyDeviceToDevice, c->stream));

@@ -147,11 +147,12 @@ gbhf_status uhf_run(gbhf_ctx* c, const gbhf_scf_opts* o, int multiplicity, gbhf_
     GBHF_TRY(axpby(c, nn, 1.0, Da.p, 1.0, Db.p, DT.p));
     GBHF_TRY(axpby(c, nn, 1.0, Da.p, -1.0, Db.p, Ds.p));
     GBHF_CUDA(c, cudaMemsetAsync(Gpp.p, 0, nn * sizeof(double), c->stream));
-    GBHF_TRY(jk_build(c, DT.p, Gpp.p, o->precision, o->schwarz_cutoff, o->mixed_cutoff, 1.0));
-    GBHF_TRY(add_sym(c, n, nullptr, Gpp.p, GT.p));
+    const double* Gff = nullptr;
+    GBHF_TRY(jk_build(c, DT.p, Gpp.p, o->precision, o->schwarz_cutoff, o->mixed_cutoff, 1.0, false, true, &Gff));
+    GBHF_TRY(add_sym(c, n, nullptr, Gpp.p, GT.p, Gff));
     GBHF_CUDA(c, cudaMemsetAsync(Gpp.p, 0, nn * sizeof(double), c->stream));
-    GBHF_TRY(jk_build(c, Ds.p, Gpp.p, o->precision, o->schwarz_cutoff, o->mixed_cutoff, 1.0, false, false));
-    GBHF_TRY(add_sym(c, n, nullptr, Gpp.p, GK.p));   // -K(D_s)/2
+    GBHF_TRY(jk_build(c, Ds.p, Gpp.p, o->precision, o->schwarz_cutoff, o->mixed_cutoff, 1.0, false, false, &Gff));
+    GBHF_TRY(add_sym(c, n, nullptr, Gpp.p, GK.p, Gff));   // -K(D_s)/2
     GBHF_TRY(axpby(c, nn, 1.0, H.p, 1.0, GT.p, T1.p));
     GBHF_TRY(axpby(c, nn, 1.0, T1.p, 1.0, GK.p, Fa.p));
     GBHF_TRY(axpby(c, nn, 1.0, T1.p, -1.0, GK.p, Fb.p));
