@@ -513,8 +513,12 @@ static gbhf_status build_task_lists(gbhf_ctx* c, TaskLists& TL, int ncombo, cons
   // 32-ket groups that a task of the s/p J/K kernels scans: the queue of survivors
   // then fills whole batches, and the bra is staged once for all of them, while
   // there are tasks enough for every warp ((H2O)64 mixed build in order: 65.9 ms
-  // at 1, 57.3 at 4, 56.2 at 8, 55.8 at 16; (H2O)16 mixed SCF 40.4, 39.3, 39.6, 40.3)
-  const int scan = P.npairs >= 65536 ? 8 : 4;
+  // at 1, 57.3 at 4, 56.2 at 8, 55.8 at 16; (H2O)16 mixed SCF 40.4, 39.3, 39.6, 40.3).
+  // Below that a task of several groups is a longer serial chain.  FP64 Fock builds at 1
+  // and 4: (H2O)2/STO-3G 0.168 and 0.195 ms, (H2O)8/6-31G 1.40 and 1.55, 10 waters 1.76
+  // and 1.90, 12 2.59 and 2.55, 16 6.31 and 5.68; gradients: (H2O)4/STO-3G 0.92 and
+  // 1.18, (H2O)8/6-31G 6.11 and 6.06.
+  const int scan = P.npairs >= 65536 ? 8 : P.npairs >= (all_pairs ? 2048 : 4096) ? 4 : 1;
   TaskGenArgs g;
   g.nitems = ni;
   g.ncombo = ncombo;
