@@ -329,6 +329,7 @@ struct gbhf_ctx {
   gbhf::DBuf<double> boysh64;    // Horner tables for the J/K kernels
   gbhf::DBuf<float> boysh32;
   gbhf::DBuf<float4> boyshff;    // two-float Horner table
+  bool boys_ff_ready = false;    // it has been made
   // basis on device (function level, for 1-e integrals and canonical ERIs)
   gbhf::DBuf<double> d_xyz, d_Z, d_coef, d_exp;
   gbhf::DBuf<int> d_fn;          // per CGF: atom, lx, ly, lz, np, off (6 ints)

@@ -253,38 +253,53 @@ static BoysHostTables build_boys_host_tables() {
   return bt;
 }
 
-// The two-float Horner table (BOYSFF_*), built and uploaded when a basis first
-// uses it: small molecules never do.
-static std::vector<float> build_boys_ff_table() {
-  std::vector<float> hff((size_t)(BOYSH_LMAX + 1) * BOYSFF_NROW * BOYSFF_STRIDE, 0.0f);
-  for (int j = 0; j < BOYSFF_NROW; ++j) {
-    double f[BOYS_NCOL];
-    const double tj = (double)j * BOYSFF_H;
-    boys_row_host(tj, f);
-    for (int L = 0; L <= BOYSH_LMAX; ++L) {
-      float* row = hff.data() + ((size_t)L * BOYSFF_NROW + j) * BOYSFF_STRIDE;
-      auto split = [](double x, float* o) {
-        o[0] = (float)x;
-        o[1] = (float)(x - (double)o[0]);
-      };
-      double fact = 1.0;
-      for (int k = 0; k < 4; ++k) {
-        if (k > 0) fact *= k;
-        split(f[L + k] / fact, row + 2 * k);
-      }
-      row[8] = (float)(f[L + 4] / 24.0);
-      row[9] = (float)(f[L + 5] / 120.0);
-      split(std::exp(-tj), row + 10);
-    }
+// The two-float Horner table (BOYSFF_*), made when a basis of the context first uses
+// it (small molecules never do).  A thread per node: the series of boys_row_host in
+// FP64 (positive terms; the reciprocals of its odd denominators shared by the block)
+// and the downward recursion, 2^-50 where the kernels keep 2^-46.  (Made on the host it
+// took 33 of the 61 ms of a process's first build: long double is software there.)
+constexpr int BFF_THREADS = 128, BFF_TERMS = 256;
+__global__ void __launch_bounds__(BFF_THREADS) k_boys_ff(float* __restrict__ tab) {
+  constexpr int MT = BOYSH_LMAX + 5;   // highest order in a row
+  __shared__ double inv[BFF_TERMS];
+  for (int k = threadIdx.x; k < BFF_TERMS; k += BFF_THREADS) inv[k] = 1.0 / (2 * MT + 2 * k + 1);
+  __syncthreads();
+  const int j = blockIdx.x * BFF_THREADS + threadIdx.x;
+  if (j >= BOYSFF_NROW) return;
+  const double x = (double)j * BOYSFF_H, ex = exp(-x);
+  double term = inv[0], sum = term, f[MT + 1];
+  for (int k = 1; k < BFF_TERMS && term > 1e-18 * sum; ++k) {
+    term *= 2 * x * inv[k];
+    sum += term;
   }
-  return hff;
+  f[MT] = ex * sum;
+#pragma unroll
+  for (int m = MT - 1; m >= 0; --m) f[m] = (2 * x * f[m + 1] + ex) * (1.0 / (2 * m + 1));
+  auto split = [](double v, float* o) {
+    o[0] = (float)v;
+    o[1] = (float)(v - (double)o[0]);
+  };
+#pragma unroll
+  for (int L = 0; L <= BOYSH_LMAX; ++L) {
+    float* row = tab + ((size_t)L * BOYSFF_NROW + j) * BOYSFF_STRIDE;
+    split(f[L], row);
+    split(f[L + 1], row + 2);
+    split(f[L + 2] * (1.0 / 2), row + 4);
+    split(f[L + 3] * (1.0 / 6), row + 6);
+    row[8] = (float)(f[L + 4] * (1.0 / 24));
+    row[9] = (float)(f[L + 5] * (1.0 / 120));
+    split(ex, row + 10);
+  }
 }
 
 static gbhf_status ensure_boys_ff(gbhf_ctx* c) {
-  if (c->boyshff.p) return GBHF_OK;
-  static const std::vector<float> hff = build_boys_ff_table();   // once per process, thread-safe
-  GBHF_CUDA(c, c->boyshff.alloc(hff.size() / 4));
-  GBHF_CUDA(c, cudaMemcpyAsync(c->boyshff.p, hff.data(), hff.size() * sizeof(float), cudaMemcpyHostToDevice, c->stream));
+  if (c->boys_ff_ready) return GBHF_OK;
+  GBHF_CUDA(c, c->boyshff.alloc((size_t)(BOYSH_LMAX + 1) * BOYSFF_NROW * BOYSFF_STRIDE / 4));
+  k_boys_ff<<<(BOYSFF_NROW + BFF_THREADS - 1) / BFF_THREADS, BFF_THREADS, 0, c->stream>>>(
+      reinterpret_cast<float*>(c->boyshff.p));
+  count_launch(c);
+  GBHF_LAUNCHED(c, "k_boys_ff launch");
+  c->boys_ff_ready = true;
   return GBHF_OK;
 }
 
