@@ -139,6 +139,12 @@ struct DBuf {
   }
 };
 
+// Array inside a block that another buffer owns.
+template <typename T>
+struct DView {
+  T* p = nullptr;
+};
+
 struct Shell {
   int atom, L, np, ncomp, f0;   // f0: first basis function (components contiguous: x,y,z; xx,xy,xz,yy,yz,zz)
   int mol = 0;                  // molecule of the shell (batched SCF); 0 for one molecule
@@ -254,22 +260,23 @@ struct TaskLists {
   double thr_exact = 0;                // per-quartet density screening cutoff of the current build
   int ncombo = 0;
   int hranges[2 * NTIER * NCOMBO_MAX] = {0};   // host copy of ranges
-  DBuf<int> f0;                        // first basis function per shell
-  DBuf<double> sscale;                 // per shell: 6 component scales (d shells; 1 otherwise)
-  DBuf<float4> cen;                    // per shell: its centre in three FP32 parts (two-float kernels)
-  DBuf<int> nc;                        // components per shell
-  DBuf<int> atom;                      // atom of each shell
-  DBuf<int> smol;                      // molecule of each shell
-  DBuf<int> mn;                        // per molecule: functions
-  DBuf<long long> moff;                // per molecule: offset of its block in stacked matrices
-  DBuf<int> fmol;                      // per function: molecule
-  DBuf<int> amol;                      // per atom: molecule
-  DBuf<int> mfo, mao;                  // per molecule: first function, first atom (nmol+1)
+  DBuf<unsigned char> shell_block;     // the arrays below up to mao, ms0 and soff (ensure_shell_arrays)
+  DView<int> f0;                        // first basis function per shell
+  DView<double> sscale;                 // per shell: 6 component scales (d shells; 1 otherwise)
+  DView<float4> cen;                    // per shell: its centre in three FP32 parts (two-float kernels)
+  DView<int> nc;                        // components per shell
+  DView<int> atom;                      // atom of each shell
+  DView<int> smol;                      // molecule of each shell
+  DView<int> mn;                        // per molecule: functions
+  DView<long long> moff;                // per molecule: offset of its block in stacked matrices
+  DView<int> fmol;                      // per function: molecule
+  DView<int> amol;                      // per atom: molecule
+  DView<int> mfo, mao;                  // per molecule: first function, first atom (nmol+1)
   DBuf<double> row, pw, pb, sw;        // density weights (incremental builds, gradient)
   DBuf<float> Ds, pbf;                 // largest |D| per shell block and per pair (per-quartet screening)
   bool screened = false;               // they belong to the current build's density
-  DBuf<int> ms0;                       // per molecule: first shell (nmol+1)
-  DBuf<long long> soff;                // per molecule: offset of its ns_m x ns_m block in Ds
+  DView<int> ms0;                      // per molecule: first shell (nmol+1)
+  DView<long long> soff;               // per molecule: offset of its ns_m x ns_m block in Ds
   size_t ds_size = 0;
   long f0_gen = -1;                    // basis generation f0 was uploaded for
 };
@@ -371,9 +378,9 @@ struct gbhf_ctx {
   std::map<std::string, std::vector<double>> sad_cache;
   gbhf_ctx* sad_ctx = nullptr;
   gbhf::DBuf<float> dfloat;
-  gbhf::DBuf<gbhf::ff> dff;         // density of the two-float kernels, scaled by 2^-e
+  gbhf::DBuf<gbhf::ff> dff;         // density of the two-float kernels, scaled by 2^-e (and gff behind it)
   gbhf::DBuf<int> dff_exp;          // e
-  gbhf::DBuf<double> gff;           // the two-float launches' accumulator of a J/K build
+  gbhf::DView<double> gff;          // the two-float launches' accumulator of a J/K build
   gbhf::DBuf<int> dev_status;
   int purify_grid = 0;              // co-resident blocks of the fused purification kernel
   int tc2_per_sm = 0;               // blocks per SM of the one-barrier TC2 kernel (0: not asked yet)
