@@ -9,6 +9,7 @@
 
 #include "../../include/gbhf.h"
 #include "gbhf_common.cuh"
+#include "side_fork.h"
 
 namespace gbhf {
 

@@ -49,12 +49,9 @@ gbhf_status grad_2e(gbhf_ctx* c, const double* d_D, double schwarz, double mixed
       nts[k][t] = gt.hranges[2 * (NTIER * k + t) + 1] - gt.hranges[2 * (NTIER * k + t)];
   const bool ev = c->prof.events;
   int ne = 0, ev_combo[NTIER * NCOMBO_MAX], ev_prec[NTIER * NCOMBO_MAX];
-  if (ev) {
-    GBHF_CUDA(c, cudaEventRecord(c->evg[0], c->stream));
-  } else {
-    GBHF_CUDA(c, cudaEventRecord(c->fork_ev, c->stream));
-    for (int i = 0; i < gbhf_ctx::NSIDE_GRAD; ++i) GBHF_CUDA(c, cudaStreamWaitEvent(c->side[i], c->fork_ev, 0));
-  }
+  SideFork side(c->stream, c->fork_ev, c->side, c->join_ev, gbhf_ctx::NSIDE_GRAD);
+  if (ev) GBHF_CUDA(c, cudaEventRecord(c->evg[0], c->stream));
+  else GBHF_CUDA(c, side.fork());
   int nl = 0;
   // heaviest first: the d combinations, then the s/p ones
   static const int order[NCOMBO_MAX] = {35, 34, 29, 33, 28, 23, 32, 27, 22, 17, 31, 26, 21, 16, 11, 30, 25, 20,
@@ -79,10 +76,7 @@ gbhf_status grad_2e(gbhf_ctx* c, const double* d_D, double schwarz, double mixed
     }
   }
   if (!ev) {
-    for (int i = 0; i < gbhf_ctx::NSIDE_GRAD; ++i) {
-      GBHF_CUDA(c, cudaEventRecord(c->join_ev[i], c->side[i]));
-      GBHF_CUDA(c, cudaStreamWaitEvent(c->stream, c->join_ev[i], 0));
-    }
+    GBHF_CUDA(c, side.join());
     return GBHF_OK;
   }
   GBHF_CUDA(c, cudaEventSynchronize(c->evg[ne]));
@@ -444,31 +438,20 @@ gbhf_status gradient_dev(gbhf_ctx* c, const double* d_D, const double* d_W, doub
   static_assert(NS >= 1, "side streams for the one-electron terms");
   const bool beside = !c->prof.events;
   auto strm = [&](int k) { return beside ? c->side[S0 + k % NS] : c->stream; };
-  if (beside) {
-    GBHF_CUDA(c, cudaEventRecord(c->fork_ev, c->stream));
-    for (int k = 0; k < NS; ++k) GBHF_CUDA(c, cudaStreamWaitEvent(c->side[S0 + k], c->fork_ev, 0));
-  }
-  auto run = [&]() -> gbhf_status {
-    constexpr int PB = G1_THREADS / G1_LANES;
-    k_grad_1e<<<dim3((max_fn + PB - 1) / PB, n), G1_THREADS, 0, strm(0)>>>(g1);
-    count_launch(c, 2);
-    GBHF_CUDA(c, cudaGetLastError());
-    GBHF_TRY((launch_vne<2, 2>(c, strm(1), 5, d_D, d_grad)));
-    GBHF_TRY((launch_vne<1, 1>(c, strm(2), 2, d_D, d_grad)));
-    GBHF_TRY((launch_vne<1, 0>(c, strm(3), 1, d_D, d_grad)));
-    GBHF_TRY((launch_vne<2, 1>(c, strm(2), 4, d_D, d_grad)));
-    GBHF_TRY((launch_vne<2, 0>(c, strm(3), 3, d_D, d_grad)));
-    GBHF_TRY((launch_vne<0, 0>(c, strm(0), 0, d_D, d_grad)));
-    return grad_2e(c, d_D, schwarz, mixed_cutoff, precision, d_grad);
-  };
-  const gbhf_status st = run();
-  // the side streams' work ends before d_grad and the densities are the caller's again, also on an error
-  if (beside)
-    for (int k = 0; k < NS; ++k) {
-      const cudaError_t e = cudaStreamSynchronize(c->side[S0 + k]);
-      if (st == GBHF_OK) GBHF_CUDA(c, e);
-    }
-  GBHF_TRY(st);
+  SideFork side(c->stream, c->fork_ev, c->side + S0, c->join_ev + S0, NS);
+  if (beside) GBHF_CUDA(c, side.fork());
+  constexpr int PB = G1_THREADS / G1_LANES;
+  k_grad_1e<<<dim3((max_fn + PB - 1) / PB, n), G1_THREADS, 0, strm(0)>>>(g1);
+  count_launch(c, 2);
+  GBHF_CUDA(c, cudaGetLastError());
+  GBHF_TRY((launch_vne<2, 2>(c, strm(1), 5, d_D, d_grad)));
+  GBHF_TRY((launch_vne<1, 1>(c, strm(2), 2, d_D, d_grad)));
+  GBHF_TRY((launch_vne<1, 0>(c, strm(3), 1, d_D, d_grad)));
+  GBHF_TRY((launch_vne<2, 1>(c, strm(2), 4, d_D, d_grad)));
+  GBHF_TRY((launch_vne<2, 0>(c, strm(3), 3, d_D, d_grad)));
+  GBHF_TRY((launch_vne<0, 0>(c, strm(0), 0, d_D, d_grad)));
+  GBHF_TRY(grad_2e(c, d_D, schwarz, mixed_cutoff, precision, d_grad));
+  if (beside) GBHF_CUDA(c, side.join());
   GBHF_CUDA(c, cudaStreamSynchronize(c->stream));
   return GBHF_OK;
 }

@@ -814,11 +814,9 @@ gbhf_status jk_build(gbhf_ctx* c, const double* d_Dsq, double* d_G, int precisio
   bool two_float = false;
   int ne = 0, nl = 0;
   int ev_combo[NTIER * NCOMBO], ev_prec[NTIER * NCOMBO];
+  SideFork side(c->stream, c->fork_ev, c->side, c->join_ev, gbhf_ctx::NSIDE);
   if (ev) GBHF_CUDA(c, cudaEventRecord(c->evc[ne], c->stream));
-  else {
-    GBHF_CUDA(c, cudaEventRecord(c->fork_ev, c->stream));
-    for (int i = 0; i < gbhf_ctx::NSIDE; ++i) GBHF_CUDA(c, cudaStreamWaitEvent(c->side[i], c->fork_ev, 0));
-  }
+  else GBHF_CUDA(c, side.fork());
   for (const int tier : tiers) {
     for (int oi = 0; oi < NCOMBO; ++oi) {
       const int k = order[oi];
@@ -839,12 +837,7 @@ gbhf_status jk_build(gbhf_ctx* c, const double* d_Dsq, double* d_G, int precisio
       }
     }
   }
-  if (!ev) {
-    for (int i = 0; i < gbhf_ctx::NSIDE; ++i) {
-      GBHF_CUDA(c, cudaEventRecord(c->join_ev[i], c->side[i]));
-      GBHF_CUDA(c, cudaStreamWaitEvent(c->stream, c->join_ev[i], 0));
-    }
-  }
+  if (!ev) GBHF_CUDA(c, side.join());
   if (d_Gff) *d_Gff = two_float ? c->gff.p : nullptr;
   else if (two_float) GBHF_TRY(axpby(c, (size_t)c->basis.stacked, 1.0, d_G, 1.0, c->gff.p, d_G));
   // statistics: read with the per-class event times when those are taken,
