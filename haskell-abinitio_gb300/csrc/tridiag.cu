@@ -47,6 +47,12 @@ __device__ __forceinline__ int scale_exponent(double amax) {
   const int x = ilogb(amax);
   return x < -400 || x > 400 ? x : 0;
 }
+// What decides whether the largest element is looked for at all: bit 0 an element of at
+// least 2^-400, bit 1 one above 2^400 (no reduction of values in the common case, 5 us
+// of a 7 x 7 solve).
+__device__ __forceinline__ int range_bits(double a) {
+  return (fabs(a) >= 0x1p-400 ? 1 : 0) | (fabs(a) > 0x1p400 ? 2 : 0);
+}
 
 // One CTA of 1024 threads.  Shared memory: packed lower triangle of A
 // (n(n+1)/2), v (n), p / w (n).  Outputs: d (n), e (n - 1), tau (n), Vt (row k:
@@ -60,22 +66,27 @@ __global__ void __launch_bounds__(1024) k_sytrd(int n, const double* __restrict_
   double* sp = sv + n;
   __shared__ double s_bc[4];
   const int tid = threadIdx.x, nt = blockDim.x;
-  double amax = 0.0;
+  int bits = 0;
   for (long q = tid; q < (long)n * n; q += nt) {
     const int i = (int)(q / n), j = (int)(q % n);
     if (j <= i) {
       P[pidx(i, j)] = A[q];
-      amax = fmax(amax, fabs(A[q]));
+      bits |= range_bits(A[q]);
     }
   }
-  amax = block_reduce(amax, true);
-  if (tid == 0) s_bc[0] = amax;
-  __syncthreads();
-  const int sx = scale_exponent(s_bc[0]);
-  if (tid == 0) scal[3] = sx;
-  if (sx)
+  const bool some = __syncthreads_or(bits & 1), large = __syncthreads_or(bits & 2);
+  int sx = 0;
+  if (!some || large) {
+    double amax = 0.0;
+    for (int q = tid; q < (int)pidx(n, 0); q += nt) amax = fmax(amax, fabs(P[q]));
+    amax = block_reduce(amax, true);
+    if (tid == 0) s_bc[0] = amax;
+    __syncthreads();
+    sx = scale_exponent(s_bc[0]);
     for (int q = tid; q < (int)pidx(n, 0); q += nt) P[q] = scalbn(P[q], -sx);
-  __syncthreads();
+    __syncthreads();
+  }
+  if (tid == 0) scal[3] = sx;
   for (int k = 0; k + 2 < n; ++k) {
     const int m = n - 1 - k;   // trailing size, >= 2
     // Householder vector of column k below the diagonal
@@ -211,6 +222,7 @@ __global__ void __launch_bounds__(SY_THREADS)
   cg::cluster_group cluster = cg::this_cluster();
   extern __shared__ double sm[];
   __shared__ double s_bc[3], s_amax;
+  __shared__ int s_bits;
   const int r = (int)cluster.block_rank(), tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int nq = n > r ? (n - r + CS - 1) / CS : 0;   // rows owned: r + CS q
   const int ld = sy_ld(n);
@@ -221,28 +233,36 @@ __global__ void __launch_bounds__(SY_THREADS)
   double* vp = v + n;       // the last step's v and w
   double* wp = vp + n;
   double* P = wp + n;       // owned rows
-  double amax = 0.0;
+  int bits = 0;
   for (int q = warp; q < nq; q += SY_WARPS)
     for (int j = lane; j < n; j += 32) {   // the lower triangle is what counts
       const int i = r + CS * q;
       const double a = j <= i ? A[(long)i * n + j] : A[(long)j * n + i];
       P[q * ld + j] = a;
-      amax = fmax(amax, fabs(a));
+      bits |= range_bits(a);
     }
   for (int i = tid; i < n; i += SY_THREADS) vp[i] = wp[i] = 0.0;
-  amax = block_reduce(amax, true);
-  if (tid == 0) s_amax = amax;
+  bits = (__syncthreads_or(bits & 1) ? 1 : 0) | (__syncthreads_or(bits & 2) ? 2 : 0);
+  if (tid == 0) s_bits = bits;
   cluster.sync();
-  amax = lane < CS ? *cluster.map_shared_rank(&s_amax, lane) : 0.0;
+  bits = lane < CS ? *cluster.map_shared_rank(&s_bits, lane) : 0;
+  int sx = 0;
+  if (!__any_sync(0xffffffffu, bits & 1) || __any_sync(0xffffffffu, bits & 2)) {   // by every thread of the cluster
+    double amax = 0.0;
+    for (int q = warp; q < nq; q += SY_WARPS)
+      for (int j = lane; j < n; j += 32) amax = fmax(amax, fabs(P[q * ld + j]));
+    amax = block_reduce(amax, true);
+    if (tid == 0) s_amax = amax;
+    cluster.sync();
+    amax = lane < CS ? *cluster.map_shared_rank(&s_amax, lane) : 0.0;
 #pragma unroll
-  for (int o = 16; o > 0; o >>= 1) amax = fmax(amax, __shfl_xor_sync(0xffffffffu, amax, o));
-  const int sx = scale_exponent(amax);   // the same in every thread of the cluster
-  if (r == 0 && tid == 0) scal[3] = sx;
-  if (sx) {
+    for (int o = 16; o > 0; o >>= 1) amax = fmax(amax, __shfl_xor_sync(0xffffffffu, amax, o));
+    sx = scale_exponent(amax);
     for (int q = warp; q < nq; q += SY_WARPS)
       for (int j = lane; j < n; j += 32) P[q * ld + j] = scalbn(P[q * ld + j], -sx);
     __syncthreads();
   }
+  if (r == 0 && tid == 0) scal[3] = sx;
   for (int k = 0; k + 2 < n; ++k) {
     const int q0 = k >= r ? (k - r) / CS + 1 : 0;   // first own row > k
     // A: column k of own rows > k, to every CTA
