@@ -294,12 +294,13 @@ __global__ void __launch_bounds__(GR_THREADS) k_grad_jk(GradArgs<T> a) {
     // the screened kets in full batches, as in k_jk ((H2O)8 FP64 gradient 11.3 -> 10.0 ms)
     if constexpr (QUEUE) {
       const BraScreen bs(a.scr, ib, pab, mol);
+      const OneCentre one(a.shell_atom, pab);
       int queued = 0, scanned = 0;
       while (true) {
         while (queued < 32 && scanned < task.z) {
           const int o = scanned + lane;
           const int jk = task.y + o;
-          const bool pass = o < task.z && bs.gamma_pass(a.scr, jk, a.jabs);
+          const bool pass = o < task.z && bs.gamma_pass(a.scr, jk, a.jabs, one, a.shell_atom);
           queue_push(sq[warp], queued, jk, pass, lane);
           scanned += 32;
         }
@@ -317,8 +318,10 @@ __global__ void __launch_bounds__(GR_THREADS) k_grad_jk(GradArgs<T> a) {
       const int lg = 32 - __clz(max(nk, 1) - 1);
       const bool active = (lane & ((1 << lg) - 1)) < nk;
       const int jk = active ? task.y + (lane & ((1 << lg) - 1)) : task.y;
-      grad_batch<LA, LB, LC, LD, T, GamT, TkT>(a, gam, tk, sbra[warp], sDab[warp], ib, pab, jk, a.scr.pinfo[jk], active, lg,
-                                               lane, Kb, sg, n, Dm, thrs, dex);
+      const int4 pcd = a.scr.pinfo[jk];
+      const bool own = active && !OneCentre(a.shell_atom, pab).holds(a.shell_atom, pcd);
+      grad_batch<LA, LB, LC, LD, T, GamT, TkT>(a, gam, tk, sbra[warp], sDab[warp], ib, pab, jk, pcd, own, lg, lane, Kb, sg,
+                                               n, Dm, thrs, dex);
       __syncwarp();
     }
   }
@@ -371,10 +374,11 @@ __global__ void __launch_bounds__(TH) k_grad_jk_step(GradArgs<T> a) {
       if (scanned < task.z) {
         const int ib = task.x;
         const BraScreen bs(a.scr, ib, a.scr.pinfo[ib], a.pmol[ib]);
+        const OneCentre one(a.shell_atom, a.scr.pinfo[ib]);
         while (queued < 32 && scanned < task.z) {
           const int o = scanned + lane;
           const int jk = task.y + o;
-          const bool pass = o < task.z && bs.gamma_pass(a.scr, jk, a.jabs);
+          const bool pass = o < task.z && bs.gamma_pass(a.scr, jk, a.jabs, one, a.shell_atom);
           queue_push(sq[warp], queued, jk, pass, lane);
           scanned += 32;
         }

@@ -15,6 +15,7 @@
 
 #include "gbhf_internal.h"
 #include "mdwarp.cuh"
+#include "screen.cuh"
 
 namespace gbhf {
 
@@ -90,10 +91,12 @@ __global__ void __launch_bounds__(GRD_THREADS) k_gradd(GradDArgs<T> a) {
     }
     const int A = a.pA[ib], B = a.pB[ib];
     const int a0 = a.shell_f0[A], b0 = a.shell_f0[B];
+    const OneCentre one(a.shell_atom, make_int4(A, B, 0, 0));
     T g[6] = {T(0), T(0), T(0), T(0), T(0), T(0)};
     for (int q = 0; q < task.z; ++q) {
       const int jk = task.y + q;
       const int Cs = a.pA[jk], Ds = a.pB[jk];
+      if (one.holds(a.shell_atom, make_int4(Cs, Ds, 0, 0))) continue;   // warp-uniform
       const int c0 = a.shell_f0[Cs], d0 = a.shell_f0[Ds];
       const S wgt = (A == B ? S(1) : S(2)) * (Cs == Ds ? S(1) : S(2));
       S gmax = S(0);

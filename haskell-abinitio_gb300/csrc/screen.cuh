@@ -33,6 +33,20 @@ inline QuartetScreen quartet_screen(const gbhf_ctx* c, double thr) {
           c->tasks.ms0.p,   c->tasks.soff.p, (float)(thr * (1.0 - 3e-7))};
 }
 
+// The gradient leaves out the quartets with all four shells on one atom: their four
+// derivatives add up to zero there (translational invariance), in floating point to the
+// rounding of terms that are the largest of all for steep shells.
+struct OneCentre {
+  int at;   // the atom of both bra shells, else -1
+  __device__ __forceinline__ OneCentre(const int* __restrict__ shell_atom, int4 pab) {
+    const int a = shell_atom[pab.x];
+    at = a == shell_atom[pab.y] ? a : -1;
+  }
+  __device__ __forceinline__ bool holds(const int* __restrict__ shell_atom, int4 pcd) const {
+    return at >= 0 && shell_atom[pcd.x] == at && shell_atom[pcd.y] == at;
+  }
+};
+
 // The bra's part of the bound.
 struct BraScreen {
   float q, dab;
@@ -56,9 +70,11 @@ struct BraScreen {
     return !(q * s.Qf[jk] * d < s.thr);
   }
   // Q_ab Q_cd times a bound of |Gamma| = |jcoef D_ab D_cd - (D_ac D_bd + D_ad D_bc) / 4|
-  __device__ __forceinline__ bool gamma_pass(const QuartetScreen& s, int jk, float jcoef) const {
-    if (!s.Ds) return true;
+  __device__ __forceinline__ bool gamma_pass(const QuartetScreen& s, int jk, float jcoef, const OneCentre& one,
+                                             const int* __restrict__ shell_atom) const {
     const int4 p = s.pinfo[jk];
+    if (one.holds(shell_atom, p)) return false;
+    if (!s.Ds) return true;
     const float g = fabsf(jcoef) * dab * s.pbf[jk] + 0.25f * (ra[p.x] * rb[p.y] + ra[p.y] * rb[p.x]);
     return !(q * s.Qf[jk] * g * 1.000001f < s.thr);
   }

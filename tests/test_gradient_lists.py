@@ -88,3 +88,23 @@ def test_gradient_of_densities_outside_the_fp32_range(ctx, open_shell):
     nuc = ctx.gradient(zero, zero)
     one, far = two_electron(1.0) - nuc, two_electron(2.0 ** 200)
     np.testing.assert_allclose(far, one, rtol=0, atol=1e-12 * np.abs(one).max())
+
+
+@pytest.mark.parametrize("waters,basis,before", [(2, "6-31g", 1.1e-13), (4, "sto-3g", 6.9e-13), (2, "6-31g*", 1.1e-13)])
+def test_translational_invariance_to_rounding(ctx, waters, basis, before):
+    """The gradient adds up to zero over the atoms.  The quartets on one atom add
+    nothing but the rounding of their terms; with them the sum was `before` (rms over
+    densities and directions), without them it stays below two thirds of it."""
+    xyz = M.water_cluster(waters, np.random.default_rng(waters))
+    fb = B.flatten(B.make_atoms(M.water_labels(waters), xyz, basis))
+    ctx.set_basis(fb)
+    pos = fb.xyz[fb.cgf_atom]
+    r = np.linalg.norm(pos[:, None] - pos[None], axis=2)
+
+    def density(seed):
+        rng = np.random.default_rng(seed)
+        d = rng.standard_normal((fb.n_cgf, fb.n_cgf)) * 0.15
+        return O.square_to_tri((d + d.T) * np.exp(-r / 1.6) + np.diag(rng.uniform(0.3, 2.0, fb.n_cgf)))
+
+    sums = [ctx.gradient(density(s), 0.2 * density(s + 10), schwarz=0.0).sum(axis=0) for s in (1, 2, 3) for _ in range(4)]
+    assert np.sqrt(np.mean(np.square(sums))) < 2.0 / 3.0 * before
