@@ -249,7 +249,7 @@ __global__ void __launch_bounds__(GR_THREADS) k_grad_jk(GradArgs<T> a) {
   constexpr int NAB = NA * NB, NOUT = NAB * NC * ND;
   __shared__ __align__(16) T sbra[GR_WARPS][KMAX_PRIM_PAIRS * BRA_SB];
   __shared__ T sDab[GR_WARPS][NAB];
-  __shared__ int sq[QUEUE ? GR_WARPS : 1][64];
+  __shared__ int sq[QUEUE ? GR_WARPS : 1][QUEUE_SLOTS];
   extern __shared__ double gsm_dyn[];
   constexpr int NT = NAB * nherm_c(LC + LD);
   using GamT = typename std::conditional<SG, GamSmem<T, NOUT, GR_THREADS>, GamReg<T, NOUT>>::type;
@@ -307,8 +307,9 @@ __global__ void __launch_bounds__(GR_THREADS) k_grad_jk(GradArgs<T> a) {
         if (queued == 0) break;
         const int nk = min(queued, 32);
         const int lg = 32 - __clz(nk - 1);
-        const bool active = (lane & ((1 << lg) - 1)) < nk;
-        const int jk = active ? sq[warp][lane & ((1 << lg) - 1)] : task.y;
+        bool active, bad;
+        const int jk = queue_ket(sq[warp], nk, lg, lane, task.y, task.z, active, bad);
+        if (bad) a.grad[0] = nan("");
         grad_batch<LA, LB, LC, LD, T, GamT, TkT>(a, gam, tk, sbra[warp], sDab[warp], ib, pab, jk, a.scr.pinfo[jk], active,
                                                  lg, lane, Kb, sg, n, Dm, thrs, dex);
         queue_pop(sq[warp], queued, nk, lane);
@@ -344,7 +345,7 @@ __global__ void __launch_bounds__(TH) k_grad_jk_step(GradArgs<T> a) {
   constexpr int NAB = NA * NB, NOUT = NAB * NC * ND, W = TH / 32;
   __shared__ __align__(16) T sbra[W][KMAX_PRIM_PAIRS * BRA_SB];
   __shared__ T sDab[W][NAB];
-  __shared__ int sq[W][64];
+  __shared__ int sq[W][QUEUE_SLOTS];
   extern __shared__ double gsm_dyn[];
   constexpr int NT = NAB * nherm_c(LC + LD);
   using GamT = typename std::conditional<SG, GamSmem<T, NOUT, TH>, GamReg<T, NOUT>>::type;
@@ -411,8 +412,9 @@ __global__ void __launch_bounds__(TH) k_grad_jk_step(GradArgs<T> a) {
       const int ib = task.x, mol = a.pmol[ib];
       const int nk = min(queued, 32);
       const int lg = 32 - __clz(nk - 1);
-      const bool active = (lane & ((1 << lg) - 1)) < nk;
-      const int jk = active ? sq[warp][lane & ((1 << lg) - 1)] : task.y;
+      bool active, bad;
+      const int jk = queue_ket(sq[warp], nk, lg, lane, task.y, task.z, active, bad);
+      if (bad) a.grad[0] = nan("");
       grad_batch<LA, LB, LC, LD, T, GamT, TkT, true>(a, gam, tk, sbra[warp], sDab[warp], ib, a.scr.pinfo[ib], jk,
                                                      a.scr.pinfo[jk], active, lg, lane,
                                                      (task.w >> 16) - (task.w & 0xffff), a.seg[a.kseg[task.y]],

@@ -14,6 +14,7 @@
 // maxima, and where those meet a zero block (NaN) the quartet is kept as well.
 #pragma once
 #include "gbhf_internal.h"
+#include "warp_queue.cuh"
 
 namespace gbhf {
 
@@ -79,22 +80,5 @@ struct BraScreen {
     return !(q * s.Qf[jk] * g * 1.000001f < s.thr);
   }
 };
-
-// Append the lanes' kets that pass to the warp's queue (at most 31 queued before).
-__device__ __forceinline__ void queue_push(int* q, int& queued, int jk, bool pass, int lane) {
-  const unsigned m = __ballot_sync(0xffffffffu, pass);
-  if (pass) q[queued + __popc(m & ((1u << lane) - 1))] = jk;
-  queued += __popc(m);
-  __syncwarp();
-}
-// Remove the first nk (at most 31 are left).
-__device__ __forceinline__ void queue_pop(int* q, int& queued, int nk, int lane) {
-  queued -= nk;
-  __syncwarp();
-  const int v = lane < queued ? q[nk + lane] : 0;
-  __syncwarp();
-  if (lane < queued) q[lane] = v;
-  __syncwarp();
-}
 
 }  // namespace gbhf

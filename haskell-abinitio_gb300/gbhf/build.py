@@ -22,7 +22,7 @@ SOURCES = ["jk.cu", "grad_ff.cu", "jk_ff.cu", "grad.cu", "jkd.cu", "gradd.cu", "
            "tune.cu", "tridiag.cu", "small_dense.cu"]
 HEADERS = ["gbhf_common.cuh", "gbhf_ff.cuh", "gbhf_internal.h", "gbhf_md.cuh", "eri_gen.cuh", "grad_gen.cuh", "jacobi.cuh",
            "dense.cuh", "mdwarp.cuh", "jk_kern.cuh",
-           "grad_kern.cuh", "screen.cuh", "side_fork.h"]
+           "grad_kern.cuh", "screen.cuh", "side_fork.h", "warp_queue.cuh"]
 
 
 def nvcc():
