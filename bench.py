@@ -397,8 +397,8 @@ def run_gbhf(args, world, rank, local):
     red = sum(v.get("l2_red_sectors_per_launch", 0.0) for v in tr_all.values()) * 32
     line["fock_scatter"] = {"algorithmic_bytes_per_build": 24 * n * n,
                             "l2_reduction_bytes_per_full_build": red or None, "dram_write_bytes_per_full_build": 0,
-                            "source": "ncu lts__t_sectors_srcunit_tex_op_red.sum x 32 B over the twelve class launches "
-                                      "of one full mixed build (profiles/traffic.json, profiles/k_jk_w16_fock_full.md): "
+                            "source": "ncu lts__t_sectors_srcunit_tex_op_red.sum x 32 B over the class launches "
+                                      "of one full mixed build (profiles/traffic.json): "
                                       "every quartet adds its J/K terms with FP64 reductions in L2; none reach DRAM"}
     peaks = load_measured_peaks()
     if peaks:
@@ -487,6 +487,7 @@ def batch_measure(args, world, rank, local, mixed_cutoff, grad_cutoff, quick=Fal
             "max_abs_grad_mixed_vs_fp64_sample": float(max(dg)) if dg else None,
             "meets_1e-6_eh_and_1e-5_eh_per_bohr": bool(de and max(de) <= 1e-6 and max(dg) <= 1e-5),
             "mixed_cutoff": mixed_cutoff, "grad_mixed_cutoff": grad_cutoff,
+            "grad_fp32_below": min(grad_cutoff or mixed_cutoff, 0.125),
             "sample": f"FP64 one-at-a-time SCF + gradient timed on {len(sample)} of {len(sub)} molecules "
                       "(every 8th) and scaled; dE and gradient errors on the same sample",
             "batch_steps": int(prof["batch_steps"]), "gpu_launches": int(prof["launches"]), "autotune": tune,

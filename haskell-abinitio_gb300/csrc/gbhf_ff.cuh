@@ -5,7 +5,7 @@
 // and cycle), so one FP64 fused multiply-add costs the issue slots of 64 FP32
 // instructions; the two-float one takes 12.  The kernels use it for the
 // quartets whose Schwarz bound makes its absolute error smaller than the error
-// that the build has anyway (ff_limit in jk.cu says which).
+// that the build has anyway (ff_limits in setup.cu says which).
 //
 // Rules of the representation: a sum keeps the exact rounding error of the
 // heads (Knuth's two-sum, D. E. Knuth, TAOCP vol. 2, 4.2.2) and a product that

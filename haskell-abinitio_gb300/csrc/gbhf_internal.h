@@ -306,7 +306,8 @@ struct TridiagWork {
 // Largest n of the tridiagonal path: the packed lower triangle of A plus two
 // vectors in one CTA's shared memory (232: 215 KiB).
 constexpr int TRIDIAG_MAX_N = 232;
-// With the rows in the shared memory of a 16-CTA cluster (608: 222 KiB each).
+// With the rows in the shared memory of a 16-CTA cluster: 38 rows and 204.5 KiB a CTA
+// at 608 (40 rows at 640, 225.3 KiB, would still fit; not measured).
 constexpr int TRIDIAG_WIDE_MAX_N = 608;
 
 struct Profile {

@@ -10,15 +10,19 @@
 // and G = G'' + G''^T equals J - K/2 of the reference's calcGmatrix
 // (HartreeFock/HartreeFock.hs:225-241): G_ab = sum_kl D_lk [(ab|kl) - (al|kb)/2].
 //
-// Work decomposition: a task is (bra pair, <= 32 consecutive kets of one ket
-// segment); one warp runs one task, lane = ket.  Kets inside a segment share
+// Work decomposition: a task is (bra pair, consecutive kets of one ket segment,
+// a range of bra primitives); one warp runs one task.  An s/p task holds up to
+// 32, 128 or 256 kets: the warp screens them by the density and evaluates the
+// survivors 32 at a time, lane = ket (screen.cuh); a d task holds at most 32, or
+// one where a warp evaluates one quartet (jkd.cu).  Kets inside a segment share
 // the primitive-pair count, so lanes do equal work; the segment is sorted by
 // Schwarz bound, so the kets that pass Q_bra Q_ket w >= cutoff form a prefix
 // found by binary search, and the split between the precision tiers (FP64,
 // two-float, FP32 in mixed precision) is two more prefix boundaries.  Two-float
 // tier (gbhf_ff.cuh): full FP64 build of (H2O)16/6-31G 26.1 -> 8.0 ms, mixed one
-// of (H2O)64 144 -> 88 ms (FP64 launches 75 ms, FP64 + two-float 21 ms).  Warps pull tasks from a per-kernel atomic counter
-// (no waiting on other warps).
+// of (H2O)64 144 -> 88 ms (FP64 launches 75 ms, FP64 + two-float 21 ms).  Warps
+// pull tasks from a per-kernel atomic counter; only the blocks of the two in-step
+// kernels wait, for their own warps (block_tick).
 #include <algorithm>
 #include <cstring>
 #include <functional>

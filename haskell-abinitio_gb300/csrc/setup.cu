@@ -428,10 +428,13 @@ __global__ void k_pair_layouts(int np, const int* __restrict__ pA, const int* __
 // floats also where FP64 is asked for: 2^-5 of the molecule's largest.  There the
 // two-float error, 2^-45 of the quartet, is 2^-50 of the largest quartet, the size
 // of the FP64 rounding (2^-53 a term) and Boys remainder (5e-15) of the large
-// ones that stay in FP64.  0 (never) below 512 primitive pairs, where a build is
-// a handful of tasks and the extra launches cost more than the arithmetic saves
-// (SCF + gradient of a water, 250 pairs: 11.0 -> 11.5 ms with the two-float
-// lists; the dimer's Fock build, 1000 pairs: 377 -> 188 us), and when an exponent, a coefficient or a
+// ones that stay in FP64; measured, the FP64 Fock matrix and gradient are closer to
+// their exact values than by FP64 lists alone (jk_build, OneCentre).  0 (never) below
+// 512 primitive pairs, where a build is a handful of tasks and the extra launches cost
+// more than the arithmetic saves (SCF + gradient of a water, 250 pairs: 11.0 -> 11.5 ms
+// with the two-float lists; the dimer's Fock build, 1000 pairs: 377 -> 188 us repeated,
+// 1.08 -> 0.91 ms with the pair set-up of a new geometry, 1.33 -> 1.30 ms with a new
+// context), and when an exponent, a coefficient or a
 // coordinate is far outside what FP32 exponents hold.  k_pair_layouts then checks what
 // each primitive pair brings into the products (ff_pair_range).
 static std::vector<FFLimit> ff_limits(const Basis& b, const PairData& P) {

@@ -466,7 +466,8 @@ __global__ void __launch_bounds__(256) k_tri_prep(int n, const double* __restric
 
 // 1/q to about an ulp with three FP64 instructions: the single-precision
 // estimate of the truncated q (exponents moved with integer operations), then
-// r0 (1 + h + h^2), h = 1 - q r0 (the neglected h^3 is below 2^-63); outside the
+// r0 (1 + h + h^2), h = 1 - q r0: |h| <= 2^-20 + 2^-23 (the estimate sees q's high
+// word), so the neglected h^3 is below 2^-59; outside the
 // single-precision range the plain quotient.
 __device__ __forceinline__ double recip_nr(double q) {
   const int hi = __double2hiint(q), ahi = hi & 0x7fffffff;

@@ -51,9 +51,13 @@ typedef enum {
 } gbhf_mode;
 
 typedef enum {
-  GBHF_PREC_FP64 = 0,  /* every ERI in FP64 */
-  GBHF_PREC_MIXED = 1  /* ERIs with Schwarz bound below mixed_cutoff in FP32; Fock accumulation,
-                          DIIS and the eigen-solve always FP64 */
+  /* Fock accumulation, DIIS and the eigen-solve are FP64 in both. */
+  GBHF_PREC_FP64 = 0,  /* ERIs in FP64; those whose Schwarz product is below 2^-5 of the molecule's largest
+                          as pairs of FP32 numbers (2^-46 an operation), in molecules of 512 primitive
+                          pairs or more whose primitives FP32 exponents hold.  The Fock matrix and the
+                          gradient are as close to their exact values as by FP64 arithmetic alone */
+  GBHF_PREC_MIXED = 1  /* ERIs with Schwarz bound below mixed_cutoff in FP32, up to 2^18 times that as
+                          pairs of FP32 numbers, the others as GBHF_PREC_FP64 */
 } gbhf_precision;
 
 /* GBHF_GUESS_SAD (superposition of atomic densities: block-diagonal densities of
@@ -85,7 +89,9 @@ typedef struct {
   double mixed_cutoff;   /* FP32 for quartets with bound below this (baseline 1e-4) */
   double charge;         /* total charge; n_occ = floor((sum Z - charge)/2) (HartreeFock.hs:75-76) */
   double grad_mixed_cutoff; /* gbhf_scf_batch gradients, mixed precision: FP32 derivative integrals for
-                               quartets with bound Q_ab Q_cd max(w)^2 below this (0: mixed_cutoff) */
+                               quartets with bound Q_ab Q_cd max(w)^2 below this (0: mixed_cutoff), at
+                               most 1/8: above it FP32 pairs take over (gradients were 1e-6 from
+                               translational invariance at 1, 1e-7 so) */
   int autotune;          /* 1: unless this context already holds tuned task budgets, run gbhf_autotune
                             on the call's basis before the first step (J/K, with the starting density)
                             and, in gbhf_scf_batch, before the gradients (with their density) */
@@ -107,7 +113,7 @@ typedef struct {
   double eri_quartets;       /* contracted shell quartets computed, summed over builds */
   double eri_fn_quartets;    /* contracted basis-function quartets computed, summed over builds */
   double eri_prim_quartets;  /* primitive quartets computed, summed over builds */
-  double eri_fp32_fraction;  /* share of primitive quartets evaluated in FP32 */
+  double eri_fp32_fraction;  /* share of primitive quartets evaluated in FP32 (pairs of FP32 numbers count as FP64) */
   double fock_builds;
 } gbhf_result;
 
@@ -286,7 +292,9 @@ gbhf_status gbhf_scf_batch(gbhf_ctx* ctx, int n_mol, const int* atom_off, const 
 /* Task budgets of the direct builds (no counterpart in the reference).  A
  * class's task list splits its work into tasks of (bra pair, up to
  * kets_per_task kets, a range of bra primitives) with at most
- * prim_quartets_per_lane primitive quartets per lane and task.  which = 0:
+ * prim_quartets_per_lane primitive quartets per lane and batch of kets.  Where
+ * lists are long an s/p task takes 4 or 8 such groups of 32 kets, where they are
+ * short some classes take a fraction of prim_quartets_per_lane.  which = 0:
  * J/K, 21 quartet classes in the order of gbhf_profile_classes; which = 1:
  * gradient, 36 (bra class, ket class) pairs, pair classes ss, ps, pp, ds, dp,
  * dd, bra-major.  budgets[2k] = prim_quartets_per_lane (1..65535),
